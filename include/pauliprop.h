@@ -299,13 +299,14 @@ int pp_power_table(double lambda, int32_t kmax, double *out);
 const char *pp_last_error(void);
 
 /* Launch configuration of the bucketed window-1 rotations (no counterpart in the
- * reference; results do not depend on it).  (bucket_cap, items_per_thread) must be
- * a compiled variant: (128, 4), (256, 4), (512, 4), (256, 8), (512, 8) or
- * (1024, 8); a CTA of 256 threads has two staging areas of 256 * items_per_thread
- * terms (a group of bucket pairs in one, the next group's terms in the other).
- * load_div (3..16): bucketing aims at a mean load of at most bucket_cap /
- * load_div.  chunk (8..256): rotations launched between host checks.
- * pauliprop's autotuner (pauliprop/tune.py) measures the variants on the device
+ * reference; results do not depend on it).  load_div (3..16): bucketing aims at a
+ * mean load of at most a bucket's slots / load_div.  chunk (8..256): rotations
+ * launched between host checks.  (bucket_cap, items_per_thread): the variant of the
+ * one-rotation kernel that key-sharded runs use -- (128, 4), (256, 4), (512, 4),
+ * (256, 8), (512, 8) or (1024, 8); a CTA of 256 threads has two staging areas of
+ * 256 * items_per_thread terms -- and the slots of their buckets (an unsharded run
+ * has buckets of 32).
+ * pauliprop's autotuner (pauliprop/tune.py) measures the settings on the device
  * and caches the fastest per (word count, SM count); a new handle starts with
  * (512, 4, 6, 128). */
 typedef struct {

@@ -28,6 +28,7 @@
 #include "kernels_algebra.cuh"
 #include "kernels_small.cuh"
 #include "kernels_bucket.cuh"
+#include "kernels_block.cuh"
 
 using namespace pp;
 
@@ -72,6 +73,12 @@ int pp_fail_msg(int code, const char *msg) { return fail(code, msg); }
 
 static const pp_filter NOFILTER_H = {INT64_MAX, INT64_MAX, INT64_MAX, -1.0, 0.0, -1.0, 0.0, -1.0};
 static constexpr int CHUNK_ROT = 64;   // rotations launched between state read-backs
+
+// Host copy of what a chunk of bucketed rotations leaves (pinned).
+struct BkStat {
+    BkRec last;
+    DevState st;
+};
 
 struct pp_spv {
     int N = 0, NW = 1, dev = 0, nsm = 148;
@@ -133,16 +140,17 @@ struct pp_spv {
     double *bkc[2] = {nullptr, nullptr};
     int *bkcnt[2] = {nullptr, nullptr};
     int bk_bits_cap = -1;
+    unsigned *bk_delta = nullptr;           // bucket hash of each generator of the call
+    long long bk_delta_cap = 0;
+    BkStat *bk_stat = nullptr;              // pinned, two chunks
+    int bb_occ[2] = {0, 0};                 // resident CTAs per SM of k_bb_block (plain, batched)
     int bk_cap = 0;
     u64 *bk_rows = nullptr;
     BkRec *bk_rec = nullptr;
     long long bk_rec_cap = 0;
-    long long *bk_off = nullptr;
     int *bk_aux = nullptr;                  // [0] largest scatter count, [1] scatter error bits
-    std::unordered_map<int, cudaGraphExec_t> bk_graphs;   // key: bits * 4 + chunk class
-    long long bk_graph_gen = -1;
     pp_tuning tune = {BK_DEFAULT_CAP, BK_DEFAULT_ITEMS, 6, 128};  // pp_set_tuning
-    struct { int occ1 = 1, occ2 = 1, occb = 1; } bk_occ[8];        // resident CTAs per SM of each variant
+    struct { int occ1 = 1, occ2 = 1; } bk_occ[8];        // resident CTAs per SM of each variant
     // key-sharded runs (pp_shard_*): foreign-term counts per bucket of each set,
     // this rank, the current layout, and a device counter for packed terms
     int *bkfcnt[2] = {nullptr, nullptr};
@@ -716,12 +724,12 @@ extern "C" int pp_destroy(pp_spv *h) {
                     h->bcos, h->bsin, h->bend, h->hfin, h->hpart, h->heout, h->hrange, h->hnout, h->sel64, h->vtmp};
     for (void *p : ptrs) if (p) cudaFree(p);
     for (int i = 0; i < 3; ++i) if (h->gexec[i]) cudaGraphExecDestroy(h->gexec[i]);
-    for (auto &kv : h->bk_graphs) cudaGraphExecDestroy(kv.second);
     void *bptrs[] = {h->bkz[0], h->bkz[1], h->bkx[0], h->bkx[1], h->bkc[0], h->bkc[1], h->bkcnt[0], h->bkcnt[1],
-                     h->bk_rows, h->bk_rec, h->bk_off, h->bk_aux, h->bkfcnt[0], h->bkfcnt[1], h->shard_cnt};
+                     h->bk_rows, h->bk_rec, h->bk_aux, h->bk_delta, h->bkfcnt[0], h->bkfcnt[1], h->shard_cnt};
     for (void *p : bptrs) if (p) cudaFree(p);
     if (h->Ph) cudaFreeHost(h->Ph);
     if (h->gens_h) cudaFreeHost(h->gens_h);
+    if (h->bk_stat) cudaFreeHost(h->bk_stat);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return PP_OK;
@@ -845,9 +853,9 @@ struct RunProf {
 
 // ------------------------------------------------------------------ bucketed window-1 rotations
 // Window-1 rotations of a live set larger than k_small_run's shared memory run
-// one k_bk_rotate launch each over a hash-bucketed copy of the live set
-// (kernels_bucket.cuh); the sequence ends with a gather into a dense array and a
-// radix sort, so the live set is dense and sorted between calls as before.
+// over a hash-bucketed copy of the live set, a block of them per k_bb_block launch
+// (kernels_block.cuh); the sequence ends with a packing into a dense array and a
+// sort, so the live set is dense and sorted between calls as before.
 static int expect_dev(pp_spv *h, const u64 *k, double *out);
 static constexpr int BK_MIN_ROT = 32;     // shorter sequences keep the sorted-merge kernels
 // Internal status (never returned by the C ABI): a bucket layout for the live set
@@ -862,17 +870,16 @@ static bool bk_enabled() {
     return !(e && strcmp(e, "tiles") == 0);
 }
 
-// Compiled variants of k_bk_rotate: (bucket capacity, staged items per thread).
+// Compiled variants of k_bk_rotate (key-sharded runs): (bucket capacity, staged items per thread).
 typedef void (*BkKernel)(BkArgs, int);
 struct BkVariant {
     int cap, items;
-    BkKernel k1, k2, kb;            // one- and two-word keys; batched instances (two-word)
+    BkKernel k1, k2;                // one- and two-word keys
     size_t smem1, smem2;
 };
 
 #define PP_BK_VARIANT(C, I)                                                                                 \
-    { C, I, k_bk_rotate<1, C, I>, k_bk_rotate<2, C, I>, k_bk_rotate<2, C, I, true>, bk_smem_bytes<1, C, I>(),     \
-      bk_smem_bytes<2, C, I>() }
+    { C, I, k_bk_rotate<1, C, I>, k_bk_rotate<2, C, I>, bk_smem_bytes<1, C, I>(), bk_smem_bytes<2, C, I>() }
 static const BkVariant BK_VARIANTS[] = {PP_BK_VARIANT(128, 4), PP_BK_VARIANT(256, 4), PP_BK_VARIANT(512, 4),
                                         PP_BK_VARIANT(256, 8), PP_BK_VARIANT(512, 8), PP_BK_VARIANT(1024, 8)};
 static constexpr int BK_NVAR = sizeof(BK_VARIANTS) / sizeof(BK_VARIANTS[0]);
@@ -889,8 +896,7 @@ static void bk_launch(pp_spv *h, const BkVariant *v, const BkArgs &A, int k) {
     // persistent grid: every resident CTA, or one per bucket pair (the kernel sizes its groups)
     const long long pairs = 1ll << (A.bits - 1);
     const auto &oc = h->bk_occ[v - BK_VARIANTS];
-    const bool batch = NW == 2 && h->batch_on;
-    const int occ = NW == 1 ? oc.occ1 : batch ? oc.occb : oc.occ2;
+    const int occ = NW == 1 ? oc.occ1 : oc.occ2;
     const int grid = (int)std::min(pairs, (long long)h->nsm * occ);
     // programmatic dependent launch: the rotation's prologue overlaps the previous
     // rotation's tail (k_bk_rotate waits for its outputs in griddepcontrol.wait)
@@ -904,7 +910,7 @@ static void bk_launch(pp_spv *h, const BkVariant *v, const BkArgs &A, int k) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, NW == 1 ? v->k1 : batch ? v->kb : v->k2, A, k);
+    cudaLaunchKernelEx(&cfg, NW == 1 ? v->k1 : v->k2, A, k);
 }
 
 // Hash rows: fixed pseudo-random words (splitmix64 from a fixed seed), so the
@@ -932,6 +938,11 @@ static int bk_rows_init(pp_spv *h) {
     h->bk_rows = dr;
     h->bk_aux = da;
     CU(cudaMemcpyAsync(h->bk_rows, rows, sizeof rows, cudaMemcpyHostToDevice, h->stream));
+    return sync_check(h);
+}
+
+// Launch attributes of the one-rotation kernel's variants (key-sharded runs).
+static int bk_variants_init(pp_spv *h) {
     for (int i = 0; i < BK_NVAR; ++i) {
         const BkVariant &v = BK_VARIANTS[i];
         CU(cudaFuncSetAttribute(v.k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem1));
@@ -943,12 +954,8 @@ static int bk_rows_init(pp_spv *h) {
         h->bk_occ[i].occ1 = std::max(1, o);
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, v.k2, BK_THREADS, v.smem2));
         h->bk_occ[i].occ2 = std::max(1, o);
-        CU(cudaFuncSetAttribute(v.kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem2));
-        CU(cudaFuncSetAttribute(v.kb, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
-        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, v.kb, BK_THREADS, v.smem2));
-        h->bk_occ[i].occb = std::max(1, o);
     }
-    return sync_check(h);
+    return PP_OK;
 }
 
 // Smallest bucket count for n terms at a mean load of at most cap / load_div.
@@ -958,7 +965,7 @@ static int bk_bits_for(long long n, int cap, int load_div) {
     return b;
 }
 
-static BkArgs bk_args(pp_spv *h, const BkVariant *v, int bits, BkRec *rec) {
+static BkArgs bk_args(pp_spv *h, int bits, BkRec *rec) {
     BkArgs A;
     memset(&A, 0, sizeof A);
     for (int s = 0; s < 2; ++s) { A.z[s] = h->bkz[s]; A.x[s] = h->bkx[s]; A.c[s] = h->bkc[s]; A.cnt[s] = h->bkcnt[s]; }
@@ -994,8 +1001,8 @@ static int bk_scatter(pp_spv *h, const u64 *SZ, const u64 *SX, const double *SC,
     const long long slots = from >= 0 ? ((long long)cap << sbits) : n;
     const int grid = (int)std::max(1ll, std::min((slots + 255) / 256, (long long)h->nsm * 16));
     k_bk_scatter<NW><<<grid, 256, 0, s>>>(SZ, SX, SC, n, from >= 0 ? h->bkcnt[from] : nullptr, sbits, h->bkz[to],
-                                          h->bkx[to], h->bkc[to], h->bkcnt[to], bits, cap, h->bk_rows, h->bk_aux,
-                                          h->bk_aux + 1);
+                                          h->bkx[to], h->bkc[to], h->bkcnt[to], bits, __builtin_ctz(cap), h->bk_rows,
+                                          h->bk_aux, h->bk_aux + 1);
     int aux[2] = {0, 0};
     CU(cudaMemcpyAsync(aux, h->bk_aux, sizeof aux, cudaMemcpyDeviceToHost, s));
     TRY(sync_check(h));
@@ -1003,15 +1010,14 @@ static int bk_scatter(pp_spv *h, const u64 *SZ, const u64 *SX, const double *SC,
     return PP_OK;
 }
 
-// Bucket sets for 2^bits buckets of the tuned capacity.  Growing the allocation
+// Bucket sets for 2^bits buckets of cap slots.  Growing the allocation
 // moves the live bucket set `*cur` (of 2^cur_bits buckets; cur_bits < 0: none)
 // into the new set 0.  Every buffer is allocated before the old ones are freed.
 template <int NW>
-static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits) {
-    if (bits <= h->bk_bits_cap && h->bk_cap == h->tune.bucket_cap) return PP_OK;
-    if (cur_bits >= 0 && h->bk_cap != h->tune.bucket_cap)
+static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
+    if (bits <= h->bk_bits_cap && h->bk_cap == cap) return PP_OK;
+    if (cur_bits >= 0 && h->bk_cap != cap)
         return fail(PP_ERROR_EXCEPTION, "internal error: bucket capacity changed inside a call");
-    const int cap = h->tune.bucket_cap;
     // the two bucket sets, and room to convert a full layout (at most slots / 2
     // terms before the next split) back to a dense sorted set, plus 4 GiB; one
     // split of headroom (2^(bits+1) buckets) when that fits, else 2^bits
@@ -1031,10 +1037,8 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits) {
     u64 *nz[2] = {nullptr, nullptr}, *nx[2] = {nullptr, nullptr};
     double *nc[2] = {nullptr, nullptr};
     int *nn[2] = {nullptr, nullptr};
-    long long *noff = nullptr;
     auto drop = [&]() {
         for (int q = 0; q < 2; ++q) { dfree(h, nz[q]); dfree(h, nx[q]); dfree(h, nc[q]); dfree(h, nn[q]); }
-        dfree(h, noff);
     };
     int r = 0;
     for (int q = 0; q < 2 && !r; ++q) {
@@ -1043,7 +1047,6 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits) {
         if (!r) r = dalloc(h, &nc[q], slots);
         if (!r) r = dalloc(h, &nn[q], 1ll << nbits);
     }
-    if (!r) r = dalloc(h, &noff, (1ll << nbits) + 1);
     if (r) { drop(); return r; }
     if (cur_bits >= 0 && h->bk_bits_cap >= 0) {
         // the live bucket set keeps its layout: copy it into new set 0
@@ -1061,8 +1064,6 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits) {
         dfree(h, h->bkz[q]); dfree(h, h->bkx[q]); dfree(h, h->bkc[q]); dfree(h, h->bkcnt[q]);
         h->bkz[q] = nz[q]; h->bkx[q] = nx[q]; h->bkc[q] = nc[q]; h->bkcnt[q] = nn[q];
     }
-    dfree(h, h->bk_off);
-    h->bk_off = noff;
     h->bk_bits_cap = nbits;
     h->bk_cap = cap;
     return PP_OK;
@@ -1076,8 +1077,6 @@ static void bk_release(pp_spv *h) {
         h->bkc[q] = nullptr;
         h->bkcnt[q] = nullptr;
     }
-    dfree(h, h->bk_off);
-    h->bk_off = nullptr;
     h->bk_bits_cap = -1;
     for (int q = 0; q < 2; ++q) { dfree(h, h->bkfcnt[q]); h->bkfcnt[q] = nullptr; }
     h->bkfcnt_bits = -1;
@@ -1093,7 +1092,7 @@ static int bk_regrid(pp_spv *h, int *cur, int *bits) {
     for (;;) {
         if (nbits + 1 > BK_ROWS) return fail(PP_OUT_OF_MEMORY, "bucketed live set exceeds 2^26 buckets");
         ++nbits;
-        TRY(bk_reserve<NW>(h, nbits, cur, *bits));
+        TRY(bk_reserve<NW>(h, nbits, cur, *bits, h->bk_cap));
         int mx = 0;
         TRY(bk_scatter<NW>(h, h->bkz[*cur], h->bkx[*cur], h->bkc[*cur], 0, *cur, *bits, *cur ^ 1, nbits, &mx));
         if (mx >= 0 && mx <= h->bk_cap / 2) break;
@@ -1103,49 +1102,24 @@ static int bk_regrid(pp_spv *h, int *cur, int *bits) {
     return PP_OK;
 }
 
-// Graph of `len` consecutive k_bk_rotate launches over 2^bits buckets.
-template <int NW>
-static int bk_graph(pp_spv *h, const BkVariant *v, int bits, int cls, int len, cudaGraphExec_t *out) {
-    if (h->bk_graph_gen != h->buf_gen) {
-        for (auto &kv : h->bk_graphs) cudaGraphExecDestroy(kv.second);
-        h->bk_graphs.clear();
-        h->bk_graph_gen = h->buf_gen;
-    }
-    const int key = bits * 4 + cls;
-    auto it = h->bk_graphs.find(key);
-    if (it != h->bk_graphs.end()) { *out = it->second; return PP_OK; }
-    const BkArgs A = bk_args(h, v, bits, h->bk_rec);
-    cudaGraph_t graph = nullptr;
-    CU(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < len; ++k) bk_launch<NW>(h, v, A, k);
-    CU(cudaStreamEndCapture(h->stream, &graph));
-    cudaGraphExec_t ex = nullptr;
-    cudaError_t e = cudaGraphInstantiate(&ex, graph, 0);
-    cudaGraphDestroy(graph);
-    if (e != cudaSuccess) return fail(PP_DEVICE_ERROR, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-    h->bk_graphs[key] = ex;
-    *out = ex;
-    return PP_OK;
-}
-
-// Gathers the bucket set `cur` (2^bits buckets) into live set 0 and
-// radix-sorts it: the live set is dense and sorted again.  Every allocation
+// Packs the n terms of the bucket set `cur` (2^bits buckets) into live set 0 and sorts
+// it: the live set is dense and sorted again.  Every allocation the packing needs
 // comes first, so a failure leaves the dense live set as it was.
 template <int NW>
-static int bk_to_dense(pp_spv *h, int cur, int bits) {
+static int bk_to_dense(pp_spv *h, int cur, int bits, long long n) {
     const int nb = 1 << bits;
     cudaStream_t s = h->stream;
-    k_bk_offsets<<<1, BKS_THREADS, 0, s>>>(h->bkcnt[cur], nb, h->bk_cap, h->bk_off);
-    long long n = 0;
-    CU(cudaMemcpyAsync(&n, h->bk_off + nb, sizeof n, cudaMemcpyDeviceToHost, s));
-    TRY(sync_check(h));
     PP_TRACE("buckets -> dense: %lld terms (2^%d buckets)", n, bits);
     TRY(radix_reserve(h, n));
     TRY(ensure_live(h, n + 1, false));
-    k_bk_gather<NW><<<std::max(1, std::min(h->nsm * 8, (nb + 7) / 8)), 256, 0, s>>>(
-        h->bkz[cur], h->bkx[cur], h->bkc[cur], h->bkcnt[cur], nb, h->bk_cap, h->bk_off, h->z[0], h->x[0], h->c[0],
-        h->cap, h->S);
+    unsigned long long *total = reinterpret_cast<unsigned long long *>(h->bk_aux);
+    CU(cudaMemsetAsync(total, 0, sizeof *total, s));
+    k_bk_pack<NW><<<(nb + 255) / 256, 256, 0, s>>>(h->bkz[cur], h->bkx[cur], h->bkc[cur], h->bkcnt[cur], nb,
+                                                  __builtin_ctz(h->bk_cap), total, h->z[0], h->x[0], h->c[0], h->cap, h->S);
+    unsigned long long got = 0;
+    CU(cudaMemcpyAsync(&got, total, sizeof got, cudaMemcpyDeviceToHost, s));
     TRY(sync_check(h));
+    if ((long long)got != n) return fail(PP_DEVICE_ERROR, "internal error: the buckets hold another number of terms");
     int in_t = 0;
     TRY(radix_sort<NW>(h, h->z[0], h->x[0], h->c[0], h->z[1], h->x[1], h->c[1], n, &in_t));
     DevState st;
@@ -1157,16 +1131,103 @@ static int bk_to_dense(pp_spv *h, int cur, int bits) {
     return PP_OK;
 }
 
+// Plan of a block of rotations from r0 over 2^bits buckets: at most len of them, as
+// long as the span of their deltas (bucket hashes) has a dimension of at most dims.
+// The span is a reduced basis, pivots ascending; a span of less than dims dimensions
+// is filled up (a larger coset costs a warp less than several small ones).
+static BbPlan bb_plan(const unsigned *delta, long long r0, int len, int bits, int dims) {
+    BbPlan pl;
+    memset(&pl, 0, sizeof pl);
+    pl.r0 = r0;
+    pl.bits = bits;
+    const unsigned mask = (1u << bits) - 1u;
+    auto add = [&](unsigned v) {           // false: v is outside the span, and the span has dims dimensions
+        for (int i = 0; i < pl.d; ++i)
+            if ((v >> pl.piv[i]) & 1u) v ^= pl.basis[i];
+        if (!v) return true;
+        if (pl.d == dims) return false;
+        const int p = __builtin_ctz(v);
+        for (int i = 0; i < pl.d; ++i)
+            if ((pl.basis[i] >> p) & 1u) pl.basis[i] ^= v;
+        int at = pl.d++;
+        for (; at > 0 && pl.piv[at - 1] > p; --at) {
+            pl.piv[at] = pl.piv[at - 1];
+            pl.basis[at] = pl.basis[at - 1];
+        }
+        pl.piv[at] = p;
+        pl.basis[at] = v;
+        return true;
+    };
+    while (pl.K < len && add(delta[r0 + pl.K] & mask)) ++pl.K;
+    for (int p = 0; p < bits && pl.d < dims; ++p) add(1u << p);
+    for (int j = 0; j < pl.K; ++j)
+        for (int i = 0; i < pl.d; ++i) pl.dl[j] |= (int)((delta[r0 + j] >> pl.piv[i]) & 1u) << i;
+    return pl;
+}
+
+template <int NW>
+static int bb_init(pp_spv *h) {
+    if (h->bb_occ[0]) return PP_OK;
+    constexpr size_t smem = bb_smem_bytes<NW>();
+    auto set = [&](auto kern, int *occ) -> int {
+        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CU(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+        int o = 0;
+        CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, 32 * BB_WARPS, smem));
+        *occ = std::max(1, o);
+        return PP_OK;
+    };
+    if constexpr (NW == 2) TRY(set(k_bb_block<2, true>, &h->bb_occ[1]));
+    return set(k_bb_block<NW, false>, &h->bb_occ[0]);
+}
+
+template <int NW>
+static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl) {
+    const bool batch = NW == 2 && h->batch_on;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min(((1ll << (pl.bits - pl.d)) + BB_WARPS - 1) / BB_WARPS,
+                                          (long long)h->nsm * h->bb_occ[batch ? 1 : 0]));
+    cfg.blockDim = dim3(32 * BB_WARPS);
+    cfg.dynamicSmemBytes = bb_smem_bytes<NW>();
+    cfg.stream = h->stream;
+    // programmatic dependent launch: a block's prologue overlaps the previous block's tail
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaError_t e;
+    if constexpr (NW == 2) e = batch ? cudaLaunchKernelEx(&cfg, k_bb_block<2, true>, A, pl) : cudaLaunchKernelEx(&cfg, k_bb_block<2, false>, A, pl);
+    else e = cudaLaunchKernelEx(&cfg, k_bb_block<1, false>, A, pl);
+    return e == cudaSuccess ? PP_OK : fail(PP_DEVICE_ERROR, std::string("launch failure: ") + cudaGetErrorString(e));
+}
+
+// Dimension of the cosets for n live terms in 2^bits buckets.  While the cosets are
+// fewer than the resident warps, a block's time is that of one warp's chain of steps,
+// which hardly depends on the coset's size up to about 128 terms (one scan, one batch
+// of pairs): larger cosets mean more rotations a launch.  With more cosets than that,
+// cosets as large as leave the resident set room for growth fill the warps' batches.
+static int bb_dims(long long n, int bits, int slots, int limit, long long warps) {
+    int d = 1;
+    while (d < limit && d < bits) {
+        const long long mean_num = n << (d + 1);                  // terms of a coset of d + 1 dimensions, times 2^bits
+        const bool small = mean_num <= (128ll << bits);
+        const bool fits = 4 * mean_num <= 3 * ((long long)slots << bits);
+        if (!(small || (fits && (1ll << (bits - d - 1)) >= warps))) break;
+        ++d;
+    }
+    return d;
+}
+
 // The window-1 sequence [start, L) on buckets.  The device cursor is at start.
-// per_rot: per-rotation times were asked for (each launch bracketed by events,
-// no graphs); otherwise the rotations replay from captured graphs, and a
-// profiled call (prof->on) times each graph replay.
+// per_rot: per-rotation times were asked for (blocks of one rotation, each launch
+// bracketed by events); a profiled call (prof->on) times each chunk of blocks.
 template <int NW>
 static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr, RunProf *prof, bool per_rot) {
     TRY(ensure_dense(h));
     TRY(bk_rows_init(h));
-    const BkVariant *var = bk_variant(h->tune.bucket_cap, h->tune.items_per_thread);
-    if (!var) return fail(PP_ERROR_EXCEPTION, "internal error: no compiled bucket variant for the tuning");
+    TRY(bb_init<NW>(h));
+    cudaStream_t s = h->stream;
     DevState st;
     TRY(read_state(h, &st));
     const long long n0 = st.n;
@@ -1175,25 +1236,31 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         TRY(dalloc(h, &h->bk_rec, L + 1));
         h->bk_rec_cap = L + 1;
     }
-    {
-        BkRec r0;
-        memset(&r0, 0, sizeof r0);
-        r0.n_in = n0;
-        r0.n_out = (unsigned long long)n0;
-        r0.acap = st.acap_logical;
-        CU(cudaMemcpyAsync(h->bk_rec + start, &r0, sizeof r0, cudaMemcpyHostToDevice, h->stream));
-        CU(cudaMemsetAsync(h->bk_rec + start + 1, 0, (L - start) * sizeof(BkRec), h->stream));
+    if (L > h->bk_delta_cap) {
+        TRY(dalloc(h, &h->bk_delta, L));
+        h->bk_delta_cap = L;
     }
+    BkRec r0;
+    memset(&r0, 0, sizeof r0);
+    r0.n_in = n0;
+    r0.n_out = (unsigned long long)n0;
+    r0.acap = st.acap_logical;
+    CU(cudaMemcpyAsync(h->bk_rec + start, &r0, sizeof r0, cudaMemcpyHostToDevice, s));
+    CU(cudaMemsetAsync(h->bk_rec + start + 1, 0, (L - start) * sizeof(BkRec), s));
+    k_bb_deltas<NW><<<(int)std::min((L - start + 127) / 128, (long long)h->nsm), 128, 0, s>>>(
+        h->gens + start, L - start, h->bk_rows, h->bk_delta + start);
+    std::vector<unsigned> delta((size_t)L);
+    CU(cudaMemcpyAsync(delta.data() + start, h->bk_delta + start, (size_t)(L - start) * sizeof(unsigned),
+                       cudaMemcpyDeviceToHost, s));
     // bucket the live set
-    int bits = bk_bits_for(n0, h->tune.bucket_cap, h->tune.load_div), cur = 0;
-    PP_TRACE("buckets: rotations [%lld, %lld), %lld live terms, 2^%d buckets of %d", start, L, n0, bits,
-             h->tune.bucket_cap);
+    int bits = bk_bits_for(n0, BB_CAP, h->tune.load_div), cur = 0;
+    PP_TRACE("buckets: rotations [%lld, %lld), %lld live terms, 2^%d buckets of %d", start, L, n0, bits, BB_CAP);
     // (when that layout does not fit, fewer and fuller buckets down to a mean load
     // of cap / 3, as long as no bucket is more than half full)
-    const int bmin = bk_bits_for(n0, h->tune.bucket_cap, 3);
+    const int bmin = bk_bits_for(n0, BB_CAP, 3);
     bool lowered = false;
     for (;;) {
-        const int rr = bk_reserve<NW>(h, bits, &cur, -1);
+        const int rr = bk_reserve<NW>(h, bits, &cur, -1, BB_CAP);
         if (rr == BK_NOFIT && bits > bmin) {
             --bits;
             lowered = true;
@@ -1202,11 +1269,15 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         if (rr) return rr;                  // BK_NOFIT: nothing changed, the dense set is the input
         int mx = 0;
         TRY(bk_scatter<NW>(h, h->z[st.cur], h->x[st.cur], h->c[st.cur], n0, -1, 0, 0, bits, &mx));
-        if (mx >= 0 && mx <= h->bk_cap / 2) break;
+        if (mx >= 0 && mx <= BB_CAP / 2) break;
         if (lowered) return BK_NOFIT;       // the fuller layout fails the half-full rule, a larger one does not fit
         if (++bits > BK_ROWS) return fail(PP_OUT_OF_MEMORY, "bucketed live set exceeds 2^26 buckets");
     }
-    cudaStream_t s = h->stream;
+    // a rotation whose input values may not have passed the strict filter starts a block
+    // that applies it to every term
+    auto full_at = [&](long long r) { return r == start || (h->gens_h[r - 1].flags & GEN_CHANNEL) != 0; };
+    struct Block { long long r0; int K; };
+    std::vector<Block> blocks;             // completed blocks, in order
     // totals and counters of rotations [start, upto) into the device state, and the
     // live set (bucket set cur) back to the dense sorted layout
     auto finish = [&](long long upto) -> int {
@@ -1216,134 +1287,181 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         TRY(read_state(h, &st));
         std::vector<long long> rr;
         if (h->rec_on) rr.assign((size_t)(4 * (upto - start)), 0);
+        long long acap = st.acap_logical;
         for (long long r = start; r < upto; ++r) {
             const BkRec &o = rec[(size_t)(r - start + 1)];
-            const long long n = o.n_in, a = (long long)o.created, tot = (long long)o.n_out, np = (long long)o.np;
+            const long long n = (long long)rec[(size_t)(r - start)].n_out, a = (long long)o.created, tot = (long long)o.n_out;
+            // the early-merge rule (spv_evolve.jl:356-362), as k_bb_block applies it
+            const bool pref = n > acap;
+            const long long np = !pref ? 0 : full_at(r) ? (long long)o.np : n;
+            if (pref && np > acap) acap = std::max(2 * acap, np);
             st.live_in += n;
             st.created += a;
             st.merge_in += n + a;
             st.merge_out += tot;
             if (tot > st.peak) st.peak = tot;
-            if (o.pref) st.early += 1;
+            if (pref) st.early += 1;
             prof->bk_rot += 1;
-            prof->bk_bytes += (double)(16 * NW + 8) * (double)(n + tot);
             if (h->rec_on) {
                 // WindowCounters of the rotation (window = 1): an early boundary merges
                 // n -> np first, the regular one np + a -> total
                 long long *q = &rr[(size_t)(4 * (r - start))];
                 q[0] = a;
-                q[1] = (o.pref ? n + np : n) + a;
-                q[2] = (o.pref ? np : 0) + tot;
-                q[3] = o.pref ? 1 : 0;
+                q[1] = (pref ? n + np : n) + a;
+                q[2] = (pref ? np : 0) + tot;
+                q[3] = pref ? 1 : 0;
             }
         }
+        for (const Block &b : blocks)      // a block reads its first rotation's terms and writes its last one's
+            prof->bk_bytes += (double)(16 * NW + 8) * ((double)rec[(size_t)(b.r0 - start)].n_out +
+                                                       (double)rec[(size_t)(b.r0 + b.K - start)].n_out);
         if (h->rec_on && upto > start)
             CU(cudaMemcpy(h->rec + 4 * start, rr.data(), rr.size() * sizeof(long long), cudaMemcpyHostToDevice));
-        {
-            // the early-merge capacity rule after the last rotation (as k_bk_rotate applies it)
-            const BkRec &o = rec.back();
-            long long acap = o.acap;
-            if (o.pref && (long long)o.np > acap) acap = std::max(2 * acap, (long long)o.np);
-            st.acap_logical = acap;
-        }
+        st.acap_logical = acap;
         st.rot = upto;
         TRY(write_state(h, &st));
-        return bk_to_dense<NW>(h, cur, bits);
+        return bk_to_dense<NW>(h, cur, bits, (long long)rec.back().n_out);
     };
     cur = 0;
-    long long done = start;
+    int limit = BB_DMAX;                   // dimension of a coset at most (less after one did not fit)
     const int chunk = h->tune.chunk;
-    std::vector<cudaEvent_t> gev;      // event pairs around the graph replays of a chunk (profiled calls)
-    struct GevGuard {
-        std::vector<cudaEvent_t> &v;
-        ~GevGuard() { for (auto e : v) cudaEventDestroy(e); }
-    } gevg{gev};
-    while (done < L) {
-        const long long len = std::min((long long)chunk, L - done);
-        if (bits < 1 || bits > h->bk_bits_cap || h->bk_cap != var->cap || L + 1 > h->bk_rec_cap || (cur & ~1))
+    if (!h->bk_stat) {
+        if (cudaMallocHost((void **)&h->bk_stat, 2 * sizeof(BkStat)) != cudaSuccess) {
+            cudaGetLastError();
+            h->bk_stat = nullptr;
+            return fail(PP_OUT_OF_MEMORY, "cudaMallocHost");
+        }
+    }
+    // the chunks launched and not yet looked at (two at most), and their events: around
+    // the launches, and behind the copy of the state that ends the chunk
+    struct Chunk {
+        long long first, end, n;           // its first block, its last rotation + 1, the terms it was planned for
+        int dims;
+    };
+    std::vector<Chunk> inflight;
+    cudaEvent_t cev[2][3] = {};
+    struct EvGuard {
+        cudaEvent_t (*v)[3];
+        ~EvGuard() { for (int i = 0; i < 2; ++i) for (int k = 0; k < 3; ++k) if (v[i][k]) cudaEventDestroy(v[i][k]); }
+    } evg{cev};
+    const bool timed = prof->on || per_rot;
+    for (int i = 0; i < 2; ++i)
+        for (int k = timed ? 0 : 2; k < 3; ++k)
+            CU(cudaEventCreateWithFlags(&cev[i][k], timed ? cudaEventDefault : cudaEventDisableTiming));
+    st.bk_fail = 0x7fffffffffffffffll;
+    st.bk_pad = 0;
+    TRY(write_state(h, &st));
+    long long done = start, launched = start, n = n0, seq = 0;
+    double growth = 4.0;                   // of the live set over the last chunk
+    // enqueues the chunk [launched, ...): blocks to the first block end at or after `chunk` rotations
+    auto enqueue = [&]() -> int {
+        const long long end = std::min(L, launched + chunk);
+        if (bits < 1 || bits > h->bk_bits_cap || h->bk_cap != BB_CAP || L + 1 > h->bk_rec_cap || (cur & ~1))
             return fail(PP_ERROR_EXCEPTION, "internal error: inconsistent bucket layout before a launch");
-        k_bk_begin<<<1, 1, 0, s>>>(h->S, done, cur, 1);
-        prof->launches += 1;
-        int ngraph = 0;
-        if (!per_rot) {
-            long long r = 0;
-            while (r < len) {
-                const int cls = (len - r >= chunk) ? 0 : (len - r >= 8) ? 1 : 2;
-                const int cl = cls == 0 ? chunk : cls == 1 ? 8 : 1;
-                if (r > 0) {
-                    // a later graph of the chunk starts at rotation done + r
-                    k_bk_begin<<<1, 1, 0, s>>>(h->S, done + r, (cur + (int)r) & 1, 0);
-                    prof->launches += 1;
-                }
-                cudaGraphExec_t ex = nullptr;
-                TRY(bk_graph<NW>(h, var, bits, cls, cl, &ex));
-                if (prof->on) {
-                    while ((int)gev.size() < 2 * (ngraph + 1)) {
-                        cudaEvent_t e;
-                        CU(cudaEventCreate(&e));
-                        gev.push_back(e);
-                    }
-                    CU(cudaEventRecord(gev[2 * ngraph], s));
-                }
-                CU(cudaGraphLaunch(ex, s));
-                if (prof->on) CU(cudaEventRecord(gev[2 * ngraph++ + 1], s));
-                prof->launches += cl;
-                r += cl;
-            }
-        } else {
-            const BkArgs A = bk_args(h, var, bits, h->bk_rec);
-            for (long long k = 0; k < len; ++k) {
-                cudaEvent_t e0, e1;
-                cudaEventCreate(&e0);
-                cudaEventCreate(&e1);
-                cudaEventRecord(e0, s);
-                bk_launch<NW>(h, var, A, (int)k);
-                cudaEventRecord(e1, s);
+        const int slot = (int)(seq & 1);
+        const BkArgs A = bk_args(h, bits, h->bk_rec);
+        const int dims = bb_dims(n, bits, bb_slots<NW>(), limit, (long long)h->nsm * BB_WARPS * h->bb_occ[0]);
+        Chunk c{(long long)blocks.size(), 0, n, dims};
+        if (timed && !per_rot) CU(cudaEventRecord(cev[slot][0], s));
+        while (launched < end) {
+            // a block ends at the end of the sequence or at a channel; up to there, blocks of equal length
+            const long long r = launched;
+            long long cut = r + 1;
+            while (cut < L && cut - r < 4 * BB_KMAX && !(h->gens_h[cut - 1].flags & GEN_CHANNEL)) ++cut;
+            const int most = per_rot ? 1 : dims;
+            const long long parts = (cut - r + most - 1) / most;
+            BbPlan pl = bb_plan(delta.data(), r, (int)((cut - r + parts - 1) / parts), bits, dims);
+            pl.full = full_at(r) ? 1 : 0;
+            pl.kprev = blocks.empty() ? 0 : blocks.back().K;
+            pl.cur = cur;
+            if (per_rot) CU(cudaEventRecord(cev[slot][0], s));
+            TRY(bb_launch<NW>(h, A, pl));
+            if (per_rot) {
+                CU(cudaEventRecord(cev[slot][1], s));
                 TRY(sync_check(h));
                 float ms = 0.f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                cudaEventDestroy(e0);
-                cudaEventDestroy(e1);
-                const long long r = done + k;
+                cudaEventElapsedTime(&ms, cev[slot][0], cev[slot][1]);
                 prof->t_merge += ms * 1e-3;
-                prof->launches += 1;
                 if (ctr && r < ctr->nwin && ctr->t_merge) ctr->t_merge[r] += ms * 1e-3;
             }
+            prof->launches += 1;
+            blocks.push_back({r, pl.K});
+            cur ^= 1;
+            launched += pl.K;
         }
-        TRY(sync_check(h));
-        for (int q = 0; q < ngraph; ++q) {
+        if (timed && !per_rot) CU(cudaEventRecord(cev[slot][1], s));
+        CU(cudaMemcpyAsync(&h->bk_stat[slot].last, h->bk_rec + launched, sizeof(BkRec), cudaMemcpyDeviceToHost, s));
+        CU(cudaMemcpyAsync(&h->bk_stat[slot].st, h->S, sizeof(DevState), cudaMemcpyDeviceToHost, s));
+        CU(cudaEventRecord(cev[slot][2], s));
+        c.end = launched;
+        inflight.push_back(c);
+        ++seq;
+        return PP_OK;
+    };
+    int split = 0;                         // the layout is to be split before the next launch
+    while (done < L) {
+        // a second chunk goes out before the first is looked at, unless the set grows so fast
+        // that it would outgrow the layout by then
+        while (launched < L && !split && (inflight.empty() || (inflight.size() == 1 && !per_rot &&
+                                          (double)n * growth * growth <= (double)(BB_CAP / 4) * (double)(1ll << bits))))
+            TRY(enqueue());
+        const Chunk c = inflight.front();
+        inflight.erase(inflight.begin());
+        const int slot = (int)((seq - 1 - (long long)inflight.size()) & 1);
+        CU(cudaEventSynchronize(cev[slot][2]));
+        CU(cudaGetLastError());
+        if (timed && !per_rot) {
             float ms = 0.f;
-            CU(cudaEventElapsedTime(&ms, gev[2 * q], gev[2 * q + 1]));
+            CU(cudaEventElapsedTime(&ms, cev[slot][0], cev[slot][1]));
             prof->t_merge += ms * 1e-3;
         }
-        TRY(read_state(h, &st));
-        if (st.err & ~ERR_OVERFLOW) return check_err(h, st);   // the dense live set is the sequence's input
-        const long long completed = (st.err & ERR_OVERFLOW) ? std::max(0ll, std::min(len, st.bk_fail - done)) : len;
-        cur = (cur + (int)(completed & 1)) & 1;
-        done += completed;
-        BkRec last;
-        CU(cudaMemcpyAsync(&last, h->bk_rec + done, sizeof last, cudaMemcpyDeviceToHost, s));
-        TRY(sync_check(h));
-        const bool over = (st.err & ERR_OVERFLOW) != 0;
-        if (over) {
+        st = h->bk_stat[slot].st;
+        BkRec last = h->bk_stat[slot].last;
+        if (st.err & ~ERR_OVERFLOW) {          // the dense live set is the sequence's input
+            TRY(sync_check(h));
+            return check_err(h, st);
+        }
+        int over = 0;
+        done = c.end;
+        if (st.err & ERR_OVERFLOW) {
+            // the blocks before the failed one stand; it and what was launched after it
+            // (which did nothing) run again
+            TRY(sync_check(h));
+            TRY(read_state(h, &st));
+            over = st.bk_pad;
+            while (!blocks.empty() && blocks.back().r0 >= st.bk_fail) { blocks.pop_back(); cur ^= 1; }
+            done = blocks.empty() ? start : blocks.back().r0 + blocks.back().K;
             st.err &= ~ERR_OVERFLOW;
+            st.bk_fail = 0x7fffffffffffffffll;
+            st.bk_pad = 0;
             TRY(write_state(h, &st));
-            CU(cudaMemsetAsync(h->bk_rec + done + 1, 0, sizeof(BkRec), s));
+            CU(cudaMemsetAsync(h->bk_rec + done + 1, 0, (launched - done) * sizeof(BkRec), s));
+            CU(cudaMemcpyAsync(&last, h->bk_rec + done, sizeof last, cudaMemcpyDeviceToHost, s));
+            TRY(sync_check(h));
+            inflight.clear();
+            launched = done;
+            if (over & 2) limit = std::max(1, c.dims - 1);
+        } else if (limit < BB_DMAX) {
+            ++limit;
         }
-        if (done < L && (over || last.maxcnt > h->bk_cap / 2)) {
-            const int rr = bk_regrid<NW>(h, &cur, &bits);
-            PP_TRACE("buckets: split at rotation %lld (largest bucket %d) -> 2^%d buckets%s", done, last.maxcnt, bits,
-                     rr == BK_NOFIT ? ": does not fit, hand-over to the sorted-merge kernels" : "");
-            if (rr == BK_NOFIT) {
-                // no room for a larger layout: the rotations so far go back to the
-                // dense sorted set, the bucket sets are freed, and the sorted-merge
-                // kernels take the rest of the sequence
-                TRY(finish(done));
-                bk_release(h);
-                return BK_NOFIT;
-            }
-            if (rr) return rr;
+        growth = std::max(1.0, (double)last.n_out / std::max(1.0, (double)c.n));
+        n = (long long)last.n_out;
+        if (done < L && ((over & 1) || last.maxcnt > 7 * BB_CAP / 8 || n > ((long long)(BB_CAP / 4) << bits)))
+            split = 1;
+        if (done == L || !split || !inflight.empty()) continue;
+        split = 0;
+        const int rr = bk_regrid<NW>(h, &cur, &bits);
+        PP_TRACE("buckets: split at rotation %lld (%lld terms, largest bucket %d) -> 2^%d buckets%s", done, n, last.maxcnt,
+                 bits, rr == BK_NOFIT ? ": does not fit, hand-over to the sorted-merge kernels" : "");
+        if (rr == BK_NOFIT) {
+            // no room for a larger layout: the rotations so far go back to the
+            // dense sorted set, the bucket sets are freed, and the sorted-merge
+            // kernels take the rest of the sequence
+            TRY(finish(done));
+            bk_release(h);
+            return BK_NOFIT;
         }
+        if (rr) return rr;
     }
     TRY(finish(L));
     if (h->batch_on) return PP_OK;      // batched instances are measured per instance at their ends
@@ -2117,11 +2235,6 @@ extern "C" int pp_set_tuning(pp_spv *h, const pp_tuning *t) {
                                        "(256, 4), (512, 4), (256, 8), (512, 8), (1024, 8)");
     if (t->load_div < 3 || t->load_div > 16) return fail(PP_ARGUMENT_ERROR, "pp_set_tuning: load_div must be in 3..16");
     if (t->chunk < 8 || t->chunk > 256) return fail(PP_ARGUMENT_ERROR, "pp_set_tuning: chunk must be in 8..256");
-    if (t->bucket_cap != h->tune.bucket_cap || t->items_per_thread != h->tune.items_per_thread ||
-        t->chunk != h->tune.chunk) {
-        for (auto &kv : h->bk_graphs) cudaGraphExecDestroy(kv.second);
-        h->bk_graphs.clear();
-    }
     h->tune = *t;
     return PP_OK;
 }
@@ -2449,10 +2562,11 @@ template <int NW>
 static int shard_begin_impl(pp_spv *h, int bits, int32_t *maxcnt) {
     TRY(ensure_dense(h));
     TRY(bk_rows_init(h));
+    TRY(bk_variants_init(h));
     DevState st;
     TRY(read_state(h, &st));
     int cur = 0;
-    const int rr = bk_reserve<NW>(h, bits, &cur, -1);
+    const int rr = bk_reserve<NW>(h, bits, &cur, -1, h->tune.bucket_cap);
     if (rr == BK_NOFIT) return fail(PP_OUT_OF_MEMORY, "the bucket layout of this shard does not fit in device memory");
     if (rr) return rr;
     int mx = 0;
@@ -2615,7 +2729,7 @@ static int shard_rotate_impl(pp_spv *h, int64_t r, int pref, int remote, int64_t
     const BkVariant *var = bk_variant(h->tune.bucket_cap, h->tune.items_per_thread);
     if (!var || var->cap != h->bk_cap) return fail(PP_ERROR_EXCEPTION, "internal error: bucket variant changed");
     cudaStream_t s = h->stream;
-    BkArgs A = bk_args(h, var, h->shard_bits, h->bk_rec);
+    BkArgs A = bk_args(h, h->shard_bits, h->bk_rec);
     A.fcnt[0] = h->bkfcnt[0];
     A.fcnt[1] = h->bkfcnt[1];
     A.remote = remote;
@@ -2657,7 +2771,7 @@ extern "C" int pp_shard_rotate(pp_spv *h, int64_t r, int32_t pref, int64_t *stat
 template <int NW>
 static int shard_regrid_impl(pp_spv *h, int bits, int32_t *maxcnt) {
     int cur = h->shard_cur;
-    const int rr = bk_reserve<NW>(h, bits, &cur, h->shard_bits);
+    const int rr = bk_reserve<NW>(h, bits, &cur, h->shard_bits, h->bk_cap);
     if (rr == BK_NOFIT) return fail(PP_OUT_OF_MEMORY, "the bucket layout of this shard does not fit in device memory");
     if (rr) return rr;
     int mx = 0;
@@ -2681,10 +2795,15 @@ extern "C" int pp_shard_end(pp_spv *h, double *expect_partial, double *stats_out
     if (!h) return fail(PP_ARGUMENT_ERROR, "null handle");
     if (!h->shard_on) return fail(PP_ARGUMENT_ERROR, "no key-sharded run in progress (pp_shard_begin)");
     h->shard_on = false;
-    TRY(h->NW == 1 ? bk_to_dense<1>(h, h->shard_cur, h->shard_bits) : bk_to_dense<2>(h, h->shard_cur, h->shard_bits));
+    DevState st;
+    TRY(read_state(h, &st));
+    BkRec o;                               // the terms after the last rotation that ran
+    CU(cudaMemcpyAsync(&o, h->bk_rec + st.rot, sizeof o, cudaMemcpyDeviceToHost, h->stream));
+    TRY(sync_check(h));
+    TRY(h->NW == 1 ? bk_to_dense<1>(h, h->shard_cur, h->shard_bits, (long long)o.n_out)
+                   : bk_to_dense<2>(h, h->shard_cur, h->shard_bits, (long long)o.n_out));
     double ev = 0.0;
     TRY(expect_dev(h, h->Ph->ket, &ev));
-    DevState st;
     TRY(read_state(h, &st));
     st.expect_val = ev;
     st.measure_valid = 1;

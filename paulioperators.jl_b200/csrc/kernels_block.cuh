@@ -1,0 +1,684 @@
+// Window-1 rotations over a hash-bucketed live set, several rotations per launch.
+//
+// The bucket hash h is GF(2)-linear (kernels_bucket.cuh): the partner P xor M of a
+// term of bucket b lies in bucket b xor h(M), for every term alike.  For a block of
+// K consecutive rotations with deltas h(M_1) .. h(M_K) the buckets therefore fall
+// into the cosets of the span D of the deltas, and no term of a coset meets a term
+// of another one within the block.  A CTA takes a coset (2^d buckets, d = dim D <=
+// K), holds its terms in shared memory through the K rotations
+// (_rotate_range! + _merge_spv!, spv_kernels.jl:146-177, 326-386, each with the
+// same arithmetic and rounding as everywhere else), and writes the survivors to
+// their buckets of the other bucket set.
+//
+// Within the block a rotation touches only the terms that anticommute with its
+// generator: the others keep their value, and a value that has passed the strict
+// filter once passes it again.  The filter is applied to every term only where
+// values may not have passed it: at the first rotation of a call and after a
+// channel (a block ends at a channel, which scales every survivor at its end).
+//
+// What bounds it: latency and instruction issue.  At 8e5 terms a block of six
+// rotations takes 64 us, of which DRAM traffic would take 10: a warp issues one
+// instruction every 11 cycles (fixed latencies, shared memory), and twelve warps are
+// what the resident sets leave room for.  A warp per coset, not a CTA: with a CTA of
+// eight warps per coset each warp found too few anticommuting terms to fill a batch,
+// and waited at a barrier per rotation (130 against 102 ms for the lattice circuit
+// below).  The index over all resident terms is built once per block and pays from
+// about three rotations on.
+// Measured (one B200, whole calls, one rotation per launch before): 8 x 8 lattice,
+// 3,520 rotations, up to 3.9e6 terms 154.9 -> 101.7 ms; 127-qubit graph, 6,504
+// rotations, up to 8e4 terms 43.4 -> 23.0 ms; 48 batched instances 60.1 -> 40.9 ms.
+#pragma once
+#include "kernels_bucket.cuh"
+
+namespace pp {
+
+constexpr int BB_CAP = 32;                     // slots of a bucket
+constexpr int BB_CAP_LOG = 5;
+constexpr int BB_KMAX = 8;                     // rotations of a block at most
+constexpr int BB_DMAX = 8;                     // dimension of a coset at most
+constexpr int BB_MEMBERS = 1 << BB_DMAX;       // buckets of a coset at most
+constexpr int BB_WARPS = 4;                    // warps of a CTA, each with a coset of its own
+constexpr unsigned BB_DEAD = 0x8000u;          // tag bit: the slot holds no live term
+
+// Slots of a warp's resident set and of its key index (twelve warps fit on an SM).
+template <int NW>
+__host__ __device__ constexpr int bb_slots() { return NW == 1 ? 448 : 288; }
+constexpr int BB_TAB = 1024;
+
+constexpr int RS_QCAP = 160;                   // entries of a warp's queue of slots (31 + 4 * 32 at most)
+
+// Shared memory of one resident set: coefficients, key words, index, tags.
+template <int NW, int SLOTS, int TAB>
+__host__ __device__ constexpr size_t rs_set_bytes() { return (size_t)SLOTS * (8 + 16 * NW + 2) + (size_t)TAB * 4; }
+template <int NW>
+__host__ __device__ constexpr size_t bb_smem_bytes() {
+    return BB_WARPS * (rs_set_bytes<NW, bb_slots<NW>(), BB_TAB>() + RS_QCAP * 2);
+}
+
+// One rotation as the steps use it: the generator's key words in 32-bit pieces
+// (z low to high, then x), the planes its parity test reads with their masks, and
+// cos / sin.
+template <int NW>
+struct RsGen {
+    double cosv, sinv;
+    unsigned g[4 * NW];
+    unsigned mask[4 * NW];
+    int plane[4 * NW];
+    int np, ng, acol, delta;
+};
+
+template <int NW>
+__device__ __forceinline__ void rs_gen(RsGen<NW> *o, const GenRec &g, int delta) {
+    o->cosv = g.cosv;
+    o->sinv = g.sinv;
+    o->ng = g.ng;
+    o->acol = g.acol;
+    o->delta = delta;
+    int np = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        o->g[2 * w] = (unsigned)g.gz[w];
+        o->g[2 * w + 1] = (unsigned)(g.gz[w] >> 32);
+        o->g[2 * NW + 2 * w] = (unsigned)g.gx[w];
+        o->g[2 * NW + 2 * w + 1] = (unsigned)(g.gx[w] >> 32);
+    }
+    // parity of popc(gx & z) + popc(gz & x): only planes under a nonzero mask
+    for (int p = 0; p < 4 * NW; ++p) {
+        const unsigned m = o->g[p < 2 * NW ? p + 2 * NW : p - 2 * NW];
+        if (m) {
+            o->plane[np] = p;
+            o->mask[np] = m;
+            ++np;
+        }
+    }
+    o->np = np;
+}
+
+// load_key through L2 only: a bucket set is rewritten by every second launch, and a
+// dependent launch may start before its predecessor's predecessor has ended, so its
+// lines must not be served from an SM's L1.
+template <int NW>
+__device__ __forceinline__ Key<NW> load_key_cg(const u64 *Z, const u64 *X, long long i) {
+    Key<NW> k;
+    if constexpr (NW == 1) {
+        k.z[0] = __ldcg(Z + i);
+        k.x[0] = __ldcg(X + i);
+    } else {
+        const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2 *>(Z) + i);
+        const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2 *>(X) + i);
+        k.z[0] = a.x; k.z[1] = a.y; k.x[0] = b.x; k.x[1] = b.y;
+    }
+    return k;
+}
+
+// A key in 32-bit words: z low to high, then x.
+template <int NW>
+struct Key32 {
+    unsigned w[4 * NW];
+};
+
+template <int NW>
+__device__ __forceinline__ Key<NW> key_wide(const Key32<NW> &k) {
+    Key<NW> o;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        o.z[w] = ((u64)k.w[2 * w + 1] << 32) | k.w[2 * w];
+        o.x[w] = ((u64)k.w[2 * NW + 2 * w + 1] << 32) | k.w[2 * NW + 2 * w];
+    }
+    return o;
+}
+
+template <int NW>
+__device__ __forceinline__ Key32<NW> key_narrow(const Key<NW> &k) {
+    Key32<NW> o;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+        o.w[2 * w] = (unsigned)k.z[w];
+        o.w[2 * w + 1] = (unsigned)(k.z[w] >> 32);
+        o.w[2 * NW + 2 * w] = (unsigned)k.x[w];
+        o.w[2 * NW + 2 * w + 1] = (unsigned)(k.x[w] >> 32);
+    }
+    return o;
+}
+
+// 32-bit multiply-xor mix of a key: its low bits are the index position, its high
+// 16 bits the fingerprint kept in the index entry.
+template <int NW>
+__device__ __forceinline__ unsigned rs_hash(const Key32<NW> &k) {
+    unsigned h = k.w[0] * 0x9E3779B1u;
+#pragma unroll
+    for (int q = 1; q < 4 * NW; ++q) h = (h ^ k.w[q]) * (q & 1 ? 0x85EBCA77u : 0xC2B2AE3Du) + (h >> 17);
+    h ^= h >> 15;
+    h *= 0x2C1B3C6Du;
+    h ^= h >> 13;
+    return h;
+}
+
+// A term set resident in shared memory: planes of 32-bit key words, coefficients,
+// tags (local bucket, BB_DEAD), and an open-addressed index of every slot's key
+// (entry: fingerprint << 16 | slot + 1).  Entries are never taken out: a dropped
+// term's slot stays indexed, and the key's return finds and revives it.
+template <int NW, int SLOTS, int TAB>
+struct ResidentSet {
+    double *c;
+    unsigned *w;                    // [4 NW][SLOTS]
+    unsigned *tab;                  // [TAB]
+    unsigned short *tag;            // [SLOTS]
+
+    __device__ __forceinline__ Key32<NW> key(int i) const {
+        Key32<NW> k;
+#pragma unroll
+        for (int p = 0; p < 4 * NW; ++p) k.w[p] = w[p * SLOTS + i];
+        return k;
+    }
+    __device__ __forceinline__ void put(int i, const Key32<NW> &k, double v, unsigned t) const {
+#pragma unroll
+        for (int p = 0; p < 4 * NW; ++p) w[p * SLOTS + i] = k.w[p];
+        c[i] = v;
+        tag[i] = (unsigned short)t;
+    }
+    __device__ __forceinline__ void insert(int i, unsigned h) const {
+        const unsigned e = (h & 0xffff0000u) | (unsigned)(i + 1);
+        unsigned p = h & (TAB - 1);
+        for (int probe = 0; probe < TAB; ++probe) {
+            if (atomicCAS(&tab[p], 0u, e) == 0u) return;
+            p = (p + 1) & (TAB - 1);
+        }
+    }
+    // slot of the key, or -1
+    __device__ __forceinline__ int find(const Key32<NW> &k, unsigned h) const {
+        unsigned p = h & (TAB - 1);
+        for (int probe = 0; probe < TAB; ++probe) {
+            const unsigned e = *(volatile unsigned *)&tab[p];
+            if (e == 0) return -1;
+            if (((e ^ h) & 0xffff0000u) == 0) {
+                const int i = (int)(e & 0xffffu) - 1;
+                unsigned d = 0;
+#pragma unroll
+                for (int q = 0; q < 4 * NW; ++q) d |= w[q * SLOTS + i] ^ k.w[q];
+                if (d == 0) return i;
+            }
+            p = (p + 1) & (TAB - 1);
+        }
+        return -1;
+    }
+};
+
+// What the steps read besides the set: the filters and, for batched instances,
+// their angle tables and ends.
+struct RsParams {
+    FQuick strict;
+    const DevFilter *strict_full;
+    const DevFilter *local;
+    bool local_on;
+    const double *bcos, *bsin;
+    const long long *bend;
+    long long ninst;
+    int ncol;
+    DevState *S;
+};
+
+// Instance of a batched term, or -1 when it has ended before rotation r (or the tag
+// is no instance).
+template <int NW>
+__device__ __forceinline__ long long rs_instance(const Key32<NW> &k, const RsParams &q, long long r) {
+    const u64 t = ((u64)k.w[3 % (4 * NW)] << 32) | k.w[2 % (4 * NW)];     // z word 1
+    if (t >= (u64)q.ninst) {
+        flag_bounds(q.S, 11, (long long)t);
+        return -1;
+    }
+    return r < q.bend[t] ? (long long)t : -1;
+}
+
+// should_drop (spv_kernels.jl:64-79) on a key in 32-bit words.
+template <int NW>
+__device__ __forceinline__ bool rs_drop(const RsParams &q, const Key32<NW> &k, double absc) {
+    if (q.strict.full) return should_drop<NW>(*q.strict_full, key_wide<NW>(k), absc);
+    int wt = 0;
+#pragma unroll
+    for (int t = 0; t < 2 * NW; ++t) wt += __popc(k.w[t] | k.w[2 * NW + t]);
+    bool drop = absc <= q.strict.thresh || wt > q.strict.wmax;
+    if (q.strict.xwmax < 64 * NW) {
+        int xw = 0;
+#pragma unroll
+        for (int t = 0; t < 2 * NW; ++t) xw += __popc(k.w[2 * NW + t]);
+        drop = drop || xw > q.strict.xwmax;
+    }
+    return drop;
+}
+
+// One rotation on one anticommuting slot i of the resident set.  Of two partners'
+// slots (live or not) the lower runs it for both, so every slot has one writer in a
+// step and no barrier is needed between the reads and the writes of a pair's
+// coefficients.  A sin branch without a slot is appended at n0 + atomicAdd(*fresh).
+// Returns the change of the live count in the low half and the sin branches appended
+// (WindowCounters) in the high half.
+template <int NW, int SLOTS, int TAB, bool BATCH>
+__device__ __forceinline__ int rs_pair(const ResidentSet<NW, SLOTS, TAB> &s, const RsGen<NW> &g, const RsParams &q, int i,
+                                       int n0, int *fresh, int *full, long long r) {
+    const unsigned ti = s.tag[i];
+    const double ci = s.c[i];
+    const Key32<NW> k = s.key(i);
+    Key32<NW> p;
+#pragma unroll
+    for (int t = 0; t < 4 * NW; ++t) p.w[t] = k.w[t] ^ g.g[t];
+    const unsigned hp = rs_hash<NW>(p);
+    const int j = s.find(p, hp);
+    const bool ai = !(ti & BB_DEAD);
+    if (j >= 0 ? j < i : !ai) return 0;
+    const unsigned tj = j >= 0 ? s.tag[j] : BB_DEAD;
+    const bool aj = !(tj & BB_DEAD);
+    if (!ai && !aj) return 0;
+    const double cj = j >= 0 ? s.c[j] : 0.0;
+    double cv = g.cosv, sv = g.sinv;
+    if constexpr (BATCH) {
+        const long long t = rs_instance<NW>(k, q, r);
+        if (t < 0) return 0;
+        cv = q.bcos[t * q.ncol + g.acol];
+        sv = q.bsin[t * q.ncol + g.acol];
+    }
+    // phase of the sin branch of P (_rotate_range!, spv_kernels.jl:155-163); the
+    // partner's has the opposite sign: k(P) + k(P xor M) = 0 mod 4, and k is odd
+    int m1 = 0, nzp = 0, nzx = 0;
+#pragma unroll
+    for (int t = 0; t < 2 * NW; ++t) {
+        m1 += __popc(g.g[2 * NW + t] & k.w[t]);
+        nzp += __popc(p.w[t] & p.w[2 * NW + t]);
+        nzx += __popc(k.w[t] & k.w[2 * NW + t]);
+    }
+    const double sgs = (double)(((nzp - g.ng - nzx + 2 * m1) & 3) - 2) * sv;
+    const double si = __dmul_rn(sgs, ci);                        // lands on P xor M
+    const double sj = __dmul_rn(-sgs, cj);                       // lands on P
+    bool oki = ai, okj = aj;
+    if (q.local_on) {
+        oki = ai && !should_drop<NW>(*q.local, key_wide<NW>(p), fabs(si));
+        okj = aj && !should_drop<NW>(*q.local, key_wide<NW>(k), fabs(sj));
+    }
+    // live value first, then the append (_try_merge!)
+    double vi = __dmul_rn(ci, cv), vj = __dmul_rn(cj, cv);
+    vi = ai ? (okj ? __dadd_rn(vi, sj) : vi) : sj;
+    vj = aj ? (oki ? __dadd_rn(vj, si) : vj) : si;
+    const bool ki = (ai || okj) && !rs_drop<NW>(q, k, fabs(vi));
+    const bool kj = (aj || oki) && !rs_drop<NW>(q, p, fabs(vj));
+    if (ki) s.c[i] = vi;
+    if (ki != ai) s.tag[i] = (unsigned short)(ti ^ BB_DEAD);
+    if (j >= 0) {
+        if (kj) s.c[j] = vj;
+        if (kj != aj) s.tag[j] = (unsigned short)(tj ^ BB_DEAD);
+    } else if (kj) {
+        const int o = n0 + atomicAdd(fresh, 1);
+        if (o < SLOTS) {
+            s.put(o, p, vj, (ti ^ (unsigned)g.delta) & ~BB_DEAD);
+            __threadfence_block();
+            s.insert(o, hp);
+        } else {
+            *full = 1;
+        }
+    }
+    return (oki ? 0x10000 : 0) + (okj ? 0x10000 : 0) + (int)ki - (int)ai + (int)kj - (int)aj;
+}
+
+// One rotation over the n slots of a resident set that T threads share (T = 32: the
+// calling warp; else the CTA; the set's earlier writes visible, a barrier of them all
+// after it).  Each warp scans 128 slots at a time with the parity test alone (one
+// 16-byte shared read per plane under the generator's mask), queues the
+// anticommuting ones, and runs rs_pair on 32 of them at a time, so that the long path
+// runs with full warps although only about a tenth of the terms take it.  Returns
+// this thread's rs_pair sums.
+template <int NW, int SLOTS, int TAB, int T, bool BATCH>
+__device__ __forceinline__ int rs_step(const ResidentSet<NW, SLOTS, TAB> &s, const RsGen<NW> &g, const RsParams &q, int n,
+                                       unsigned short *queue, int *fresh, int *full, long long r) {
+    const int lane = threadIdx.x & 31, warp = T == 32 ? 0 : threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    int cnt = 0, out = 0;
+    const int np = g.np;
+    const int p0 = g.plane[0] * SLOTS;
+    const unsigned m0 = g.mask[0];
+    for (int base = warp * 128;; base += (T / 32) * 128) {
+        const bool more = base < n;                     // warp-uniform
+        if (more) {
+            const int i0 = base + 4 * lane;
+            uint4 a = make_uint4(0u, 0u, 0u, 0u);
+            if (i0 < n && np > 0) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(s.w + p0 + i0);
+                a = make_uint4(v.x & m0, v.y & m0, v.z & m0, v.w & m0);
+                for (int t = 1; t < np; ++t) {
+                    const uint4 u = *reinterpret_cast<const uint4 *>(s.w + g.plane[t] * SLOTS + i0);
+                    const unsigned m = g.mask[t];
+                    a.x ^= u.x & m;
+                    a.y ^= u.y & m;
+                    a.z ^= u.z & m;
+                    a.w ^= u.w & m;
+                }
+            }
+            const unsigned b[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const bool on = (__popc(b[e]) & 1) != 0 && i0 + e < n;
+                const unsigned m = __ballot_sync(0xffffffffu, on);
+                if (on) queue[cnt + __popc(m & lt)] = (unsigned short)(i0 + e);
+                cnt += __popc(m);
+            }
+            __syncwarp();
+        }
+        // 32 queued slots at a time (the rest, too, once the scan is done)
+        while (cnt >= 32 || (!more && cnt > 0)) {
+            const int take = min(cnt, 32);
+            cnt -= take;
+            if (lane < take) out += rs_pair<NW, SLOTS, TAB, BATCH>(s, g, q, queue[cnt + lane], n, fresh, full, r);
+            __syncwarp();
+        }
+        if (!more) break;
+    }
+    return out;
+}
+
+// The strict filter over every live slot (terms whose values have not passed it yet);
+// returns the change of the live count.
+template <int NW, int SLOTS, int TAB, int T, bool BATCH>
+__device__ __forceinline__ int rs_filter(const ResidentSet<NW, SLOTS, TAB> &s, const RsParams &q, int n, long long r) {
+    int out = 0;
+    for (int i = threadIdx.x & (T - 1); i < n; i += T) {
+        const unsigned t = s.tag[i];
+        if (t & BB_DEAD) continue;
+        const Key32<NW> k = s.key(i);
+        if constexpr (BATCH) {
+            if (rs_instance<NW>(k, q, r) < 0) continue;
+        }
+        if (rs_drop<NW>(q, k, fabs(s.c[i]))) {
+            s.tag[i] = (unsigned short)(t | BB_DEAD);
+            out -= 1;
+        }
+    }
+    return out;
+}
+
+// A block of rotations [r0, r0 + K): the span of its deltas as a reduced basis
+// (basis[q] has bit piv[q], no other basis vector has it; piv ascending), and each
+// delta's coordinates (the bits at piv).
+struct BbPlan {
+    long long r0;
+    int K, d, full, kprev, cur, bits;
+    unsigned basis[BB_KMAX];
+    int piv[BB_KMAX];
+    int dl[BB_KMAX];
+};
+
+// Deltas of the generators [0, n): the bucket hash of each with all BK_ROWS rows (a
+// layout of 2^bits buckets uses the low bits).
+template <int NW>
+__global__ void k_bb_deltas(const GenRec *gens, long long n, const u64 *rows, unsigned *out) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        out[i] = bk_hash<NW>(gens[i].gz, gens[i].gx, rows, BK_ROWS);
+}
+
+// One block of rotations; input bucket set pl.cur, output set pl.cur ^ 1 (the input
+// stays intact, so a block that does not fit -- a coset beyond the resident set, or
+// an output bucket beyond BB_CAP -- is flagged and run again by the host, after a
+// split or with fewer rotations).  Persistent grid; every warp takes cosets of its
+// own, so no block barrier stands between a rotation and the next.
+template <int NW, bool BATCH>
+__global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_constant__ BkArgs A,
+                                                               const __grid_constant__ BbPlan pl) {
+    constexpr int SLOTS = bb_slots<NW>();
+    constexpr int TAB = BB_TAB;
+    static_assert(2 * 2 * BB_CAP <= SLOTS, "a block of one rotation always fits");
+    static_assert(!BATCH || NW == 2, "batched instances use two-word keys");
+    DevState *S = A.S;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    __shared__ RsGen<NW> s_g[BB_KMAX];
+    __shared__ int s_x[BB_MEMBERS];                        // a member's place in its coset
+    __shared__ int s_cw[BB_WARPS][BB_MEMBERS];
+    __shared__ unsigned short s_ow[BB_WARPS][BB_MEMBERS];
+    __shared__ int s_fw[BB_WARPS][2];                      // fresh slots of the step, resident set full
+    __shared__ int s_tot[BB_KMAX][2], s_np, s_mx, s_over, s_err, s_pref, s_bad;
+    extern __shared__ __align__(16) unsigned char bbm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    ResidentSet<NW, SLOTS, TAB> set;
+    unsigned char *mine = bbm + warp * rs_set_bytes<NW, SLOTS, TAB>();
+    set.c = reinterpret_cast<double *>(mine);
+    set.w = reinterpret_cast<unsigned *>(set.c + SLOTS);
+    set.tab = set.w + 4 * NW * SLOTS;
+    set.tag = reinterpret_cast<unsigned short *>(set.tab + TAB);
+    unsigned short *queue = reinterpret_cast<unsigned short *>(bbm + BB_WARPS * rs_set_bytes<NW, SLOTS, TAB>()) + warp * RS_QCAP;
+    int *scnt = s_cw[warp];
+    unsigned short *soff = s_ow[warp];
+    int *fresh = &s_fw[warp][0], *full = &s_fw[warp][1];
+    const int K = pl.K, d = pl.d, mem = 1 << d;
+    const long long r0 = pl.r0;
+    if (tid < K) {
+        rs_gen<NW>(&s_g[tid], A.gens[r0 + tid], pl.dl[tid]);
+        s_tot[tid][0] = s_tot[tid][1] = 0;
+    }
+    const int last_flags = A.gens[r0 + K - 1].flags;
+    if (tid == 0) { s_over = 0; s_bad = 0; s_mx = 0; s_np = 0; }
+    for (int m = tid; m < mem; m += 32 * BB_WARPS) {
+        unsigned b = 0;
+        for (int e = 0; e < d; ++e)
+            if ((m >> e) & 1) b ^= pl.basis[e];
+        s_x[m] = (int)b;
+    }
+    for (int i = lane; i < TAB / 4; i += 32) reinterpret_cast<uint4 *>(set.tab)[i] = make_uint4(0u, 0u, 0u, 0u);
+    const DevParams &P = *A.P;
+    RsParams q;
+    q.strict = fquick(P.strict);
+    q.strict_full = &P.strict;
+    q.local = &P.local;
+    q.local_on = P.local_active != 0;
+    q.bcos = A.bcos;
+    q.bsin = A.bsin;
+    q.bend = A.bend;
+    q.ninst = A.ninst;
+    q.ncol = A.ncol;
+    q.S = S;
+    const bool do_chan = (last_flags & GEN_CHANNEL) != 0 && P.chan_kind >= 0;
+    const int cur = pl.cur;
+    const int *CNT = cur ? A.cnt[1] : A.cnt[0];
+    int *OCNT = cur ? A.cnt[0] : A.cnt[1];
+    const u64 *Z = cur ? A.z[1] : A.z[0], *X = cur ? A.x[1] : A.x[0];
+    const double *C = cur ? A.c[1] : A.c[0];
+    u64 *OZ = cur ? A.z[0] : A.z[1], *OX = cur ? A.x[0] : A.x[1];
+    double *OC = cur ? A.c[0] : A.c[1];
+    // the previous block's outputs, records and error word are visible from here on
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (tid == 0) {
+        s_err = *(volatile int *)&S->err;
+        // the early-merge rule of spv_evolve.jl:356-362 up to r0, from the previous
+        // block's records (after a rotation every live value has passed the filter, so a
+        // rotation inside a block that starts with an early merge drops nothing by it)
+        const volatile BkRec *rec = A.rec;
+        const long long nin = (long long)rec[r0].n_out;
+        long long acap = rec[r0].acap;
+        if (pl.kprev > 0) {
+            const long long b = r0 - pl.kprev;
+            long long nr[BB_KMAX];
+#pragma unroll
+            for (int e = 1; e < BB_KMAX; ++e) nr[e] = e < pl.kprev ? (long long)rec[b + e].n_out : 0;
+            acap = rec[b + 1].acap;
+            const long long np = (long long)rec[b + 1].np;
+            if (rec[b + 1].pref && np > acap) acap = max(2 * acap, np);
+#pragma unroll
+            for (int e = 1; e < BB_KMAX; ++e)
+                if (nr[e] > acap) acap = 2 * acap > nr[e] ? 2 * acap : nr[e];
+        }
+        const int pref = nin > acap ? 1 : 0;
+        s_pref = pref;
+        if (blockIdx.x == 0) {
+            BkRec &me = A.rec[r0 + 1];
+            me.n_in = nin;
+            me.acap = acap;
+            me.pref = pref;
+            if (pref && !pl.full) me.np = (unsigned long long)nin;
+        }
+    }
+    __syncthreads();
+    if (s_err) return;
+    const bool drop_first = pl.full && s_pref;
+    const long long nb = 1ll << pl.bits;
+    if (pl.bits > A.bits_cap || d > pl.bits || d > BB_DMAX || K > BB_KMAX || r0 + K >= A.rec_len) {
+        if (tid == 0) flag_bounds(S, 1, ((long long)pl.bits << 16) | d);
+        return;
+    }
+    const long long ncos = nb >> d;
+    int tot_out = 0, tot_cre = 0;                          // lane j < K: rotation r0 + j
+    int tot_np = 0, mx = 0;
+    bool over = false;
+    for (long long cs = blockIdx.x * BB_WARPS + warp; cs < ncos; cs += (long long)gridDim.x * BB_WARPS) {
+        // ---- the coset's buckets and their places in the resident set
+        int total = 0;
+        unsigned rep = (unsigned)cs;                       // member m is bucket rep ^ s_x[m]
+        {
+            for (int e = 0; e < d; ++e) {
+                const int p = pl.piv[e];
+                rep = ((rep >> p) << (p + 1)) | (rep & ((1u << p) - 1u));
+            }
+            int nm[BB_MEMBERS / 32];
+#pragma unroll
+            for (int e = 0; e < BB_MEMBERS / 32; ++e) {
+                const int m = 32 * e + lane;
+                nm[e] = 0;
+                if (m < mem) {
+                    const unsigned b = rep ^ (unsigned)s_x[m];
+                    if (b < nb) nm[e] = __ldcg(CNT + b);
+                    else { flag_bounds(S, 3, b); s_bad = 1; }
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < BB_MEMBERS / 32; ++e) {
+                if (32 * e < mem) {
+                    if (nm[e] < 0 || nm[e] > BB_CAP) { flag_bounds(S, 4, nm[e]); s_bad = 1; nm[e] = 0; }
+                    const int inc = warp_incl_scan(nm[e], OpSum());
+                    const int m = 32 * e + lane;
+                    const int o = total + inc - nm[e];
+                    if (m < mem) {
+                        soff[m] = (unsigned short)o;
+                        scnt[m] = 0;
+                        if (o + nm[e] <= SLOTS)            // each slot's bucket
+                            for (int t = 0; t < nm[e]; ++t) set.tag[o + t] = (unsigned short)m;
+                    }
+                    total += __shfl_sync(0xffffffffu, inc, 31);
+                }
+            }
+            if (lane == 0) { *fresh = 0; *full = 0; }
+            __syncwarp();
+        }
+        if (total > SLOTS) { over = true; continue; }      // uniform
+        // ---- load and index, four terms a lane in flight
+        int dropped = 0;
+        for (int b0 = 0; b0 < total; b0 += 128) {
+            Key<NW> kk[4];
+            double cc[4];
+            int lb[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = b0 + u * 32 + lane;
+                if (i < total) {
+                    lb[u] = set.tag[i];
+                    const long long o = ((long long)(rep ^ (unsigned)s_x[lb[u]]) << BB_CAP_LOG) + (i - soff[lb[u]]);
+                    kk[u] = load_key_cg<NW>(Z, X, o);
+                    cc[u] = __ldcg(C + o);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = b0 + u * 32 + lane;
+                if (i < total) {
+                    const Key32<NW> k = key_narrow<NW>(kk[u]);
+                    bool dead = false;
+                    if (drop_first) {
+                        dead = rs_drop<NW>(q, k, fabs(cc[u]));
+                        if constexpr (BATCH) dead = dead && rs_instance<NW>(k, q, r0) >= 0;
+                    }
+                    dropped += dead ? 1 : 0;
+                    set.put(i, k, cc[u], (unsigned)lb[u] | (dead ? BB_DEAD : 0u));
+                    set.insert(i, rs_hash<NW>(k));
+                }
+            }
+        }
+        int alive = total;
+        if (drop_first) {
+            alive -= __reduce_add_sync(0xffffffffu, dropped);
+            tot_np += alive;
+        }
+        __syncwarp();
+        // ---- the K rotations
+        int n = total;
+        for (int j = 0; j < K; ++j) {
+            int out = rs_step<NW, SLOTS, TAB, 32, BATCH>(set, s_g[j], q, n, queue, fresh, full, r0 + j);
+            out = __reduce_add_sync(0xffffffffu, out);
+            __syncwarp();
+            n = min(n + *fresh, SLOTS);
+            __syncwarp();
+            if (lane == 0) *fresh = 0;
+            __syncwarp();
+            int dn = (int)(short)(out & 0xffff);
+            if (lane == j) tot_cre += (out - dn) >> 16;
+            if (j == 0 && pl.full) {
+                dn += __reduce_add_sync(0xffffffffu, rs_filter<NW, SLOTS, TAB, 32, BATCH>(set, q, n, r0));
+                __syncwarp();
+            }
+            alive += dn;
+            if (lane == j) tot_out += alive;
+        }
+        // ---- the survivors to their buckets of the output set, the index cleared
+        if (*full) {
+            over = true;
+        } else {
+            for (int base = 0; base < n; base += 32) {
+                const int i = base + lane;
+                const unsigned t = i < n ? set.tag[i] : BB_DEAD | 0x7fffu;
+                const bool live = !(t & BB_DEAD);
+                const int lb = (int)(t & 0xff);
+                const unsigned seg = bk_segment((int)(t & 0x7fffu), lane);
+                const int po = bk_claim(scnt, lb, live, seg, lane);
+                if (live && po < BB_CAP && lb < mem) {
+                    const Key<NW> kw = key_wide<NW>(set.key(i));
+                    double v = set.c[i];
+                    bool ch = do_chan;
+                    if constexpr (BATCH) ch = ch && rs_instance<NW>(set.key(i), q, r0 + K - 1) >= 0;
+                    if (ch) v = __dmul_rn(v, channel_factor<NW>(P, kw));
+                    const long long o = ((long long)(rep ^ (unsigned)s_x[lb]) << BB_CAP_LOG) + po;
+                    store_key<NW>(OZ, OX, o, kw);
+                    OC[o] = v;
+                }
+            }
+        }
+        for (int i = lane; i < TAB / 4; i += 32) reinterpret_cast<uint4 *>(set.tab)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncwarp();
+        for (int m = lane; m < mem; m += 32) {
+            const int c = scnt[m];
+            const unsigned b = rep ^ (unsigned)s_x[m];
+            if (b < nb) OCNT[b] = min(c, BB_CAP);
+            mx = max(mx, c);
+        }
+        __syncwarp();
+    }
+    // ---- the block's totals
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane < K) {
+        atomicAdd(&s_tot[lane][0], tot_out);
+        atomicAdd(&s_tot[lane][1], tot_cre);
+    }
+    if (lane == 0) {
+        atomicMax(&s_mx, mx);
+        atomicAdd(&s_np, tot_np);
+        if (over || mx > BB_CAP) atomicOr(&s_over, (over ? 2 : 0) | (mx > BB_CAP ? 1 : 0));
+    }
+    __syncthreads();
+    if (tid < K) {
+        atomicAdd(&A.rec[r0 + tid + 1].n_out, (unsigned long long)s_tot[tid][0]);
+        atomicAdd(&A.rec[r0 + tid + 1].created, (unsigned long long)s_tot[tid][1]);
+    }
+    if (tid == 0) {
+        if (drop_first) atomicAdd(&A.rec[r0 + 1].np, (unsigned long long)s_np);
+        atomicMax(&A.rec[r0 + K].maxcnt, s_mx);
+        if (s_over) {
+            atomicOr(&S->bk_pad, s_over);                  // 1: a bucket overflowed, 2: a coset beyond the resident set
+            atomicMin(&S->bk_fail, r0);
+            atomicOr(&S->err, ERR_OVERFLOW);
+        }
+        if (s_bad) atomicOr(&S->err, ERR_BOUNDS);
+    }
+}
+
+}  // namespace pp

@@ -1,4 +1,6 @@
-// Window-1 rotations over a hash-bucketed live set: one kernel per rotation.
+// The hash-bucketed live set: its layout, scatter and packing, and the one-rotation
+// kernel of key-sharded runs (kernels_block.cuh runs the rotations of an unsharded
+// vector, several per launch; a sharded run exchanges terms between rotations).
 //
 // A window-1 rotation (_rotate_range! + _merge_spv!, spv_kernels.jl:146-177,
 // 326-386, driven as in spv_evolve.jl:352-385) maps the live set {P} to
@@ -28,7 +30,7 @@
 // pre-filtered), the local filter on sin branches, the strict filter on the
 // unscaled sum, and the channel factor -- the same arithmetic, in the same
 // rounding steps, as the sorted-merge kernels.  The live set goes back to a
-// dense, sorted layout (gather + radix sort) when the call ends.
+// dense, sorted layout (packing and a sort) when the call ends.
 #pragma once
 #include "blockscan.cuh"
 
@@ -255,13 +257,7 @@ __device__ __forceinline__ void bk_pair(unsigned delta, long long p, int *b0, in
 // group: staged terms visible, key index built, outputs claimed.  k is the
 // rotation's index within the launched graph (rotation S->bk_rot0 + k, input set
 // (S->bk_cur0 + k) & 1).
-//
-// BATCH (two-word keys only): the live set holds many instances, instance i's
-// terms carrying i in z word 1, which no generator changes, so a term's partner
-// is in its own instance.  Each term rotates by its instance's angle column; a
-// term whose instance has ended is kept as it is (no rotation, no filter, no
-// channel) until it is harvested.
-template <int NW, int CAP, int ITEMS, bool BATCH = false>
+template <int NW, int CAP, int ITEMS>
 __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rotate(BkArgs A, int k) {
     constexpr int T = BK_THREADS;
     constexpr int SMI = T * ITEMS;                 // staged terms per area
@@ -271,7 +267,6 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
     static_assert(2 * CAP <= SMI, "a pair of full buckets fits");
     static_assert(NBK <= 32, "one warp handles a group's buckets");
     static_assert(SMI < 0x10000, "16-bit key index entries");
-    static_assert(!BATCH || NW == 2, "batched instances use two-word keys");
     DevState *S = A.S;
     // Launched as a programmatic dependent of the previous rotation: the next
     // rotation's CTAs may start as this one's finish.  Everything before
@@ -529,25 +524,10 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
                 double v = c;
                 Key<NW> qk;
                 double sg = 0.0;
-                double cvt = cv, svt = sv;
-                bool act = true;                                 // the term's instance is running
-                if constexpr (BATCH) {
-                    const u64 t = kk.z[NW - 1];
-                    if (t >= (u64)A.ninst) {
-                        flag_bounds(S, 11, (long long)t);
-                        act = false;
-                    } else if (r >= A.bend[t]) {
-                        act = false;
-                    } else {
-                        const long long ai = (long long)t * A.ncol + g.acol;
-                        cvt = A.bcos[ai];
-                        svt = A.bsin[ai];
-                    }
-                }
-                if (act && (tag & 0x20)) {
+                if (tag & 0x20) {
                     rotate_anti<NW>(kk, gk, &qk, &sg);
-                    v = __dmul_rn(c, cvt);
-                    const double s = __dmul_rn(sg * svt, c);     // (k - 2) * sin(theta) * c, spv_kernels.jl:163
+                    v = __dmul_rn(c, cv);
+                    const double s = __dmul_rn(sg * sv, c);     // (k - 2) * sin(theta) * c, spv_kernels.jl:163
                     const bool s_ok = !(local_on && should_drop<NW>(P.local, qk, fabs(s)));
                     cre += (s_ok && !fgn) ? 1 : 0;
                     const int j = find(qk);
@@ -557,7 +537,7 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
                         // the append.  Its phase factor is -sg: for Q = P xor G,
                         // k(P) + k(Q) = 2 (m1(P) + m1(Q) - ng) = 4 (m1(P) - popc(gx & gz & zP))
                         // (mod 4) in _rotate_range!'s k (spv_kernels.jl:162-163), and k is odd
-                        const double t = __dmul_rn(-(sg * svt), sc(a)[j]);
+                        const double t = __dmul_rn(-(sg * sv), sc(a)[j]);
                         if (!(local_on && should_drop<NW>(P.local, kk, fabs(t)))) v = __dadd_rn(v, t);
                     } else if (s_ok && (fgn || !remote) && !drop_q<NW>(fs, P.strict, qk, fabs(s))) {
                         // (a local term's sin branch belongs to the partner rank when remote)
@@ -567,9 +547,6 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
                 }
                 if (fgn) {
                     // a foreign term's own key belongs to the partner rank
-                } else if (!act) {
-                    oval = v;                                    // an ended instance is kept as it is
-                    own = true;
                 } else if (!drop_q<NW>(fs, P.strict, kk, fabs(v))) {
                     oval = do_chan ? __dmul_rn(v, channel_factor<NW>(P, kk)) : v;
                     own = true;
@@ -711,18 +688,19 @@ __global__ void k_bk_begin(DevState *S, long long rot0, int cur0, int reset_fail
     if (reset_fail) S->bk_fail = 0x7fffffffffffffffll;
 }
 
-// Scatter into a bucket layout of capacity cap (counts zeroed beforehand).
+// Scatter into a bucket layout of capacity 2^cap_log (counts zeroed beforehand).
 // Source: a dense array of n terms (scnt == nullptr) or a bucket layout of
 // 2^sbits buckets.  The largest destination count is recorded in *maxcnt; a
 // full bucket sets ERR_OVERFLOW in *err (the caller retries with more buckets).
 template <int NW>
 __global__ void k_bk_scatter(const u64 *SZ, const u64 *SX, const double *SC, long long n, const int *scnt, int sbits,
-                             u64 *DZ, u64 *DX, double *DC, int *dcnt, int dbits, int cap, const u64 *rows,
+                             u64 *DZ, u64 *DX, double *DC, int *dcnt, int dbits, int cap_log, const u64 *rows,
                              int *maxcnt, int *err) {
+    const int cap = 1 << cap_log;
     const long long slots = scnt ? ((long long)cap << sbits) : n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < slots;
          i += (long long)gridDim.x * blockDim.x) {
-        if (scnt && (int)(i % cap) >= scnt[i / cap]) continue;
+        if (scnt && (int)(i & (cap - 1)) >= scnt[i >> cap_log]) continue;
         const Key<NW> kk = load_key<NW>(SZ, SX, i);
         const unsigned b = bk_hash<NW>(kk.z, kk.x, rows, dbits);
         if (b >= (1u << dbits)) {
@@ -734,47 +712,48 @@ __global__ void k_bk_scatter(const u64 *SZ, const u64 *SX, const double *SC, lon
             atomicOr(err, ERR_OVERFLOW);
             continue;
         }
-        const long long o = (long long)b * cap + pos;
+        const long long o = ((long long)b << cap_log) + pos;
         store_key<NW>(DZ, DX, o, kk);
         DC[o] = SC[i];
         atomicMax(maxcnt, pos + 1);
     }
 }
 
-// Exclusive scan of the bucket counts into dense offsets (one CTA), total in
-// off[nb]; counts above cap are clipped (a flagged overflow leaves them so).
-constexpr int BKS_THREADS = 1024;
-__global__ void __launch_bounds__(BKS_THREADS) k_bk_offsets(const int *cnt, int nb, int cap, long long *off) {
-    __shared__ long long sm[BKS_THREADS / 32 + 1];
-    const int per = (nb + BKS_THREADS - 1) / BKS_THREADS;
-    const int t0 = min((int)threadIdx.x * per, nb), t1 = min(t0 + per, nb);
-    long long loc = 0;
-    for (int b = t0; b < t1; ++b) loc += min(cnt[b], cap);
-    long long total;
-    long long run = block_excl_scan<BKS_THREADS>(loc, 0ll, OpSum(), sm, &total);
-    for (int b = t0; b < t1; ++b) { off[b] = run; run += min(cnt[b], cap); }
-    if (threadIdx.x == 0) off[nb] = total;
-}
-
-// Gather of a bucket layout into a dense array (one warp per bucket).
+// A bucket layout's terms into a dense array, in no particular order (a CTA takes its
+// 256 buckets' range from one atomic); more than dcap terms are flagged.
 template <int NW>
-__global__ void k_bk_gather(const u64 *SZ, const u64 *SX, const double *SC, const int *cnt, int nb, int cap,
-                            const long long *off, u64 *DZ, u64 *DX, double *DC, long long dcap, DevState *S) {
-    const int lane = threadIdx.x & 31;
-    const long long w0 = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long b = w0; b < nb; b += nw) {
-        const int m = min(cnt[b], cap);
-        const long long o = off[b];
-        if (o < 0 || o + m > dcap) {
-            if (lane == 0) flag_bounds(S, 9, o);
-            continue;
+__global__ void __launch_bounds__(256) k_bk_pack(const u64 *SZ, const u64 *SX, const double *SC, const int *cnt, int nb,
+                                                 int cap_log, unsigned long long *total, u64 *DZ, u64 *DX, double *DC,
+                                                 long long dcap, DevState *S) {
+    __shared__ int sm[256 / 32 + 1];
+    __shared__ int s_off[257];
+    __shared__ unsigned long long s_base;
+    const int tid = threadIdx.x;
+    const int b0 = blockIdx.x * 256;
+    int m = b0 + tid < nb ? cnt[b0 + tid] : 0;
+    m = min(max(m, 0), 1 << cap_log);
+    int tot;
+    const int off = block_excl_scan<256>(m, 0, OpSum(), sm, &tot);
+    s_off[tid] = off;
+    if (tid == 0) {
+        s_off[256] = tot;
+        s_base = tot ? atomicAdd(total, (unsigned long long)tot) : 0ull;
+    }
+    __syncthreads();
+    if ((long long)s_base + tot > dcap) {
+        if (tid == 0) flag_bounds(S, 9, (long long)s_base);
+        return;
+    }
+    for (int i = tid; i < tot; i += 256) {
+        int lo = 0, hi = 255;                                     // the last bucket that starts at or before i
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_off[mid] <= i) lo = mid;
+            else hi = mid - 1;
         }
-        for (int j = lane; j < m; j += 32) {
-            const long long s = b * cap + j;
-            store_key<NW>(DZ, DX, o + j, load_key<NW>(SZ, SX, s));
-            DC[o + j] = SC[s];
-        }
+        const long long s = ((long long)(b0 + lo) << cap_log) + (i - s_off[lo]), o = (long long)s_base + i;
+        store_key<NW>(DZ, DX, o, load_key<NW>(SZ, SX, s));
+        DC[o] = SC[s];
     }
 }
 

@@ -29,6 +29,7 @@
 #include "kernels_small.cuh"
 #include "kernels_bucket.cuh"
 #include "kernels_block.cuh"
+#include "kernels_sort.cuh"
 
 using namespace pp;
 
@@ -148,6 +149,10 @@ struct pp_spv {
     u64 *bk_rows = nullptr;
     BkRec *bk_rec = nullptr;
     long long bk_rec_cap = 0;
+    u64 *ss_z = nullptr, *ss_x = nullptr, *ss_ws = nullptr;   // sample sort: bucketed records, samples
+    double *ss_c = nullptr;
+    unsigned *ss_p = nullptr;
+    long long ss_cap = 0;
     int *bk_aux = nullptr;                  // [0] largest scatter count, [1] scatter error bits
     pp_tuning tune = {BK_DEFAULT_CAP, BK_DEFAULT_ITEMS, 6, 128};  // pp_set_tuning
     struct { int occ1 = 1, occ2 = 1; } bk_occ[8];        // resident CTAs per SM of each variant
@@ -580,6 +585,8 @@ static int launch_setup(pp_spv *h) {
     CU(cudaFuncSetAttribute(k_tilescan<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tilescan_smem<NW>()));
     CU(cudaFuncSetAttribute(k_merge<NW, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)merge_smem_bytes<NW>()));
     CU(cudaFuncSetAttribute(k_merge<NW, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)merge_smem_bytes<NW>()));
+    CU(cudaFuncSetAttribute(k_ss_scatter<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ss_scatter_smem<NW>(SS_MAXB)));
+    CU(cudaFuncSetAttribute(k_ss_sort<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ss_sort_smem<NW>(SS_CAP)));
     CU(cudaFuncSetAttribute(k_small_run<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small_smem<NW>()));
     if (NW == 2) {
         // two merge CTAs per SM need the largest shared-memory carveout (2 x 113 KB);
@@ -630,12 +637,91 @@ static int radix_reserve(pp_spv *h, long long n) {
     return PP_OK;
 }
 
-// Stable LSD radix sort of n records in set A (za, xa, ca) using set T as the
-// ping-pong partner.  *in_t = 1 if the result ended in T.
+// Plan of a sample sort of n records.
+struct SsPlan {
+    int nbk, os, S, cap;
+};
+static SsPlan ss_plan(long long n) {
+    SsPlan p;
+    // buckets of about 600 records; above 1024 buckets, samples are fewer and buckets may get larger
+    p.nbk = (int)std::min((n + 599) / 600, (long long)SS_MAXB);
+    if (p.nbk > 1024 && n <= 1024ll * 1300) p.nbk = 1024;
+    p.os = p.nbk > 1024 ? 4 : 8;
+    p.S = p.nbk * p.os;
+    p.cap = n <= 700ll * p.nbk && p.os == 8 ? SS_CAP / 2 : SS_CAP;
+    return p;
+}
+
+// Workspaces of a sample sort of n records; false when it is not for this size or
+// device memory is short (the digit sort needs none of them).
+template <int NW>
+static bool ss_reserve(pp_spv *h, long long n) {
+    if (n > SS_MAX) return false;
+    if (n <= SS_CAP) return true;
+    const SsPlan p = ss_plan(n);
+    const long long need = (long long)p.nbk * p.cap;
+    if (need > h->ss_cap) {
+        size_t freeb = 0, totalb = 0;
+        if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess &&
+            (double)need * (16 * NW + 12) + 4.0 * (1ull << 30) > (double)freeb)
+            return false;
+        h->ss_cap = 0;
+        if (dalloc(h, &h->ss_z, need * NW) || dalloc(h, &h->ss_x, need * NW) || dalloc(h, &h->ss_c, need) ||
+            dalloc(h, &h->ss_p, need))
+            return false;
+        h->ss_cap = need;
+    }
+    if (!h->ss_ws) {
+        // sample keys, splitter keys; positions of both, ranks, bucket counts, overflow flag
+        const long long words = 2ll * NW * (SS_SAMPLES + SS_MAXB) + (3ll * SS_MAXB + 2 * SS_SAMPLES + 8) / 2;
+        if (dalloc(h, &h->ss_ws, words)) return false;
+    }
+    return true;
+}
+
+// Stable sample sort of n records in place; *ok = false when a bucket overflowed (the
+// records are as they were).
+template <int NW>
+static int ss_sort(pp_spv *h, u64 *z, u64 *x, double *c, long long n, bool *ok) {
+    cudaStream_t s = h->stream;
+    *ok = true;
+    if (n <= SS_CAP) {
+        const int cap = n <= 1024 ? 1024 : SS_CAP;
+        k_ss_sort<NW><<<1, SSS_THREADS, ss_sort_smem<NW>(cap), s>>>(z, x, c, nullptr, nullptr, (int)n, cap, nullptr, z, x, c, n);
+        return sync_check(h);
+    }
+    const SsPlan p = ss_plan(n);
+    Key<NW> *key = reinterpret_cast<Key<NW> *>(h->ss_ws), *skey = key + SS_SAMPLES;
+    unsigned *pos = reinterpret_cast<unsigned *>(skey + SS_MAXB), *spos = pos + SS_SAMPLES;
+    int *rank = reinterpret_cast<int *>(spos + SS_MAXB), *cnt = rank + SS_SAMPLES, *over = cnt + SS_MAXB;
+    k_ss_sample<NW><<<(p.S + 255) / 256, 256, 0, s>>>(z, x, n, p.S, key, pos, rank, cnt, p.nbk, over);
+    const int rb = (p.S + SSR - 1) / SSR;
+    k_ss_rank<NW><<<dim3(rb, rb), SSR, 0, s>>>(key, pos, p.S, rank);
+    k_ss_split<NW><<<rb, SSR, 0, s>>>(key, pos, rank, p.S, p.os, p.nbk, skey, spos);
+    const long long per = SS_THREADS * SS_ITEMS;
+    k_ss_scatter<NW><<<(int)((n + per - 1) / per), SS_THREADS, ss_scatter_smem<NW>(p.nbk), s>>>(
+        z, x, c, n, skey, spos, p.nbk, cnt, h->ss_z, h->ss_x, h->ss_c, h->ss_p, p.cap, over);
+    k_ss_sort<NW><<<p.nbk, SSS_THREADS, ss_sort_smem<NW>(p.cap), s>>>(h->ss_z, h->ss_x, h->ss_c, h->ss_p, cnt, 0, p.cap, over,
+                                                                     z, x, c, n);
+    int o = 0;
+    CU(cudaMemcpyAsync(&o, over, sizeof o, cudaMemcpyDeviceToHost, s));
+    TRY(sync_check(h));
+    *ok = o == 0;
+    return PP_OK;
+}
+
+// Stable sort of n records in set A (za, xa, ca): the sample sort up to SS_MAX records,
+// else an LSD radix sort with set T as the ping-pong partner.  *in_t = 1 if the result
+// ended in T.
 template <int NW>
 static int radix_sort(pp_spv *h, u64 *za, u64 *xa, double *ca, u64 *zt, u64 *xt, double *ct, long long n, int *in_t) {
     *in_t = 0;
     if (n <= 1) return PP_OK;
+    if (ss_reserve<NW>(h, n)) {
+        bool ok = false;
+        TRY(ss_sort<NW>(h, za, xa, ca, n, &ok));
+        if (ok) return PP_OK;
+    }
     cudaStream_t s = h->stream;
     u64 init[8] = {0, 0, 0, 0, ~0ull, ~0ull, ~0ull, ~0ull};
     CU(cudaMemcpyAsync(h->orand, init, sizeof init, cudaMemcpyHostToDevice, s));
@@ -725,7 +811,7 @@ extern "C" int pp_destroy(pp_spv *h) {
     for (void *p : ptrs) if (p) cudaFree(p);
     for (int i = 0; i < 3; ++i) if (h->gexec[i]) cudaGraphExecDestroy(h->gexec[i]);
     void *bptrs[] = {h->bkz[0], h->bkz[1], h->bkx[0], h->bkx[1], h->bkc[0], h->bkc[1], h->bkcnt[0], h->bkcnt[1],
-                     h->bk_rows, h->bk_rec, h->bk_aux, h->bk_delta, h->bkfcnt[0], h->bkfcnt[1], h->shard_cnt};
+                     h->bk_rows, h->bk_rec, h->bk_aux, h->bk_delta, h->ss_z, h->ss_x, h->ss_ws, h->ss_c, h->ss_p, h->bkfcnt[0], h->bkfcnt[1], h->shard_cnt};
     for (void *p : bptrs) if (p) cudaFree(p);
     if (h->Ph) cudaFreeHost(h->Ph);
     if (h->gens_h) cudaFreeHost(h->gens_h);
@@ -1110,7 +1196,7 @@ static int bk_to_dense(pp_spv *h, int cur, int bits, long long n) {
     const int nb = 1 << bits;
     cudaStream_t s = h->stream;
     PP_TRACE("buckets -> dense: %lld terms (2^%d buckets)", n, bits);
-    TRY(radix_reserve(h, n));
+    if (!ss_reserve<NW>(h, n)) TRY(radix_reserve(h, n));
     TRY(ensure_live(h, n + 1, false));
     unsigned long long *total = reinterpret_cast<unsigned long long *>(h->bk_aux);
     CU(cudaMemsetAsync(total, 0, sizeof *total, s));

@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -166,15 +167,112 @@ struct pp_spv {
     unsigned long long *shard_cnt = nullptr;
 };
 
+// ------------------------------------------------------------------ device memory
+// Device memory comes from a stream-ordered pool per device (cudaMallocFromPoolAsync),
+// shared by every handle of the process: an evolve of a copy, or a product into a new
+// vector, allocates and frees some fifty buffers, and cudaMalloc / cudaFree cost more
+// than the kernels between them (1.5e6 terms, nine rotations: 12 of 14 ms).  The pool
+// orders reuse between streams itself.  Memory it holds unused is bounded by POOL_KEEP
+// (checked whenever a handle frees a large part) and all returned when the last
+// handle is destroyed.
+static constexpr size_t POOL_KEEP = 4ull << 30;
+struct DevPool {
+    std::mutex mu;
+    cudaMemPool_t pool = nullptr;
+    long long handles = 0;                 // handles alive on the device
+    std::vector<cudaStream_t> streams;     // idle streams of destroyed handles (at most MAX_STREAMS)
+    bool setup[2] = {false, false};        // launch attributes and occupancies of each word count
+    int occ[2][4] = {};
+    static constexpr size_t MAX_STREAMS = 16;
+};
+static DevPool &dev_pool(int dev) {
+    static DevPool pools[64];
+    return pools[dev & 63];
+}
+
+static int pool_get(int dev, cudaMemPool_t *out) {
+    DevPool &d = dev_pool(dev);
+    std::lock_guard<std::mutex> lk(d.mu);
+    if (!d.pool) {
+        cudaMemPoolProps pr;
+        memset(&pr, 0, sizeof pr);
+        pr.allocType = cudaMemAllocationTypePinned;
+        pr.handleTypes = cudaMemHandleTypeNone;
+        pr.location.type = cudaMemLocationTypeDevice;
+        pr.location.id = dev;
+        CU(cudaMemPoolCreate(&d.pool, &pr));
+        unsigned long long keep = ~0ull;   // trimmed by pool_trim, not at every synchronisation
+        CU(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
+    *out = d.pool;
+    return PP_OK;
+}
+
+// Bytes the pool holds beyond what is in use.
+static size_t pool_unused(int dev) {
+    cudaMemPool_t pool = dev_pool(dev).pool;
+    unsigned long long res = 0, used = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &res) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return res > used ? (size_t)(res - used) : 0;
+}
+
+// Returns what the pool holds unused above keep bytes.
+static void pool_trim(int dev, size_t keep) {
+    cudaMemPool_t pool = dev_pool(dev).pool;
+    if (!pool) return;
+    const size_t un = pool_unused(dev);
+    if (un <= keep) return;
+    unsigned long long used = 0;
+    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+        cudaMemPoolTrimTo(pool, (size_t)used + keep);
+    cudaGetLastError();
+}
+
+// Free device memory, what the pool holds unused included.
+static bool dev_room(int dev, size_t *room) {
+    size_t freeb = 0, totalb = 0;
+    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) { cudaGetLastError(); return false; }
+    *room = freeb + pool_unused(dev);
+    return true;
+}
+
 // ------------------------------------------------------------------ helpers
 static void dfree(pp_spv *h, void *p) {
     if (!p) return;
     auto it = h->sizes.find(p);
+    size_t b = 0;
     if (it != h->sizes.end()) {
-        h->bytes -= (long long)it->second;
+        b = it->second;
+        h->bytes -= (long long)b;
         h->sizes.erase(it);
     }
-    cudaFree(p);
+    cudaFreeAsync(p, h->stream);
+    if (b >= (1ull << 28)) {               // (only memory whose free has run can be returned)
+        cudaStreamSynchronize(h->stream);
+        pool_trim(h->dev, POOL_KEEP);
+    }
+}
+
+// Memory of the pool for work on stream s; nullptr when the device has no more (after
+// one try with everything unused returned to it).
+static void *pool_alloc(int dev, size_t b, cudaStream_t s, cudaError_t *e) {
+    cudaMemPool_t pool = nullptr;
+    void *q = nullptr;
+    *e = cudaErrorMemoryAllocation;
+    if (pool_get(dev, &pool)) return nullptr;
+    *e = cudaMallocFromPoolAsync(&q, b, pool, s);
+    if (*e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaStreamSynchronize(s);
+        pool_trim(dev, 0);
+        *e = cudaMallocFromPoolAsync(&q, b, pool, s);
+    }
+    if (*e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return q;
 }
 
 // (Re)allocates *p for count elements.  The new buffer is allocated before the
@@ -192,13 +290,10 @@ static int dalloc(pp_spv *h, T **p, long long count) {
     if (count <= 0) count = 1;
     if (g_fail_alloc_after.load() > 0 && g_fail_alloc_after.fetch_sub(1) == 1)
         return fail(PP_OUT_OF_MEMORY, "cudaMalloc: injected allocation failure (pp_debug_fail_alloc)");
-    void *q = nullptr;
     const size_t b = (size_t)count * sizeof(T);
-    cudaError_t e = cudaMalloc(&q, b);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        return fail(PP_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-    }
+    cudaError_t e;
+    void *q = pool_alloc(h->dev, b, h->stream, &e);
+    if (!q) return fail(PP_OUT_OF_MEMORY, std::string("device allocation: ") + cudaGetErrorString(e));
     dfree(h, *p);
     *p = (T *)q;
     h->sizes[q] = b;
@@ -311,9 +406,10 @@ static int grow_live(pp_spv *h, long long need, bool preserve = true, long long 
     // refuse a growth that would leave less than 4 GiB of device memory free; when
     // the doubled capacity does not fit, step down towards the capacity needed
     {
-        size_t freeb = 0, totalb = 0;
-        if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess) {
-            const double per = 2.0 * (2 * h->NW * 8 + 8) + 12.0 + 4.0 * TAU_MAX * 2.0 / SEG;
+        // (no question where the pool holds enough: the growth takes no more of the device)
+        size_t freeb = 0;
+        const double per = 2.0 * (2 * h->NW * 8 + 8) + 12.0 + 4.0 * TAU_MAX * 2.0 / SEG;
+        if (1.25 * (double)newcap * per > (double)pool_unused(h->dev) && dev_room(h->dev, &freeb)) {
             const double room = (double)freeb - 4.0 * (1ull << 30);
             while ((double)newcap * per > room && newcap > need) newcap = std::max(need, newcap - newcap / 4);
             if ((double)newcap * per > room)
@@ -562,13 +658,13 @@ static int make_gen(const pp_spv *h, const u64 *gz, const u64 *gx, double cv, do
     g->ng = ng;
     int k = 0;
     bool ok = true;
-    for (int lvl = 128 * h->NW - 1; lvl >= 0; --lvl) {
-        int bit;
-        if (lvl >= 64 * h->NW) { int l = lvl - 64 * h->NW; bit = (int)((g->gz[l >> 6] >> (l & 63)) & 1); }
-        else bit = (int)((g->gx[lvl >> 6] >> (lvl & 63)) & 1);
-        if (!bit) continue;
-        if (k < KMAX) g->level[k] = (short)lvl;
-        ++k;
+    for (int w = 2 * h->NW - 1; w >= 0; --w) {                       // z words, then x words, each from its top bit
+        for (u64 v = w >= h->NW ? g->gz[w - h->NW] : g->gx[w]; v;) {
+            const int b = 63 - __builtin_clzll(v);
+            v ^= 1ull << b;
+            if (k < KMAX) g->level[k] = (short)(64 * w + b);
+            ++k;
+        }
     }
     if (k > KMAX) { ok = false; k = KMAX; }
     g->k = k;
@@ -579,6 +675,11 @@ static int make_gen(const pp_spv *h, const u64 *gz, const u64 *gx, double cv, do
 // ------------------------------------------------------------------ launches
 template <int NW>
 static int launch_setup(pp_spv *h) {
+    // the same for every handle of the device: asked once
+    DevPool &dp = dev_pool(h->dev);
+    std::lock_guard<std::mutex> lk(dp.mu);
+    int *oc = dp.occ[NW - 1];
+    if (!dp.setup[NW - 1]) {
     CU(cudaFuncSetAttribute(k_classify<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)(2 * NW * A_TILE * 8 + A_TILE)));
     CU(cudaFuncSetAttribute(k_merge<NW, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)merge_smem_bytes<NW>()));
@@ -598,13 +699,16 @@ static int launch_setup(pp_spv *h) {
     }
     int occ = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_classify<NW>, A_THREADS, 2 * NW * A_TILE * 8 + A_TILE));
-    h->occA1 = std::max(1, occ);
+    oc[0] = std::max(1, occ);
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_permute<NW>, A_THREADS, 0));
-    h->occA3 = std::max(1, occ);
+    oc[1] = std::max(1, occ);
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_merge<NW, 0>, B_THREADS, merge_smem_bytes<NW>()));
-    h->occB = std::max(1, occ);
+    oc[2] = std::max(1, occ);
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rotate_general<NW>, G_THREADS, 0));
-    h->occG = std::max(1, occ);
+    oc[3] = std::max(1, occ);
+    dp.setup[NW - 1] = true;
+    }
+    h->occA1 = oc[0]; h->occA3 = oc[1]; h->occB = oc[2]; h->occG = oc[3];
     return PP_OK;
 }
 
@@ -661,10 +765,8 @@ static bool ss_reserve(pp_spv *h, long long n) {
     const SsPlan p = ss_plan(n);
     const long long need = (long long)p.nbk * p.cap;
     if (need > h->ss_cap) {
-        size_t freeb = 0, totalb = 0;
-        if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess &&
-            (double)need * (16 * NW + 12) + 4.0 * (1ull << 30) > (double)freeb)
-            return false;
+        size_t freeb = 0;
+        if (dev_room(h->dev, &freeb) && (double)need * (16 * NW + 12) + 4.0 * (1ull << 30) > (double)freeb) return false;
         h->ss_cap = 0;
         if (dalloc(h, &h->ss_z, need * NW) || dalloc(h, &h->ss_x, need * NW) || dalloc(h, &h->ss_c, need) ||
             dalloc(h, &h->ss_p, need))
@@ -774,8 +876,19 @@ extern "C" int pp_create(int32_t N, int64_t live_cap, int64_t append_cap, pp_spv
     cudaError_t e = cudaGetDevice(&h->dev);
     if (e != cudaSuccess) { g_err = std::string("no CUDA device: ") + cudaGetErrorString(e); delete h; return PP_DEVICE_ERROR; }
     cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, h->dev);
-    e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    if (e != cudaSuccess) { g_err = cudaGetErrorString(e); delete h; return PP_DEVICE_ERROR; }
+    {
+        DevPool &dp = dev_pool(h->dev);
+        std::lock_guard<std::mutex> lk(dp.mu);
+        dp.handles += 1;
+        if (!dp.streams.empty()) {
+            h->stream = dp.streams.back();
+            dp.streams.pop_back();
+        }
+    }
+    if (!h->stream) {
+        e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
+        if (e != cudaSuccess) { h->stream = nullptr; return bail(fail(PP_DEVICE_ERROR, cudaGetErrorString(e))); }
+    }
     int r = h->NW == 1 ? launch_setup<1>(h) : launch_setup<2>(h);
     if (r) return bail(r);
     if ((r = dalloc(h, &h->S, 1))) return bail(r);
@@ -803,20 +916,32 @@ extern "C" int pp_create(int32_t N, int64_t live_cap, int64_t append_cap, pp_spv
 extern "C" int pp_destroy(pp_spv *h) {
     if (!h) return PP_OK;
     if (h->stream) cudaStreamSynchronize(h->stream);
-    void *ptrs[] = {h->z[0], h->z[1], h->x[0], h->x[1], h->c[0], h->c[1], h->srcidx, h->src, h->meta, h->aggA,
-                    h->offA, h->hfirstA, h->fwdA, h->bwdA, h->split_i, h->split_j, h->tstat, h->gstat, h->part,
-                    h->az, h->ax, h->ac, h->tz, h->tx, h->tc, h->rhist, h->rsums, h->orand, h->epart, h->eout,
-                    h->S, h->P, h->gens, h->rec, h->sphys, h->soff, h->kcnt, h->split_k,
-                    h->bcos, h->bsin, h->bend, h->hfin, h->hpart, h->heout, h->hrange, h->hnout, h->sel64, h->vtmp};
-    for (void *p : ptrs) if (p) cudaFree(p);
     for (int i = 0; i < 3; ++i) if (h->gexec[i]) cudaGraphExecDestroy(h->gexec[i]);
-    void *bptrs[] = {h->bkz[0], h->bkz[1], h->bkx[0], h->bkx[1], h->bkc[0], h->bkc[1], h->bkcnt[0], h->bkcnt[1],
-                     h->bk_rows, h->bk_rec, h->bk_aux, h->bk_delta, h->ss_z, h->ss_x, h->ss_ws, h->ss_c, h->ss_p, h->bkfcnt[0], h->bkfcnt[1], h->shard_cnt};
-    for (void *p : bptrs) if (p) cudaFree(p);
+    std::vector<void *> live;              // every device buffer of the handle
+    live.reserve(h->sizes.size());
+    for (auto &kv : h->sizes) live.push_back(kv.first);
+    for (void *p : live) cudaFreeAsync(p, h->stream);
+    if (h->bytes >= (1ll << 28)) cudaStreamSynchronize(h->stream);   // (freed memory can be returned then)
     if (h->Ph) cudaFreeHost(h->Ph);
     if (h->gens_h) cudaFreeHost(h->gens_h);
     if (h->bk_stat) cudaFreeHost(h->bk_stat);
-    if (h->stream) cudaStreamDestroy(h->stream);
+    {
+        // the stream goes to the next handle; unused memory beyond the pool's bound, or all
+        // of it with the last handle, goes back to the device
+        DevPool &dp = dev_pool(h->dev);
+        bool last;
+        {
+            std::lock_guard<std::mutex> lk(dp.mu);
+            last = --dp.handles == 0;
+            if (h->stream && dp.streams.size() < DevPool::MAX_STREAMS) {
+                dp.streams.push_back(h->stream);
+                h->stream = nullptr;
+            }
+        }
+        if (h->stream) cudaStreamDestroy(h->stream);
+        if (last) cudaDeviceSynchronize();
+        pool_trim(h->dev, last ? 0 : POOL_KEEP);
+    }
     delete h;
     return PP_OK;
 }
@@ -889,6 +1014,8 @@ extern "C" int pp_copy(pp_spv *h, pp_spv **out) {
     so.acap_logical = st.acap_logical;
     so.seg_dense = 1;
     int r = write_state(o, &so);
+    // h may free or rewrite its buffers on its own stream from here on
+    if (!r) r = sync_check(o);
     if (r) { pp_destroy(o); return r; }
     *out = o;
     return PP_OK;
@@ -1108,8 +1235,8 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
     // terms before the next split) back to a dense sorted set, plus 4 GiB; one
     // split of headroom (2^(bits+1) buckets) when that fits, else 2^bits
     auto fits = [&](long long sl) {
-        size_t freeb = 0, totalb = 0;
-        if (cudaMemGetInfo(&freeb, &totalb) == cudaSuccess) {
+        size_t freeb = 0;
+        if (dev_room(h->dev, &freeb)) {
             const double B = 16.0 * NW + 8.0;
             if (3.5 * (double)sl * B + 4.0 * (1ull << 30) > (double)freeb) return false;
         }
@@ -1815,17 +1942,18 @@ static int variance_dev(pp_spv *h, const u64 *ket, double *out) {
     return h->NW == 1 ? variance_nw<1>(h, ket, out) : variance_nw<2>(h, ket, out);
 }
 
-// Device scratch of one stochastic truncation call (freed on return).
+// Device scratch of one call on the handle's stream (freed on return).
 struct Scratch {
+    pp_spv *h;
     std::vector<void *> p;
-    ~Scratch() { for (void *q : p) cudaFree(q); }
+    explicit Scratch(pp_spv *h_) : h(h_) {}
+    Scratch(const Scratch &) = delete;
+    ~Scratch() { for (void *q : p) cudaFreeAsync(q, h->stream); }
     template <typename T>
     int get(T **out, long long count) {
-        void *q = nullptr;
-        if (cudaMalloc(&q, (size_t)std::max(1ll, count) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            return fail(PP_OUT_OF_MEMORY, "cudaMalloc (scratch buffer)");
-        }
+        cudaError_t e;
+        void *q = pool_alloc(h->dev, (size_t)std::max(1ll, count) * sizeof(T), h->stream, &e);
+        if (!q) return fail(PP_OUT_OF_MEMORY, "device allocation (scratch buffer)");
         p.push_back(q);
         *out = (T *)q;
         return PP_OK;
@@ -1864,7 +1992,7 @@ static int stoch_clip_apply(pp_spv *h, double eps, unsigned long long seed) {
     TRY(read_state(h, &st));
     const long long n = st.n;
     if (n == 0) return PP_OK;
-    Scratch sc;
+    Scratch sc(h);
     unsigned char *keep;
     double *nc;
     TRY(sc.get(&keep, n));
@@ -1881,7 +2009,7 @@ static int stoch_sample_apply(pp_spv *h, long long n_keep, unsigned long long se
     TRY(read_state(h, &st));
     const long long n = st.n;
     if (n <= n_keep) return PP_OK;
-    Scratch sc;
+    Scratch sc(h);
     unsigned long long *key;
     unsigned char *keep, *keyeq;
     int *tcnt, *toff;
@@ -3203,7 +3331,7 @@ extern "C" int pp_learned_truncate(pp_spv *h, pp_mlp *m, const pp_feature_ctx *c
     k_sel_scan<<<1, 1024, 0, s>>>(ntiles, m->sel, m->cgt, m->ceq, m->tie_off, m->out_off, m->total);
     k_sel_write<<<g, SL_THREADS, 0, s>>>(m->score, n, m->sel, m->tie_off, m->out_off, h->z[cur], h->x[cur], h->c[cur],
                                          h->z[cur ^ 1], h->x[cur ^ 1], h->c[cur ^ 1]);
-    Scratch sample_buf;             // the drop sample's device buffer, freed on every return
+    Scratch sample_buf(h);          // the drop sample's device buffer, freed on every return
     u64 *sbuf = nullptr;
     unsigned long long *scnt = nullptr;
     long long scap = sample ? sample->cap : 0;
@@ -3367,7 +3495,7 @@ extern "C" int pp_norm(pp_spv *h, double p, double *out) {
     TRY(read_state(h, &st));
     *out = 0.0;
     if (st.n == 0) return PP_OK;
-    Scratch sc;
+    Scratch sc(h);
     const int nb = std::min(4096, h->nsm * 8);
     double *part, *res;
     TRY(sc.get(&part, nb));
@@ -3434,7 +3562,7 @@ extern "C" int pp_inner_product(pp_spv *a, pp_spv *b, double *out) {
     *out = 0.0;
     if (sa.n == 0 || sb.n == 0) return PP_OK;
     CU(cudaStreamSynchronize(b->stream));
-    Scratch sc;
+    Scratch sc(a);
     const int nb = std::min(4096, a->nsm * 8);
     double *val, *part, *res;
     TRY(sc.get(&val, sa.n));
@@ -3463,7 +3591,7 @@ static int product_nw(pp_spv *out, pp_spv *a, pp_spv *b, int kind) {
     CU(cudaStreamSynchronize(a->stream));
     CU(cudaStreamSynchronize(b->stream));
     TRY(ensure_append(out, std::max(tot, out->acap_phys), 0));
-    Scratch sc;
+    Scratch sc(out);
     unsigned char *keep;
     int *err;
     TRY(sc.get(&keep, tot));

@@ -1863,7 +1863,7 @@ static int expect_dev(pp_spv *h, const u64 *k, double *out) {
     const int nb = std::min(4096, h->nsm * 8);
     if (h->NW == 1) k_expect<1><<<nb, 256, 0, h->stream>>>(B, k[0], k[1], h->epart);
     else k_expect<2><<<nb, 256, 0, h->stream>>>(B, k[0], k[1], h->epart);
-    k_expect_final<<<1, 32, 0, h->stream>>>(h->epart, nb, h->eout);
+    k_expect_final<<<1, EF_THREADS, 0, h->stream>>>(h->epart, nb, h->eout);
     CU(cudaMemcpyAsync(out, h->eout, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     return sync_check(h);
 }
@@ -1875,28 +1875,34 @@ static int expect_dev(pp_spv *h, const u64 *k, double *out) {
 static int adaptive_apply(pp_spv *h, long long max_terms, double min_thresh) {
     DevState st;
     TRY(read_state(h, &st));
-    double thr = min_thresh;
-    if (st.n > max_terms) {
-        if (!h->sel64) TRY(dalloc(h, &h->sel64, 1));
-        Select64 s0;
-        memset(&s0, 0, sizeof s0);
-        s0.remaining = max_terms + 1;
-        CU(cudaMemcpyAsync(h->sel64, &s0, sizeof s0, cudaMemcpyHostToDevice, h->stream));
-        const double *C = h->c[st.cur];
-        for (int shift = 56; shift >= 0; shift -= 8) {
-            k_abs_hist<<<h->nsm * 4, 256, 0, h->stream>>>(C, st.n, h->sel64, shift);
-            k_sel64_pick<<<1, 32, 0, h->stream>>>(h->sel64, shift);
-        }
-        Select64 sf;
-        CU(cudaMemcpyAsync(&sf, h->sel64, sizeof sf, cudaMemcpyDeviceToHost, h->stream));
-        TRY(sync_check(h));
-        memcpy(&thr, &sf.prefix, sizeof thr);
-    }
     pp_filter f = NOFILTER_H;
-    f.thresh = thr;
-    compile_filter(&f, &h->Ph->clip);
-    TRY(upload_params(h));
-    TRY(read_state(h, &st));
+    if (st.n <= AS_MAX) {
+        // the threshold stays on the device
+        compile_filter(&f, &h->Ph->clip);
+        TRY(upload_params(h));
+        k_abs_select<<<1, AS_THREADS, 0, h->stream>>>(h->c[0], h->c[1], h->S, max_terms, min_thresh, &h->P->clip.thresh);
+    } else {
+        f.thresh = min_thresh;
+        if (st.n > max_terms) {
+            if (!h->sel64) TRY(dalloc(h, &h->sel64, 1));
+            Select64 s0;
+            memset(&s0, 0, sizeof s0);
+            s0.remaining = max_terms + 1;
+            CU(cudaMemcpyAsync(h->sel64, &s0, sizeof s0, cudaMemcpyHostToDevice, h->stream));
+            const double *C = h->c[st.cur];
+            for (int shift = 56; shift >= 0; shift -= 8) {
+                k_abs_hist<<<h->nsm * 4, 256, 0, h->stream>>>(C, st.n, h->sel64, shift);
+                k_sel64_pick<<<1, 256, 0, h->stream>>>(h->sel64, shift);
+            }
+            Select64 sf;
+            CU(cudaMemcpyAsync(&sf, h->sel64, sizeof sf, cudaMemcpyDeviceToHost, h->stream));
+            TRY(sync_check(h));
+            memcpy(&f.thresh, &sf.prefix, sizeof f.thresh);
+        }
+        compile_filter(&f, &h->Ph->clip);
+        TRY(upload_params(h));
+        TRY(read_state(h, &st));
+    }
     st.an = 0;
     TRY(write_state(h, &st));
     Bufs B = make_bufs(h);
@@ -1925,11 +1931,14 @@ static int variance_nw(pp_spv *h, const u64 *ket, double *out) {
     const u64 *RZ = in_t ? h->tz : h->az, *RX = in_t ? h->tx : h->ax;
     const double *RC = in_t ? h->tc : h->ac;
     double *gval = in_t ? h->ac : h->tc;
+    u64 *list = in_t ? h->az : h->tz;      // long runs (two words each, fewer than n / VG_SERIAL)
+    unsigned long long *nlist = reinterpret_cast<unsigned long long *>(h->vtmp + 1);
     CU(cudaMemsetAsync(h->vtmp, 0, 2 * sizeof(double), s));
-    k_var_groups<NW><<<h->nsm * 8, 256, 0, s>>>(RZ, RX, RC, n, gval, h->vtmp);
+    k_var_groups<NW><<<h->nsm * 8, 256, 0, s>>>(RZ, RX, RC, n, gval, h->vtmp, list, nlist);
+    k_var_long<NW><<<h->nsm * 2, 256, 0, s>>>(RZ, RX, RC, gval, h->vtmp, list, nlist);
     const int nb = std::min(4096, h->nsm * 8);
     k_sum_partials<<<nb, 256, 0, s>>>(gval, n, h->epart);
-    k_expect_final<<<1, 32, 0, s>>>(h->epart, nb, h->eout);
+    k_expect_final<<<1, EF_THREADS, 0, s>>>(h->epart, nb, h->eout);
     double e2 = 0.0, e1 = 0.0;
     CU(cudaMemcpyAsync(&e2, h->eout, sizeof(double), cudaMemcpyDeviceToHost, s));
     CU(cudaMemcpyAsync(&e1, h->vtmp, sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -2037,7 +2046,7 @@ static int stoch_sample_apply(pp_spv *h, long long n_keep, unsigned long long se
     CU(cudaMemcpyAsync(sel, &s0, sizeof s0, cudaMemcpyHostToDevice, s));
     for (int shift = 56; shift >= 0; shift -= 8) {
         k_key64_hist<<<h->nsm * 4, 256, 0, s>>>(key, n, sel, shift);
-        k_sel64_pick<<<1, 32, 0, s>>>(sel, shift);
+        k_sel64_pick<<<1, 256, 0, s>>>(sel, shift);
     }
     k_stoch_sample_mark<<<h->nsm * 8, 256, 0, s>>>(key, n, sel, keep, keyeq);
     const int g = (int)std::min<long long>(ntiles, 8ll * h->nsm);
@@ -2045,8 +2054,8 @@ static int stoch_sample_apply(pp_spv *h, long long n_keep, unsigned long long se
     k_flag_scan<<<1, 1024, 0, s>>>(ntiles, tcnt, toff, ttot);
     k_stoch_sample_ties<<<g, FC_THREADS, 0, s>>>(n, sel, keyeq, toff, keep);
     k_norm_partials<<<nb, 256, 0, s>>>(C, keep, n, pall, pkept);
-    k_expect_final<<<1, 32, 0, s>>>(pall, nb, nrm);
-    k_expect_final<<<1, 32, 0, s>>>(pkept, nb, nrm + 1);
+    k_expect_final<<<1, EF_THREADS, 0, s>>>(pall, nb, nrm);
+    k_expect_final<<<1, EF_THREADS, 0, s>>>(pkept, nb, nrm + 1);
     k_norm_scale<<<1, 32, 0, s>>>(nrm, nrm + 1, nrm + 2);
     return flag_compact(h, st, keep, nullptr, nrm + 2, sc);
 }
@@ -2402,7 +2411,7 @@ extern "C" int pp_expect_ket(pp_spv *h, const void *ket, double *out) {
     const int nb = std::min(4096, h->nsm * 8);
     if (h->NW == 1) k_expect<1><<<nb, 256, 0, h->stream>>>(B, k[0], k[1], h->epart);
     else k_expect<2><<<nb, 256, 0, h->stream>>>(B, k[0], k[1], h->epart);
-    k_expect_final<<<1, 32, 0, h->stream>>>(h->epart, nb, h->eout);
+    k_expect_final<<<1, EF_THREADS, 0, h->stream>>>(h->epart, nb, h->eout);
     CU(cudaMemcpyAsync(out, h->eout, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     return sync_check(h);
 }
@@ -3510,7 +3519,7 @@ extern "C" int pp_norm(pp_spv *h, double p, double *out) {
         TRY(sc.get(&val, st.n));
         k_norm_terms<<<h->nsm * 8, 256, 0, s>>>(C, st.n, p, val);
         k_sum_partials<<<nb, 256, 0, s>>>(val, st.n, part);
-        k_expect_final<<<1, 32, 0, s>>>(part, nb, res);
+        k_expect_final<<<1, EF_THREADS, 0, s>>>(part, nb, res);
     }
     double r = 0.0;
     CU(cudaMemcpyAsync(&r, res, sizeof r, cudaMemcpyDeviceToHost, s));
@@ -3576,7 +3585,7 @@ extern "C" int pp_inner_product(pp_spv *a, pp_spv *b, double *out) {
         k_inner_terms<2><<<a->nsm * 8, 256, 0, s>>>(a->z[sa.cur], a->x[sa.cur], a->c[sa.cur], sa.n, b->z[sb.cur],
                                                      b->x[sb.cur], b->c[sb.cur], sb.n, val);
     k_sum_partials<<<nb, 256, 0, s>>>(val, sa.n, part);
-    k_expect_final<<<1, 32, 0, s>>>(part, nb, res);
+    k_expect_final<<<1, EF_THREADS, 0, s>>>(part, nb, res);
     CU(cudaMemcpyAsync(out, res, sizeof(double), cudaMemcpyDeviceToHost, s));
     return sync_check(a);
 }

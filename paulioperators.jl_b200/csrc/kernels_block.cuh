@@ -64,34 +64,39 @@ struct RsGen {
     unsigned g[4 * NW];
     unsigned mask[4 * NW];
     int plane[4 * NW];
-    int np, ng, acol, delta;
+    int np, ng, acol, delta, flags;
 };
 
+// Made by one warp (all lanes), a lane per plane.
 template <int NW>
 __device__ __forceinline__ void rs_gen(RsGen<NW> *o, const GenRec &g, int delta) {
-    o->cosv = g.cosv;
-    o->sinv = g.sinv;
-    o->ng = g.ng;
-    o->acol = g.acol;
-    o->delta = delta;
-    int np = 0;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) {
-        o->g[2 * w] = (unsigned)g.gz[w];
-        o->g[2 * w + 1] = (unsigned)(g.gz[w] >> 32);
-        o->g[2 * NW + 2 * w] = (unsigned)g.gx[w];
-        o->g[2 * NW + 2 * w + 1] = (unsigned)(g.gx[w] >> 32);
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) {
+        o->cosv = g.cosv;
+        o->sinv = g.sinv;
+        o->ng = g.ng;
+        o->acol = g.acol;
+        o->delta = delta;
+        o->flags = g.flags;
     }
-    // parity of popc(gx & z) + popc(gz & x): only planes under a nonzero mask
-    for (int p = 0; p < 4 * NW; ++p) {
-        const unsigned m = o->g[p < 2 * NW ? p + 2 * NW : p - 2 * NW];
+    // plane p: the key's words z low to high, then x; its parity test (gx against z, gz
+    // against x) reads only planes under a nonzero mask
+    const int p = lane & (4 * NW - 1), q = p ^ (2 * NW);
+    auto word = [&](int t) {
+        const u64 v = t < 2 * NW ? g.gz[t >> 1] : g.gx[(t - 2 * NW) >> 1];
+        return t & 1 ? (unsigned)(v >> 32) : (unsigned)v;
+    };
+    const unsigned mine = word(p), m = word(q);
+    const unsigned on = __ballot_sync(0xffffffffu, lane < 4 * NW && m != 0);
+    if (lane < 4 * NW) {
+        o->g[p] = mine;
         if (m) {
-            o->plane[np] = p;
-            o->mask[np] = m;
-            ++np;
+            const int at = __popc(on & ((1u << lane) - 1u));
+            o->plane[at] = p;
+            o->mask[at] = m;
         }
     }
-    o->np = np;
+    if (lane == 0) o->np = __popc(on);
 }
 
 // load_key through L2 only: a bucket set is rewritten by every second launch, and a
@@ -230,21 +235,25 @@ __device__ __forceinline__ long long rs_instance(const Key32<NW> &k, const RsPar
     return r < q.bend[t] ? (long long)t : -1;
 }
 
-// should_drop (spv_kernels.jl:64-79) on a key in 32-bit words.
+// Weight and X-weight caps of the strict filter on a key in 32-bit words (the rest of
+// should_drop, spv_kernels.jl:64-79, is the coefficient's; a filter with other
+// criteria is evaluated in full).  Without branches: the two keys of a pair are tested
+// side by side, which a chain of short-circuit tests made 350 cycles of a step's 1,500.
+template <int NW>
+__device__ __forceinline__ bool rs_heavy(const RsParams &q, const Key32<NW> &k) {
+    int wt = 0, xw = 0;
+#pragma unroll
+    for (int t = 0; t < 2 * NW; ++t) {
+        wt += __popc(k.w[t] | k.w[2 * NW + t]);
+        xw += __popc(k.w[2 * NW + t]);
+    }
+    return (wt > q.strict.wmax) | (xw > q.strict.xwmax);
+}
+
 template <int NW>
 __device__ __forceinline__ bool rs_drop(const RsParams &q, const Key32<NW> &k, double absc) {
     if (q.strict.full) return should_drop<NW>(*q.strict_full, key_wide<NW>(k), absc);
-    int wt = 0;
-#pragma unroll
-    for (int t = 0; t < 2 * NW; ++t) wt += __popc(k.w[t] | k.w[2 * NW + t]);
-    bool drop = absc <= q.strict.thresh || wt > q.strict.wmax;
-    if (q.strict.xwmax < 64 * NW) {
-        int xw = 0;
-#pragma unroll
-        for (int t = 0; t < 2 * NW; ++t) xw += __popc(k.w[2 * NW + t]);
-        drop = drop || xw > q.strict.xwmax;
-    }
-    return drop;
+    return (absc <= q.strict.thresh) | rs_heavy<NW>(q, k);
 }
 
 // One rotation on one anticommuting slot i of the resident set.  Of two partners'
@@ -263,6 +272,16 @@ __device__ __forceinline__ int rs_pair(const ResidentSet<NW, SLOTS, TAB> &s, con
 #pragma unroll
     for (int t = 0; t < 4 * NW; ++t) p.w[t] = k.w[t] ^ g.g[t];
     const unsigned hp = rs_hash<NW>(p);
+    const bool hk = rs_heavy<NW>(q, k), hq = rs_heavy<NW>(q, p);
+    // phase of the sin branch of P (_rotate_range!, spv_kernels.jl:155-163); the
+    // partner's has the opposite sign: k(P) + k(P xor M) = 0 mod 4, and k is odd
+    int m1 = 0, nzp = 0, nzx = 0;
+#pragma unroll
+    for (int t = 0; t < 2 * NW; ++t) {
+        m1 += __popc(g.g[2 * NW + t] & k.w[t]);
+        nzp += __popc(p.w[t] & p.w[2 * NW + t]);
+        nzx += __popc(k.w[t] & k.w[2 * NW + t]);
+    }
     const int j = s.find(p, hp);
     const bool ai = !(ti & BB_DEAD);
     if (j >= 0 ? j < i : !ai) return 0;
@@ -277,16 +296,7 @@ __device__ __forceinline__ int rs_pair(const ResidentSet<NW, SLOTS, TAB> &s, con
         cv = q.bcos[t * q.ncol + g.acol];
         sv = q.bsin[t * q.ncol + g.acol];
     }
-    // phase of the sin branch of P (_rotate_range!, spv_kernels.jl:155-163); the
-    // partner's has the opposite sign: k(P) + k(P xor M) = 0 mod 4, and k is odd
-    int m1 = 0, nzp = 0, nzx = 0;
-#pragma unroll
-    for (int t = 0; t < 2 * NW; ++t) {
-        m1 += __popc(g.g[2 * NW + t] & k.w[t]);
-        nzp += __popc(p.w[t] & p.w[2 * NW + t]);
-        nzx += __popc(k.w[t] & k.w[2 * NW + t]);
-    }
-    const double sgs = (double)(((nzp - g.ng - nzx + 2 * m1) & 3) - 2) * sv;
+    const double sgs = (nzp - g.ng - nzx + 2 * m1) & 2 ? sv : -sv;      // (k - 2) sin, k = 1 or 3
     const double si = __dmul_rn(sgs, ci);                        // lands on P xor M
     const double sj = __dmul_rn(-sgs, cj);                       // lands on P
     bool oki = ai, okj = aj;
@@ -296,10 +306,17 @@ __device__ __forceinline__ int rs_pair(const ResidentSet<NW, SLOTS, TAB> &s, con
     }
     // live value first, then the append (_try_merge!)
     double vi = __dmul_rn(ci, cv), vj = __dmul_rn(cj, cv);
-    vi = ai ? (okj ? __dadd_rn(vi, sj) : vi) : sj;
-    vj = aj ? (oki ? __dadd_rn(vj, si) : vj) : si;
-    const bool ki = (ai || okj) && !rs_drop<NW>(q, k, fabs(vi));
-    const bool kj = (aj || oki) && !rs_drop<NW>(q, p, fabs(vj));
+    const double wi = __dadd_rn(vi, sj), wj = __dadd_rn(vj, si);
+    vi = ai ? (okj ? wi : vi) : sj;
+    vj = aj ? (oki ? wj : vj) : si;
+    bool ki = ai | okj, kj = aj | oki;
+    if (q.strict.full) {
+        ki = ki && !should_drop<NW>(*q.strict_full, key_wide<NW>(k), fabs(vi));
+        kj = kj && !should_drop<NW>(*q.strict_full, key_wide<NW>(p), fabs(vj));
+    } else {
+        ki &= !((fabs(vi) <= q.strict.thresh) | hk);
+        kj &= !((fabs(vj) <= q.strict.thresh) | hq);
+    }
     if (ki) s.c[i] = vi;
     if (ki != ai) s.tag[i] = (unsigned short)(ti ^ BB_DEAD);
     if (j >= 0) {
@@ -332,6 +349,15 @@ __device__ __forceinline__ int rs_step(const ResidentSet<NW, SLOTS, TAB> &s, con
     const unsigned lt = (1u << lane) - 1u;
     int cnt = 0, out = 0;
     const int np = g.np;
+    if constexpr (T > 32) {
+        if (n <= T) {                                   // a thread per slot: no queue in the chain
+            const int i = threadIdx.x;
+            unsigned a = 0;
+            if (i < n)
+                for (int t = 0; t < np; ++t) a ^= s.w[g.plane[t] * SLOTS + i] & g.mask[t];
+            return __popc(a) & 1 ? rs_pair<NW, SLOTS, TAB, BATCH>(s, g, q, i, n, fresh, full, r) : 0;
+        }
+    }
     const int p0 = g.plane[0] * SLOTS;
     const unsigned m0 = g.mask[0];
     for (int base = warp * 128;; base += (T / 32) * 128) {
@@ -446,10 +472,8 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     int *fresh = &s_fw[warp][0], *full = &s_fw[warp][1];
     const int K = pl.K, d = pl.d, mem = 1 << d;
     const long long r0 = pl.r0;
-    if (tid < K) {
-        rs_gen<NW>(&s_g[tid], A.gens[r0 + tid], pl.dl[tid]);
-        s_tot[tid][0] = s_tot[tid][1] = 0;
-    }
+    for (int j = warp; j < K; j += BB_WARPS) rs_gen<NW>(&s_g[j], A.gens[r0 + j], pl.dl[j]);
+    if (tid < K) s_tot[tid][0] = s_tot[tid][1] = 0;
     const int last_flags = A.gens[r0 + K - 1].flags;
     if (tid == 0) { s_over = 0; s_bad = 0; s_mx = 0; s_np = 0; }
     for (int m = tid; m < mem; m += 32 * BB_WARPS) {

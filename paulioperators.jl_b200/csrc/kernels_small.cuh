@@ -1,102 +1,96 @@
 // Window-1 rotations of a small live set in one CTA.  While the live set holds at
 // most small_cap<NW>() terms, one launch runs rotation after rotation with the
-// whole set in shared memory, instead of one grid-wide launch per rotation,
-// whose fixed latency dominates small sets.  It is the same sequence
+// whole set in shared memory, instead of a launch per block of rotations, whose
+// fixed latency dominates small sets.  It is the same sequence
 // (spv_evolve.jl:352-385, spv_kernels.jl:146-177, 326-386) with the same per-term
-// arithmetic, so results are bit-identical to the other paths.  As in the
-// bucketed kernel, an output key sums at most two terms (the live P and the sin
-// branch of its partner P xor M), so no order is needed between rotations:
-//   - early-merge pre-filter when n > acap (live terms failing the strict filter
-//     emit nothing and are dropped, counted in the early-merge rule);
-//   - the live terms that anticommute with G and survive the pre-filter are
-//     indexed in a shared-memory hash table (only they can be a partner);
-//   - per live term: cos branch, partner lookup, partner's sin branch added to
-//     the live value (its phase is -sg: k(P) + k(P xor M) = 0 mod 4), strict
-//     filter on the unscaled sum, channel; a sin branch whose partner is absent
-//     becomes a new term;
+// arithmetic (the resident set and its steps of kernels_block.cuh), so results are
+// bit-identical to the other paths:
+//   - the set and the index of its keys stay from rotation to rotation; a rotation
+//     touches the anticommuting terms only.  Dropped terms leave dead slots, and when
+//     the slots run out the live terms are moved together and indexed anew;
+//   - where values may not have passed the strict filter yet (the first rotation, and
+//     the one after a channel) it is applied to every term: before the rotation when
+//     it starts with an early merge (n > acap), else after it;
+//   - a channel scales every live term after its rotation;
 //   - counters and WindowCounters records as the other paths write them.
-// Three barriers per rotation.  The set is sorted once, when the launch ends
-// (bitonic over an index array; keys are distinct), and <ket|O|ket> of a
-// measured last rotation is reduced on the sorted set.  The launch stops when
-// the set outgrows small_cap or the call's rotations are done, and leaves the
-// live set dense and sorted in the other buffer set.  It does not handle local
-// truncation, corrections or batched instances; the host launches it only
-// without them.  No waits: every barrier is in uniform control flow, every loop
-// is bounded by the rotation count, the set size or the table size.
+// One barrier per rotation (two at a channel).  The set is sorted once, when the launch ends (bitonic
+// over an index array; keys are distinct), and <ket|O|ket> of a measured last rotation
+// is reduced on the sorted set.  The launch stops when the set outgrows small_cap or
+// the call's rotations are done, and leaves the live set dense and sorted in the other
+// buffer set.  It does not handle local truncation, corrections or batched instances;
+// the host launches it only without them.  No waits: every barrier is in uniform
+// control flow, every loop is bounded by the rotation count, the set size or the table
+// size.
+// Bound by the latency of a rotation's chain: parity test, index look-up, two products
+// and a sum, filter, barrier -- about 1,700 cycles at 170 terms.  Measured (one B200,
+// with a table and a copy of the set made anew every rotation before): 20-qubit chain,
+// 312 rotations of 170 terms on average, 458 -> 302 us of kernel; the first 1,444
+// rotations of a 127-qubit circuit 2.07 -> 1.15 ms.
 #pragma once
 #include "kernels_struct.cuh"
-#include "kernels_bucket.cuh"
+#include "kernels_block.cuh"
 
 namespace pp {
 
-constexpr int SM_THREADS = 256;                   // 1024 measured 9 % slower on chain20 (idle warps at barriers)
+constexpr int SM_THREADS = 512;                   // a thread per slot up to 512 (256: 6 % slower on a 20-qubit chain)
 
 template <int NW>
 __host__ __device__ constexpr int small_cap() { return NW == 1 ? 2048 : 1024; }
 
-// two term sets of 2C (the live set and the next one; a rotation at most doubles
-// the set), the key index (16-bit slots, 2C), pre-filter marks (2C) and the final
-// sort's index array (2C)
+// a resident set of 2C slots (a rotation at most doubles the set), the warps' queues
 template <int NW>
 constexpr size_t small_smem() {
-    constexpr size_t C = small_cap<NW>();
-    return 2 * (2 * C) * (2 * NW * 8 + 8) + 2 * C * 2 + 2 * C + 2 * C * 2;
-}
-
-template <int NW>
-__device__ __forceinline__ Key<NW> sm_key(const u64 *Z, const u64 *X, int stride, int i) {
-    Key<NW> k;
-#pragma unroll
-    for (int w = 0; w < NW; ++w) { k.z[w] = Z[w * stride + i]; k.x[w] = X[w * stride + i]; }
-    return k;
-}
-
-template <int NW>
-__device__ __forceinline__ void sm_put(u64 *Z, u64 *X, int stride, int i, const Key<NW> &k) {
-#pragma unroll
-    for (int w = 0; w < NW; ++w) { Z[w * stride + i] = k.z[w]; X[w * stride + i] = k.x[w]; }
+    constexpr int C = small_cap<NW>();
+    return rs_set_bytes<NW, 2 * C, 4 * C>() + (SM_THREADS / 32) * RS_QCAP * 2;
 }
 
 template <int NW>
 __global__ void __launch_bounds__(SM_THREADS, 1) k_small_run(Bufs B) {
     constexpr int C = small_cap<NW>();
-    constexpr int C2 = 2 * C;                      // capacity of each term set
-    constexpr int TAB = 2 * C;                     // key index slots
+    constexpr int SLOTS = 2 * C, TAB = 4 * C;
     constexpr int T = SM_THREADS;
+    static_assert(SLOTS < 0x8000, "slots in 16 bits");
     DevState *S = B.S;
-    __shared__ int s_go;
-    __shared__ int s_cnt[2][3];                    // per rotation parity: outputs, sin branches, pre-filtered
-    __shared__ double s_red[SM_THREADS / 32];
-    __shared__ double s_expw[130], s_expxw[130];
-    __shared__ __align__(16) GenRec gs[2];         // this rotation's generator and the next one (prefetched)
+    __shared__ int s_go, s_full;
+    __shared__ int s_cnt[3][3];                    // of rotation r in r % 3: fresh slots, change of the live count, sin branches
+    __shared__ int s_scan[T / 32 + 1];
+    __shared__ double s_red[T / 32];
+    __shared__ __align__(16) GenRec gs[2];         // generators on their way in (the last warp's)
+    __shared__ RsGen<NW> rg[3];                    // of this rotation and the next two, r % 3
     static_assert(sizeof(GenRec) % 16 == 0, "generator records copy in 16-byte pieces");
     constexpr int GQ = (int)(sizeof(GenRec) / 16);
-    extern __shared__ u64 sm[];
-    // term sets t = 0, 1: keys (NW words, stride C2) and coefficients
-    auto tz = [&](int t) { return sm + t * (2 * NW + 1) * C2; };
-    auto tx = [&](int t) { return sm + t * (2 * NW + 1) * C2 + NW * C2; };
-    auto tc = [&](int t) { return reinterpret_cast<double *>(sm + t * (2 * NW + 1) * C2 + 2 * NW * C2); };
-    unsigned short *tab = reinterpret_cast<unsigned short *>(sm + 2 * (2 * NW + 1) * C2);   // [TAB]
-    unsigned char *sdead = reinterpret_cast<unsigned char *>(tab + TAB);                   // [C2]
-    unsigned short *sa = reinterpret_cast<unsigned short *>(sdead + C2);                   // [C2]
+    extern __shared__ __align__(16) unsigned char smr[];
+    ResidentSet<NW, SLOTS, TAB> set;
+    set.c = reinterpret_cast<double *>(smr);
+    set.w = reinterpret_cast<unsigned *>(set.c + SLOTS);
+    set.tab = set.w + 4 * NW * SLOTS;
+    set.tag = reinterpret_cast<unsigned short *>(set.tab + TAB);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned short *queue = set.tag + SLOTS + warp * RS_QCAP;
 
-    if (tid == 0) s_go = (S->err == 0 && S->rot < S->rot_end && S->n <= C) ? 1 : 0;
+    if (tid == 0) {
+        s_go = (S->err == 0 && S->rot < S->rot_end && S->n <= C) ? 1 : 0;
+        s_full = 0;
+    }
+    if (tid < 9) (&s_cnt[0][0])[tid] = 0;
     __syncthreads();
     if (!s_go) return;
     const DevParams &P = *B.P;
-    const DevFilter &F = P.strict;
-    const FLite fl = flite(F);
-    for (int i = tid; i < 130; i += T) {
-        s_expw[i] = fl.use_dw ? F.expw[i] : 0.0;
-        s_expxw[i] = fl.use_dxw ? F.expxw[i] : 0.0;
-    }
+    RsParams q;
+    memset(&q, 0, sizeof q);
+    q.strict = fquick(P.strict);
+    q.strict_full = &P.strict;
+    q.local = &P.local;
+    q.S = S;
     const u64 ket[2] = {P.ket[0], P.ket[1]};
     const int chan_kind = P.chan_kind;
-    const u64 chan_mask[2] = {P.chan_mask[0], P.chan_mask[1]};
     const int cur = S->cur;
-    int n = (int)S->n;
-    int li = 0;                                    // the term set holding the live set
+    int n = (int)S->n, alive = n;                  // slots in use, live terms
+    auto clear_index = [&]() {
+        for (int i = tid; i < TAB / 4; i += T) reinterpret_cast<uint4 *>(set.tab)[i] = make_uint4(0u, 0u, 0u, 0u);
+    };
+    clear_index();
+    __syncthreads();
     {
         // the live set: dense, or the segment table of the last multi-kernel merge
         const u64 *Z = B.z[cur], *X = B.x[cur];
@@ -114,170 +108,173 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_small_run(Bufs B) {
                 p = (long long)B.sphys[lo] + (i - B.soff[lo]);
             }
             if (p < 0 || p >= B.cap) { atomicOr(&S->err, ERR_BOUNDS); p = 0; }
-            sm_put<NW>(tz(0), tx(0), C2, i, load_key<NW>(Z, X, p));
-            tc(0)[i] = Cc[p];
+            const Key32<NW> k = key_narrow<NW>(load_key<NW>(Z, X, p));
+            set.put(i, k, Cc[p], 0u);
+            set.insert(i, rs_hash<NW>(k));
         }
     }
-    for (int i = tid; i < TAB / 8; i += T) reinterpret_cast<uint4 *>(tab)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid < 6) (&s_cnt[0][0])[tid] = 0;
     long long rot = S->rot;
-    const long long rot_end = S->rot_end;
-    // the first generator; later ones are copied in during the rotation before
-    auto fetch_gen = [&](int slot, long long q) {
-        if (tid < GQ) {
-            cp_async16(reinterpret_cast<char *>(&gs[slot]) + 16 * tid, reinterpret_cast<const char *>(B.gens + q) + 16 * tid);
-            cp_async_commit();
+    const long long rot0 = rot, rot_end = S->rot_end;
+    // the last warp copies generators in two rotations ahead and prepares them one
+    // rotation later, while the others work; a barrier publishes them
+    const bool feeder = warp == T / 32 - 1;
+    auto fetch_gen = [&](long long r) {
+        if (r < rot_end && lane < GQ)
+            cp_async16(reinterpret_cast<char *>(&gs[r & 1]) + 16 * lane, reinterpret_cast<const char *>(B.gens + r) + 16 * lane);
+        cp_async_commit();
+    };
+    auto make_gen = [&](long long r) {                // copied in before
+        cp_async_wait_all();
+        __syncwarp();
+        if (r < rot_end) rs_gen<NW>(&rg[(r - rot0) % 3], gs[r & 1], 0);
+        __syncwarp();
+    };
+    if (feeder)
+        for (int k = 0; k < 3; ++k) {
+            fetch_gen(rot + k);
+            if (k < 2) make_gen(rot + k);
+        }
+    long long acap = S->acap_logical;
+    long long created = 0, merge_out = 0, live_in = 0;
+    int early = 0, peak = 0;
+    bool measure_last = false, full = true;
+    // the change of the live count and the sin branches of a pass, added up in s_cnt[k]
+    auto count = [&](int out, int k) {
+        if (__any_sync(0xffffffffu, out != 0)) {
+            out = __reduce_add_sync(0xffffffffu, out);
+            if (lane == 0) {
+                const int dn = (int)(short)(out & 0xffff);
+                if (dn) atomicAdd(&s_cnt[k][1], dn);
+                if (out - dn) atomicAdd(&s_cnt[k][2], (out - dn) >> 16);
+            }
         }
     };
-    fetch_gen(0, rot);
-    if (tid < GQ) cp_async_wait_all();
-    long long acap = S->acap_logical;
-    long long created = 0, merge_in = 0, merge_out = 0, live_in = 0, early = 0, peak = S->peak;
-    bool measure_last = false;
 
-    for (int par = 0;; par ^= 1) {
-        __syncthreads();
-        const GenRec &g = gs[par];
-        if (rot + 1 < rot_end) fetch_gen(par ^ 1, rot + 1);   // the previous readers of that slot passed the barrier
-        // the next rotation's counters start from zero (their last readers passed this barrier)
-        if (tid < 3) s_cnt[par ^ 1][tid] = 0;
-        const bool pref = n > acap;
+    __syncthreads();
+    for (int k3 = 0;; k3 = k3 == 2 ? 0 : k3 + 1) {
+        const RsGen<NW> &g = rg[k3];
+        if (feeder) {
+            // the next rotation's counters start from zero (their last readers have passed a barrier)
+            if (lane < 3) s_cnt[k3 == 2 ? 0 : k3 + 1][lane] = 0;
+            make_gen(rot + 2);
+            fetch_gen(rot + 3);
+        }
+        const bool pref = alive > acap;
         const int flags = g.flags;
         const bool do_chan = (flags & GEN_CHANNEL) != 0 && chan_kind >= 0;
         measure_last = (flags & GEN_MEASURE) != 0;
-        const u64 *LZ = tz(li), *LX = tx(li);
-        const double *LC = tc(li);
-        u64 *OZ = tz(li ^ 1), *OX = tx(li ^ 1);
-        double *OC = tc(li ^ 1);
-        // ---- pre-filter marks, and the index of the live anticommuting terms
-        int nd = 0, na = 0;
-        for (int i = tid; i < n; i += T) {
-            const Key<NW> k = sm_key<NW>(LZ, LX, C2, i);
-            const bool dead = pref && drop_lite<NW>(fl, s_expw, s_expxw, k, fabs(LC[i]));
-            sdead[i] = dead ? 1 : 0;
-            nd += dead ? 1 : 0;
-            if (dead || !anticommutes<NW>(k, g)) continue;
-            ++na;
-            unsigned h = bk_slot<NW, TAB>(k);
-            for (int probe = 0; probe < TAB; ++probe) {
-                if (atomicCAS(&tab[h], (unsigned short)0, (unsigned short)(i + 1)) == (unsigned short)0) break;
-                h = (h + 1) & (TAB - 1);
+        // room for every live term's sin branch: else the live terms are moved together
+        if (n + alive > SLOTS) {
+            unsigned short *list = reinterpret_cast<unsigned short *>(set.tab);
+            int m = 0;
+            for (int base = 0; base < n; base += T) {
+                const int i = base + tid;
+                const int on = i < n && !(set.tag[i] & BB_DEAD) ? 1 : 0;
+                int tot;
+                const int o = m + block_excl_scan<T>(on, 0, OpSum(), s_scan, &tot);
+                if (on) list[o] = (unsigned short)i;
+                m += tot;
             }
+            __syncthreads();
+            for (int base = 0; base < m; base += T) {         // a term's new slot is never above its old one
+                const int i = base + tid;
+                Key32<NW> k;
+                double v = 0.0;
+                if (i < m) { k = set.key(list[i]); v = set.c[list[i]]; }
+                __syncthreads();
+                if (i < m) set.put(i, k, v, 0u);
+                __syncthreads();
+            }
+            clear_index();
+            __syncthreads();
+            for (int i = tid; i < m; i += T) set.insert(i, rs_hash<NW>(set.key(i)));
+            n = m;
+            __syncthreads();
         }
-        if (nd) atomicAdd(&s_cnt[par][2], nd);
-        if (na) atomicAdd(&s_cnt[par][1], na);
+        const int n_in = alive;
+        long long np = n_in;
+        if (full && pref) {
+            count(rs_filter<NW, SLOTS, TAB, T, false>(set, q, n, rot), k3);
+            __syncthreads();
+            np = n_in + s_cnt[k3][1];
+            __syncthreads();                       // read by every thread before the rotation adds to it
+        }
+        const int out = rs_step<NW, SLOTS, TAB, T, false>(set, g, q, n, queue, &s_cnt[k3][0], &s_full, rot);
+        count(out, k3);
         __syncthreads();
-        // ---- outputs: own term (cos branch plus the partner's sin branch), new sin branches
-        const int rounds = (n + T - 1) / T;
-        for (int rd = 0; rd < rounds; ++rd) {
-            const int i = rd * T + tid;
-            bool own = false, nw_ = false;
-            double oval = 0.0, nval = 0.0;
-            Key<NW> kk, qk;
-            if (i < n && !sdead[i]) {
-                kk = sm_key<NW>(LZ, LX, C2, i);
-                const double c = LC[i];
-                double v = c;
-                double sg = 0.0;
-                if (rotate_term<NW>(kk, g, &qk, &sg)) {
-                    v = __dmul_rn(c, g.cosv);
-                    const double sv = g.sinv;
-                    // the partner P xor G in the index (live, anticommuting, not pre-filtered)
-                    int j = -1;
-                    unsigned h = bk_slot<NW, TAB>(qk);
-                    for (int probe = 0; probe < TAB; ++probe) {
-                        const int e = tab[h];
-                        if (e == 0) break;
-                        if (e - 1 < n && key_eq<NW>(sm_key<NW>(LZ, LX, C2, e - 1), qk)) { j = e - 1; break; }
-                        h = (h + 1) & (TAB - 1);
-                    }
-                    if (j >= 0) {
-                        // live value first, then the partner's sin branch (phase -sg)
-                        v = __dadd_rn(v, __dmul_rn(-(sg * sv), LC[j]));
-                    } else {
-                        const double sbr = __dmul_rn(sg * sv, c);   // (k - 2) * sin(theta) * c, spv_kernels.jl:163
-                        if (!drop_lite<NW>(fl, s_expw, s_expxw, qk, fabs(sbr))) {
-                            nval = do_chan ? __dmul_rn(sbr, chan_lite<NW>(chan_kind, chan_mask, P.chanX, P.chanY,
-                                                                           P.chanZ, qk))
-                                           : sbr;
-                            nw_ = true;
-                        }
-                    }
-                }
-                if (!drop_lite<NW>(fl, s_expw, s_expxw, kk, fabs(v))) {
-                    oval = do_chan ? __dmul_rn(v, chan_lite<NW>(chan_kind, chan_mask, P.chanX, P.chanY, P.chanZ, kk))
-                                   : v;
-                    own = true;
-                }
-            }
-            // slots: the warp's claiming lanes take consecutive slots from one atomic
-            const unsigned w1 = __ballot_sync(0xffffffffu, own), w2 = __ballot_sync(0xffffffffu, nw_);
-            const int c1 = __popc(w1);
-            const int leader = __ffs(w1 | w2) - 1;
-            int base = 0;
-            if (lane == leader) base = atomicAdd(&s_cnt[par][0], c1 + __popc(w2));
-            base = __shfl_sync(0xffffffffu, base, leader < 0 ? 0 : leader);
-            const unsigned lt = (1u << lane) - 1u;
-            if (own) {
-                const int o = base + __popc(w1 & lt);
-                if (o < C2) { sm_put<NW>(OZ, OX, C2, o, kk); OC[o] = oval; }
-            }
-            if (nw_) {
-                const int o = base + c1 + __popc(w2 & lt);
-                if (o < C2) { sm_put<NW>(OZ, OX, C2, o, qk); OC[o] = nval; }
-            }
+        n = min(n + s_cnt[k3][0], SLOTS);
+        if (full && !pref) {
+            count(rs_filter<NW, SLOTS, TAB, T, false>(set, q, n, rot), k3);
+            __syncthreads();
         }
-        __syncthreads();
-        for (int q = tid; q < TAB / 8; q += T) reinterpret_cast<uint4 *>(tab)[q] = make_uint4(0u, 0u, 0u, 0u);
-        // ---- commit (every thread keeps the same counts; thread 0 records)
-        const int total = s_cnt[par][0], a = s_cnt[par][1], ndead = s_cnt[par][2];
-        const long long np = pref ? (long long)(n - ndead) : (long long)n;
-        if (tid == 0 && B.rec) {
-            long long *r = B.rec + 4 * rot;
-            r[0] = a;
-            r[1] = (pref ? n : 0) + np + a;
-            r[2] = (pref ? np : 0) + total;
-            r[3] = pref ? 1 : 0;
+        if (do_chan) {
+            for (int i = tid; i < n; i += T)
+                if (!(set.tag[i] & BB_DEAD)) set.c[i] = __dmul_rn(set.c[i], channel_factor<NW>(P, key_wide<NW>(set.key(i))));
+            __syncthreads();
         }
-        if (total > C2 && tid == 0) atomicOr(&S->err, ERR_BOUNDS);   // n + a <= 2n <= C2: never
-        created += a;
-        merge_in += n + a;
-        merge_out += total;
-        live_in += n;
-        if (total > peak) peak = total;
-        if (pref) {
-            early += 1;
-            if (np > acap) acap = max(2 * acap, np);
+        full = do_chan;
+        // ---- commit (every thread keeps the live count and the capacity; thread 0 the totals)
+        const int total = n_in + s_cnt[k3][1];
+        if (pref && np > acap) acap = max(2 * acap, np);
+        if (tid == 0) {
+            const int a = s_cnt[k3][2];
+            if (B.rec) {
+                long long *r = B.rec + 4 * rot;
+                r[0] = a;
+                r[1] = (pref ? n_in : 0) + np + a;
+                r[2] = (pref ? np : 0) + total;
+                r[3] = pref ? 1 : 0;
+            }
+            created += a;
+            merge_out += total;
+            live_in += n_in;
+            peak = max(peak, total);
+            early += pref ? 1 : 0;
         }
-        n = min(total, C2);
-        li ^= 1;
+        alive = total;
         ++rot;
-        if (tid < GQ) cp_async_wait_all();   // the next generator has landed (published by the next barrier)
-        if (rot >= rot_end || n > C) break;
+        if (rot >= rot_end || alive > C) break;
     }
     __syncthreads();
-    // ---- sort the survivors once (bitonic over an index array; keys are distinct)
-    const u64 *LZ = tz(li), *LX = tx(li);
-    const double *LC = tc(li);
+    if (s_full && tid == 0) atomicOr(&S->err, ERR_BOUNDS);       // n + alive <= SLOTS: never
+    // ---- an index array of the live slots (in the key index's memory)
+    unsigned short *sa = reinterpret_cast<unsigned short *>(set.tab);
+    {
+        int m = 0;
+        for (int base = 0; base < n; base += T) {
+            const int i = base + tid;
+            const int on = i < n && !(set.tag[i] & BB_DEAD) ? 1 : 0;
+            int tot;
+            const int o = m + block_excl_scan<T>(on, 0, OpSum(), s_scan, &tot);
+            if (on) sa[o] = (unsigned short)i;
+            m += tot;
+        }
+        n = m;
+    }
+    __syncthreads();
+    // ---- sort the survivors once (bitonic over an index array; keys are distinct;
+    // entries from n up, 0xffff, stay behind every slot)
     int pa = 1;
     while (pa < n) pa <<= 1;
-    for (int j = tid; j < pa; j += T) sa[j] = (unsigned short)j;
+    for (int j = n + tid; j < pa; j += T) sa[j] = 0xffffu;
     __syncthreads();
     for (int k = 2; k <= pa; k <<= 1) {
         for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = tid; i < pa; i += T) {
-                const int l = i ^ j;
-                if (l > i) {
-                    const int u = sa[i], v = sa[l];
-                    bool gt;   // element u after element v
-                    if (u >= n) gt = v >= n ? u > v : true;
-                    else if (v >= n) gt = false;
-                    else gt = key_lt<NW>(sm_key<NW>(LZ, LX, C2, v), sm_key<NW>(LZ, LX, C2, u));
-                    if (gt == ((i & k) == 0)) { sa[i] = (unsigned short)v; sa[l] = (unsigned short)u; }
-                }
+            for (int e = tid; e < pa / 2; e += T) {
+                const int i = ((e & ~(j - 1)) << 1) | (e & (j - 1)), l = i | j;
+                const int u = sa[i], v = sa[l];
+                // element u after element v (no order among the entries behind every slot)
+                const bool up = (i & k) == 0;
+                bool swap;
+                if (u == 0xffff || v == 0xffff) swap = u != v && (u == 0xffff) == up;
+                else swap = key_lt<NW>(key_wide<NW>(set.key(v)), key_wide<NW>(set.key(u))) == up;
+                if (swap) { sa[i] = (unsigned short)v; sa[l] = (unsigned short)u; }
             }
-            __syncthreads();
+            // pairs less than 32 apart stay within the 64 entries of a warp's 32 threads
+            if (j > 32) __syncthreads();
+            else __syncwarp();
         }
+        __syncthreads();
     }
     // ---- the survivors, dense and sorted, into the other buffer set; <ket|O|ket>
     // of a measured last rotation over the sorted set (contiguous runs per thread,
@@ -293,8 +290,8 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_small_run(Bufs B) {
     Neu acc{0.0, 0.0};
     for (int i = i0; i < i1; ++i) {
         const int src = sa[i];
-        const Key<NW> k = sm_key<NW>(LZ, LX, C2, src);
-        const double c = LC[src];
+        const Key<NW> k = key_wide<NW>(set.key(src));
+        const double c = set.c[src];
         store_key<NW>(Z, X, i, k);
         Cc[i] = c;
         if (measure_last && is_diag<NW>(k)) acc.add(ket_sign<NW>(k, ket) * c);
@@ -320,11 +317,11 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_small_run(Bufs B) {
         S->rot = rot;
         S->acap_logical = acap;
         S->created += created;
-        S->merge_in += merge_in;
+        S->merge_in += live_in + created;
         S->merge_out += merge_out;
         S->live_in += live_in;
         S->early += early;
-        S->peak = peak;
+        S->peak = max(S->peak, (long long)peak);
         S->npref = 0;
         if (measure_last) { S->expect_val = expect; S->measure_valid = 1; }
     }

@@ -145,7 +145,9 @@ struct pp_spv {
     unsigned *bk_delta = nullptr;           // bucket hash of each generator of the call
     long long bk_delta_cap = 0;
     BkStat *bk_stat = nullptr;              // pinned, two chunks
-    int bb_occ[2] = {0, 0};                 // resident CTAs per SM of k_bb_block (plain, batched)
+    int bb_occ[3] = {0, 0, 0};              // resident CTAs per SM of k_bb_block (plain, batched, adaptive)
+    double *bk_thr = nullptr, *bk_vals = nullptr;   // adaptive sequences: thresholds, survivors' |c|
+    long long bk_thr_cap = 0, bk_vals_cap = 0;
     int bk_cap = 0;
     u64 *bk_rows = nullptr;
     BkRec *bk_rec = nullptr;
@@ -1390,16 +1392,17 @@ static int bb_init(pp_spv *h) {
         *occ = std::max(1, o);
         return PP_OK;
     };
-    if constexpr (NW == 2) TRY(set(k_bb_block<2, true>, &h->bb_occ[1]));
-    return set(k_bb_block<NW, false>, &h->bb_occ[0]);
+    if constexpr (NW == 2) TRY(set(k_bb_block<2, BB_BATCH>, &h->bb_occ[1]));
+    TRY(set(k_bb_block<NW, BB_ADAPT>, &h->bb_occ[2]));
+    return set(k_bb_block<NW, BB_PLAIN>, &h->bb_occ[0]);
 }
 
 template <int NW>
 static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl) {
-    const bool batch = NW == 2 && h->batch_on;
+    const int mode = A.thr ? BB_ADAPT : NW == 2 && h->batch_on ? BB_BATCH : BB_PLAIN;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)std::min(((1ll << (pl.bits - pl.d)) + BB_WARPS - 1) / BB_WARPS,
-                                          (long long)h->nsm * h->bb_occ[batch ? 1 : 0]));
+                                          (long long)h->nsm * h->bb_occ[mode]));
     cfg.blockDim = dim3(32 * BB_WARPS);
     cfg.dynamicSmemBytes = bb_smem_bytes<NW>();
     cfg.stream = h->stream;
@@ -1410,8 +1413,10 @@ static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl) {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaError_t e;
-    if constexpr (NW == 2) e = batch ? cudaLaunchKernelEx(&cfg, k_bb_block<2, true>, A, pl) : cudaLaunchKernelEx(&cfg, k_bb_block<2, false>, A, pl);
-    else e = cudaLaunchKernelEx(&cfg, k_bb_block<1, false>, A, pl);
+    if (mode == BB_ADAPT) e = cudaLaunchKernelEx(&cfg, k_bb_block<NW, BB_ADAPT>, A, pl);
+    else if (mode == BB_PLAIN) e = cudaLaunchKernelEx(&cfg, k_bb_block<NW, BB_PLAIN>, A, pl);
+    else if constexpr (NW == 2) e = cudaLaunchKernelEx(&cfg, k_bb_block<2, BB_BATCH>, A, pl);
+    else e = cudaErrorInvalidValue;
     return e == cudaSuccess ? PP_OK : fail(PP_DEVICE_ERROR, std::string("launch failure: ") + cudaGetErrorString(e));
 }
 
@@ -1880,7 +1885,7 @@ static int adaptive_apply(pp_spv *h, long long max_terms, double min_thresh) {
         // the threshold stays on the device
         compile_filter(&f, &h->Ph->clip);
         TRY(upload_params(h));
-        k_abs_select<<<1, AS_THREADS, 0, h->stream>>>(h->c[0], h->c[1], h->S, max_terms, min_thresh, &h->P->clip.thresh);
+        k_abs_select<<<1, AS_THREADS, 0, h->stream>>>(h->c[0], h->c[1], h->S, nullptr, max_terms, min_thresh, &h->P->clip.thresh);
     } else {
         f.thresh = min_thresh;
         if (st.n > max_terms) {
@@ -2119,6 +2124,173 @@ static int adapt_step(pp_spv *h, AdaptSpec &A) {
     return PP_OK;
 }
 
+// AdaptiveTruncation sequences at window 1 on buckets: rotations [start, L) with
+// _apply!(v, ::AdaptiveTruncation) (spv_evolve.jl:103-114) after each.  A rotation is one
+// unfiltered block (k_bb_block, adaptive mode) that first drops what the previous
+// rotation's threshold cuts, and one launch that selects the next threshold from the
+// listed |c|; nothing comes back to the host but the state of a chunk of rotations.
+// For sequences without early merges (the caller has seen to that: n and max_terms are
+// at most the append capacity), corrections and WindowCounters.  period: a channel after
+// every period-th rotation, behind its truncation.  BK_NOFIT: nothing was changed.
+// Measured (one B200, budget 20,000 on a 30-qubit chain, 351 rotations): 70.5 ms with a
+// sorted merge, a select and a clip per rotation, each with host round trips (200 us a
+// rotation).
+static constexpr int ADAPT_MIN_ROT = 8;
+static constexpr int ADAPT_CHUNK = 64;
+
+template <int NW>
+static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, int chan_flags, RunProf *prof, AdaptSpec &Q) {
+    TRY(bk_rows_init(h));
+    TRY(bb_init<NW>(h));
+    cudaStream_t s = h->stream;
+    DevState st;
+    TRY(read_state(h, &st));
+    const long long n0 = st.n, most = std::max(n0, std::min(2 * Q.max_terms, (long long)1 << 31));
+    int bits = bk_bits_for(most, BB_CAP, h->tune.load_div), cur = 0;
+    // sized for the budget at once: the set grows to twice that within a rotation
+    for (;;) {
+        const int rr = bk_reserve<NW>(h, bits, &cur, -1, BB_CAP);
+        if (rr == BK_NOFIT && bits > bk_bits_for(most, BB_CAP, 3)) { --bits; continue; }
+        if (rr) return rr;
+        break;
+    }
+    if (L + 1 > h->bk_rec_cap) {
+        TRY(dalloc(h, &h->bk_rec, L + 1));
+        h->bk_rec_cap = L + 1;
+    }
+    if (L > h->bk_delta_cap) {
+        TRY(dalloc(h, &h->bk_delta, L));
+        h->bk_delta_cap = L;
+    }
+    if (L + 1 > h->bk_thr_cap) {
+        TRY(dalloc(h, &h->bk_thr, L + 1));
+        h->bk_thr_cap = L + 1;
+    }
+    auto vals_reserve = [&]() -> int {
+        const long long slots = (long long)BB_CAP << bits;
+        if (slots <= h->bk_vals_cap) return PP_OK;
+        TRY(dalloc(h, &h->bk_vals, slots));
+        h->bk_vals_cap = slots;
+        return PP_OK;
+    };
+    TRY(vals_reserve());
+    int mx = 0;
+    for (;;) {
+        TRY(bk_scatter<NW>(h, h->z[st.cur], h->x[st.cur], h->c[st.cur], n0, -1, 0, 0, bits, &mx));
+        if (mx >= 0 && mx <= BB_CAP / 2) break;
+        const int rr = ++bits > BK_ROWS ? BK_NOFIT : bk_reserve<NW>(h, bits, &cur, -1, BB_CAP);
+        if (rr) return rr;
+        TRY(vals_reserve());
+    }
+    BkRec r0;
+    memset(&r0, 0, sizeof r0);
+    r0.n_out = (unsigned long long)n0;
+    r0.acap = 1ll << 62;
+    const double none = -1.0;              // the entering set is not cut
+    CU(cudaMemcpyAsync(h->bk_rec + start, &r0, sizeof r0, cudaMemcpyHostToDevice, s));
+    CU(cudaMemsetAsync(h->bk_rec + start + 1, 0, (L - start) * sizeof(BkRec), s));
+    CU(cudaMemcpyAsync(h->bk_thr + start, &none, sizeof none, cudaMemcpyHostToDevice, s));
+    k_bb_deltas<NW><<<(int)std::min((L - start + 127) / 128, (long long)h->nsm), 128, 0, s>>>(
+        h->gens + start, L - start, h->bk_rows, h->bk_delta + start);
+    std::vector<unsigned> delta((size_t)L);
+    CU(cudaMemcpyAsync(delta.data() + start, h->bk_delta + start, (size_t)(L - start) * sizeof(unsigned),
+                       cudaMemcpyDeviceToHost, s));
+    TRY(sync_check(h));
+    PP_TRACE("adaptive on buckets: rotations [%lld, %lld), %lld live terms, 2^%d buckets", start, L, n0, bits);
+    int limit = BB_DMAX;
+    long long done = start;
+    while (done < L) {
+        const long long end = std::min(L, done + ADAPT_CHUNK);
+        BkArgs A = bk_args(h, bits, h->bk_rec);
+        A.thr = h->bk_thr;
+        A.vals = h->bk_vals;
+        A.vals_cap = h->bk_vals_cap;
+        const int dims = bb_dims(most, bits, bb_slots<NW>(), limit, (long long)h->nsm * BB_WARPS * h->bb_occ[2]);
+        st.bk_fail = 0x7fffffffffffffffll;
+        st.bk_pad = 0;
+        TRY(write_state(h, &st));
+        for (long long r = done; r < end; ++r) {
+            BbPlan pl = bb_plan(delta.data(), r, 1, bits, dims);
+            pl.cur = (cur + (int)(r - done)) & 1;
+            pl.prechan = r > start && (h->gens_h[r - 1].flags & chan_flags) && h->Ph->chan_kind >= 0 ? 1 : 0;
+            TRY(bb_launch<NW>(h, A, pl));
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(1);
+            cfg.blockDim = dim3(AS_THREADS);
+            cfg.stream = s;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            CU(cudaLaunchKernelEx(&cfg, k_abs_select, (const double *)h->bk_vals, (const double *)nullptr, (const DevState *)h->S,
+                                  (const unsigned long long *)&h->bk_rec[r + 1].nval, Q.max_terms, Q.min_thresh,
+                                  h->bk_thr + r + 1));
+            prof->launches += 2;
+        }
+        TRY(sync_check(h));
+        TRY(read_state(h, &st));
+        if (st.err & ~ERR_OVERFLOW) return check_err(h, st);
+        const long long upto = st.err & ERR_OVERFLOW ? std::max(done, std::min(end, st.bk_fail)) : end;
+        cur = (cur + (int)(upto - done)) & 1;
+        done = upto;
+        if (st.err & ERR_OVERFLOW) {
+            const int over = st.bk_pad;
+            st.err &= ~ERR_OVERFLOW;
+            TRY(write_state(h, &st));
+            CU(cudaMemsetAsync(h->bk_rec + done + 1, 0, (end - done) * sizeof(BkRec), s));
+            if (over & 2) limit = std::max(1, dims - 1);
+            if (over & 1) {
+                const int rr = bk_regrid<NW>(h, &cur, &bits);
+                if (rr == BK_NOFIT) return fail(PP_OUT_OF_MEMORY, "the bucket layout of this sequence does not fit in device memory");
+                if (rr) return rr;
+                TRY(vals_reserve());
+            }
+        }
+    }
+    // totals, as the merges and clips of the general path count them
+    std::vector<BkRec> rec((size_t)(L - start + 1));
+    CU(cudaMemcpyAsync(rec.data(), h->bk_rec + start, rec.size() * sizeof(BkRec), cudaMemcpyDeviceToHost, s));
+    TRY(sync_check(h));
+    for (long long r = start; r < L; ++r) {
+        const BkRec &o = rec[(size_t)(r - start + 1)];
+        st.live_in += (long long)o.np;
+        st.created += (long long)o.created;
+        st.merge_in += (long long)o.np + (long long)o.created + (long long)o.n_out;
+        st.merge_out += (long long)o.n_out + (r + 1 < L ? (long long)rec[(size_t)(r - start + 2)].np : 0);
+        st.peak = std::max(st.peak, (long long)o.n_out);
+    }
+    const long long n = (long long)rec.back().n_out;
+    st.merge_in -= n;                      // the last clip is a merge of its own below
+    prof->bk_rot += L - start;
+    TRY(write_state(h, &st));
+    TRY(bk_to_dense<NW>(h, cur, bits, n));
+    // the cut after the last rotation, its channel, and <ket|O|ket>
+    compile_filter(nullptr, &h->Ph->clip);
+    TRY(upload_params(h));
+    CU(cudaMemcpyAsync(&h->P->clip.thresh, h->bk_thr + L, sizeof(double), cudaMemcpyDeviceToDevice, s));
+    Bufs B = make_bufs(h);
+    launch_merge<NW, 2>(h, B, 0);
+    prof->launches += 3;
+    TRY(sync_check(h));
+    TRY(read_state(h, &st));
+    TRY(check_err(h, st));
+    if (h->Ph->chan_kind >= 0 && (h->gens_h[L - 1].flags & chan_flags)) {
+        Bufs Bc = make_bufs(h);
+        k_channel<NW><<<h->nsm * 8, 256, 0, s>>>(Bc);
+        TRY(sync_check(h));
+    }
+    if (last_flags & GEN_MEASURE) {
+        double e = 0.0;
+        TRY(expect_dev(h, h->Ph->ket, &e));
+        TRY(read_state(h, &st));
+        st.expect_val = e;
+        st.measure_valid = 1;
+        TRY(write_state(h, &st));
+    }
+    return PP_OK;
+}
+
 // General path: the sequence driver of spv_evolve.jl:352-385 with host decisions.
 // `period` > 0 makes every period-th rotation end a separate evolve! call (the
 // window count restarts and a boundary closes the layer), which is the
@@ -2128,11 +2300,19 @@ static int run_general(pp_spv *h, const std::vector<GenRec> &G, long long window
                        long long period, int chan_flags, RunProf *prof, AdaptSpec &A) {
     const long long L = (long long)G.size();
     long long since = 0;
+    // (above AS_MAX values a threshold is better selected by the whole grid)
+    bool adapt_bk = window == 1 && A.on && A.kind == 1 && !A.corr && !ctr && bk_enabled() && 2 * A.max_terms <= AS_MAX;
     for (long long i = 1; i <= L; ++i) {
         const long long w = (i + window - 1) / window;
         const long long irel = period > 0 ? (i - 1) % period + 1 : i;
         DevState st;
         TRY(read_state(h, &st));
+        if (adapt_bk && L - i + 1 >= ADAPT_MIN_ROT && st.an == 0 && st.n <= AS_MAX && std::max(st.n, A.max_terms) <= st.acap_logical) {
+            // no early merge from here on: the rest on buckets
+            const int rr = run_adapt<NW>(h, i - 1, L, last_flags, chan_flags, prof, A);
+            if (rr != BK_NOFIT) return rr;
+            adapt_bk = false;
+        }
         if (2 * st.an + st.n > st.acap_logical) {
             long long ni, no;
             TRY(general_boundary<NW>(h, 0, &ni, &no));

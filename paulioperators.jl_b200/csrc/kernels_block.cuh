@@ -424,7 +424,7 @@ __device__ __forceinline__ int rs_filter(const ResidentSet<NW, SLOTS, TAB> &s, c
 // delta's coordinates (the bits at piv).
 struct BbPlan {
     long long r0;
-    int K, d, full, kprev, cur, bits;
+    int K, d, full, kprev, cur, bits, prechan;
     unsigned basis[BB_KMAX];
     int piv[BB_KMAX];
     int dl[BB_KMAX];
@@ -438,14 +438,23 @@ __global__ void k_bb_deltas(const GenRec *gens, long long n, const u64 *rows, un
         out[i] = bk_hash<NW>(gens[i].gz, gens[i].gx, rows, BK_ROWS);
 }
 
+// Modes of k_bb_block: plain; batched instances; adaptive sequences (blocks of one
+// rotation, unfiltered: the terms that AdaptiveTruncation drops after the previous
+// rotation -- |c| at most thr[r0] -- are dropped as they are loaded, a channel between
+// the two (pl.prechan) is applied there, and the survivors' |c| are listed for the next
+// threshold).
+constexpr int BB_PLAIN = 0, BB_BATCH = 1, BB_ADAPT = 2;
+
 // One block of rotations; input bucket set pl.cur, output set pl.cur ^ 1 (the input
 // stays intact, so a block that does not fit -- a coset beyond the resident set, or
 // an output bucket beyond BB_CAP -- is flagged and run again by the host, after a
 // split or with fewer rotations).  Persistent grid; every warp takes cosets of its
 // own, so no block barrier stands between a rotation and the next.
-template <int NW, bool BATCH>
+template <int NW, int MODE>
 __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_constant__ BkArgs A,
                                                                const __grid_constant__ BbPlan pl) {
+    constexpr bool BATCH = MODE == BB_BATCH;
+    constexpr bool ADAPT = MODE == BB_ADAPT;
     constexpr int SLOTS = bb_slots<NW>();
     constexpr int TAB = BB_TAB;
     static_assert(2 * 2 * BB_CAP <= SLOTS, "a block of one rotation always fits");
@@ -458,6 +467,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     __shared__ unsigned short s_ow[BB_WARPS][BB_MEMBERS];
     __shared__ int s_fw[BB_WARPS][2];                      // fresh slots of the step, resident set full
     __shared__ int s_tot[BB_KMAX][2], s_np, s_mx, s_over, s_err, s_pref, s_bad;
+    __shared__ double s_thr;
     extern __shared__ __align__(16) unsigned char bbm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     ResidentSet<NW, SLOTS, TAB> set;
@@ -495,7 +505,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     q.ninst = A.ninst;
     q.ncol = A.ncol;
     q.S = S;
-    const bool do_chan = (last_flags & GEN_CHANNEL) != 0 && P.chan_kind >= 0;
+    const bool do_chan = !ADAPT && (last_flags & GEN_CHANNEL) != 0 && P.chan_kind >= 0;
     const int cur = pl.cur;
     const int *CNT = cur ? A.cnt[1] : A.cnt[0];
     int *OCNT = cur ? A.cnt[0] : A.cnt[1];
@@ -507,6 +517,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tid == 0) {
         s_err = *(volatile int *)&S->err;
+        if constexpr (ADAPT) s_thr = *(const volatile double *)&A.thr[r0];
         // the early-merge rule of spv_evolve.jl:356-362 up to r0, from the previous
         // block's records (after a rotation every live value has passed the filter, so a
         // rotation inside a block that starts with an early merge drops nothing by it)
@@ -537,7 +548,8 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     }
     __syncthreads();
     if (s_err) return;
-    const bool drop_first = pl.full && s_pref;
+    const bool drop_first = ADAPT || (pl.full && s_pref);
+    const double thr = ADAPT ? s_thr : 0.0;
     const long long nb = 1ll << pl.bits;
     if (pl.bits > A.bits_cap || d > pl.bits || d > BB_DMAX || K > BB_KMAX || r0 + K >= A.rec_len) {
         if (tid == 0) flag_bounds(S, 1, ((long long)pl.bits << 16) | d);
@@ -609,7 +621,10 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                 if (i < total) {
                     const Key32<NW> k = key_narrow<NW>(kk[u]);
                     bool dead = false;
-                    if (drop_first) {
+                    if constexpr (ADAPT) {
+                        dead = fabs(cc[u]) <= thr;
+                        if (pl.prechan && !dead) cc[u] = __dmul_rn(cc[u], channel_factor<NW>(P, kk[u]));
+                    } else if (drop_first) {
                         dead = rs_drop<NW>(q, k, fabs(cc[u]));
                         if constexpr (BATCH) dead = dead && rs_instance<NW>(k, q, r0) >= 0;
                     }
@@ -648,10 +663,21 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
         if (*full) {
             over = true;
         } else {
+            long long vat = 0;                             // adaptive: where this coset's values go
+            if constexpr (ADAPT) {
+                if (lane == 0) vat = (long long)atomicAdd(&A.rec[r0 + 1].nval, (unsigned long long)alive);
+                vat = __shfl_sync(0xffffffffu, vat, 0);
+            }
             for (int base = 0; base < n; base += 32) {
                 const int i = base + lane;
                 const unsigned t = i < n ? set.tag[i] : BB_DEAD | 0x7fffu;
                 const bool live = !(t & BB_DEAD);
+                if constexpr (ADAPT) {
+                    const unsigned m = __ballot_sync(0xffffffffu, live);
+                    const long long o = vat + __popc(m & ((1u << lane) - 1u));
+                    if (live && o < A.vals_cap) A.vals[o] = fabs(set.c[i]);
+                    vat += __popc(m);
+                }
                 const int lb = (int)(t & 0xff);
                 const unsigned seg = bk_segment((int)(t & 0x7fffu), lane);
                 const int po = bk_claim(scnt, lb, live, seg, lane);

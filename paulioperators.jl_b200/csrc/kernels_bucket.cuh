@@ -57,6 +57,7 @@ struct BkRec {
     unsigned long long n_out;       // survivors (sum over CTAs)
     unsigned long long np;          // survivors of the early-merge pre-filter (when pref)
     unsigned long long created;     // sin branches appended (after the local filter)
+    unsigned long long nval;        // adaptive sequences: values listed for the next threshold
     int pref;                       // the rotation began with an early merge (CTA 0)
     int maxcnt;                     // largest output bucket
 };
@@ -86,6 +87,11 @@ struct BkArgs {
     int *fcnt[2];
     int remote;
     int pref_forced;
+    // adaptive sequences: the threshold that cuts the set entering each rotation, and the
+    // list of the survivors' |c|
+    const double *thr;
+    double *vals;
+    long long vals_cap;
 };
 
 // Bucket of a key: the low `bits` bits of the GF(2)-linear hash.

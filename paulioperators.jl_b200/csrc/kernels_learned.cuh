@@ -869,8 +869,10 @@ constexpr long long AS_MAX = 1 << 18;
 constexpr int AS_BINS = 2048;
 constexpr int AS_KEEP = 3072;
 
+// With nval, the values are C0[0, *nval) instead of the live set's.
 __global__ void __launch_bounds__(AS_THREADS) k_abs_select(const double *C0, const double *C1, const DevState *S,
-                                                           long long max_terms, double min_thresh, double *thresh) {
+                                                           const unsigned long long *nval, long long max_terms,
+                                                           double min_thresh, double *thresh) {
     __shared__ unsigned h[AS_BINS];
     __shared__ unsigned long long keep[AS_KEEP];
     __shared__ long long sm[AS_THREADS / 32 + 1];
@@ -878,9 +880,11 @@ __global__ void __launch_bounds__(AS_THREADS) k_abs_select(const double *C0, con
     __shared__ long long s_rem;
     __shared__ unsigned s_cnt, s_n;
     const int tid = threadIdx.x;
-    if (S->err) return;
-    const long long n = S->n;
-    const double *C = S->cur ? C1 : C0;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (*(const volatile int *)&S->err) return;
+    const long long n = nval ? (long long)*(const volatile unsigned long long *)nval : S->n;
+    const double *C = nval || !S->cur ? C0 : C1;
     if (n <= max_terms) {
         if (tid == 0) *thresh = min_thresh;
         return;
@@ -897,7 +901,7 @@ __global__ void __launch_bounds__(AS_THREADS) k_abs_select(const double *C0, con
         const unsigned long long pre = s_pre;
         if (!listed) {
             for (long long i = tid; i < n; i += AS_THREADS) {
-                const unsigned long long k = (unsigned long long)__double_as_longlong(fabs(C[i]));
+                const unsigned long long k = (unsigned long long)__double_as_longlong(fabs(__ldcg(C + i)));
                 if ((k & mask) == pre) atomicAdd(&h[(k >> shift) & ((1u << w) - 1u)], 1u);
             }
         } else {
@@ -925,7 +929,7 @@ __global__ void __launch_bounds__(AS_THREADS) k_abs_select(const double *C0, con
             // the candidates fit: the remaining digits need no further pass over n values
             const unsigned long long cm = ~0ull << top, cp = s_pre;
             for (long long i = tid; i < n; i += AS_THREADS) {
-                const unsigned long long k = (unsigned long long)__double_as_longlong(fabs(C[i]));
+                const unsigned long long k = (unsigned long long)__double_as_longlong(fabs(__ldcg(C + i)));
                 if ((k & cm) == cp) {
                     const unsigned o = atomicAdd(&s_n, 1u);
                     if (o < AS_KEEP) keep[o] = k;

@@ -792,7 +792,7 @@ static int ss_sort(pp_spv *h, u64 *z, u64 *x, double *c, long long n, bool *ok) 
     if (n <= SS_CAP) {
         const int cap = n <= 1024 ? 1024 : SS_CAP;
         k_ss_sort<NW><<<1, SSS_THREADS, ss_sort_smem<NW>(cap), s>>>(z, x, c, nullptr, nullptr, (int)n, cap, nullptr, z, x, c, n);
-        return sync_check(h);
+        return PP_OK;                      // (nothing to ask the device about)
     }
     const SsPlan p = ss_plan(n);
     Key<NW> *key = reinterpret_cast<Key<NW> *>(h->ss_ws), *skey = key + SS_SAMPLES;
@@ -1837,15 +1837,14 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
     return dense ? PP_OK : ensure_dense(h);
 }
 
-// General path boundary: sort pending appends, merge (MODE 1).
+// General path boundary: sort pending appends, merge (MODE 1).  *st: the state after it.
 template <int NW>
-static int general_boundary(pp_spv *h, int flags, long long *n_in, long long *n_out) {
-    DevState st;
-    TRY(read_state(h, &st));
-    const long long an = st.an;
-    *n_in = st.n + an;
-    TRY(ensure_live(h, st.n + an));
-    TRY(read_state(h, &st));
+static int general_boundary(pp_spv *h, int flags, long long *n_in, long long *n_out, DevState *st) {
+    TRY(read_state(h, st));
+    TRY(check_err(h, *st));
+    const long long an = st->an;
+    *n_in = st->n + an;
+    TRY(ensure_live(h, st->n + an));
     Bufs B = make_bufs(h);
     if (an > 0) {
         int in_t = 0;
@@ -1856,9 +1855,9 @@ static int general_boundary(pp_spv *h, int flags, long long *n_in, long long *n_
     }
     launch_merge<NW, 1>(h, B, flags);
     TRY(sync_check(h));
-    TRY(read_state(h, &st));
-    TRY(check_err(h, st));
-    *n_out = st.n;
+    TRY(read_state(h, st));
+    TRY(check_err(h, *st));
+    *n_out = st->n;
     return PP_OK;
 }
 
@@ -2302,20 +2301,36 @@ static int run_general(pp_spv *h, const std::vector<GenRec> &G, long long window
     long long since = 0;
     // (above AS_MAX values a threshold is better selected by the whole grid)
     bool adapt_bk = window == 1 && A.on && A.kind == 1 && !A.corr && !ctr && bk_enabled() && 2 * A.max_terms <= AS_MAX;
+    // The state as far as the host knows it: without WindowCounters the rotations between
+    // two boundaries go out without a look at their results, as long as a bound on the
+    // pending appends (a rotation at most doubles live and pending terms) rules out an
+    // early merge and fits the append buffers.
+    DevState st;
+    bool exact = false;
+    long long ub = 0;                      // at least the pending appends
+    auto look = [&]() -> int {
+        if (exact) return PP_OK;
+        TRY(read_state(h, &st));
+        TRY(check_err(h, st));
+        exact = true;
+        ub = st.an;
+        return PP_OK;
+    };
     for (long long i = 1; i <= L; ++i) {
         const long long w = (i + window - 1) / window;
         const long long irel = period > 0 ? (i - 1) % period + 1 : i;
-        DevState st;
-        TRY(read_state(h, &st));
-        if (adapt_bk && L - i + 1 >= ADAPT_MIN_ROT && st.an == 0 && st.n <= AS_MAX && std::max(st.n, A.max_terms) <= st.acap_logical) {
+        if (i == 1 || ctr || 2 * ub + st.n > st.acap_logical || std::max(st.acap_logical, 2 * ub + st.n) > h->acap_phys)
+            TRY(look());
+        if (adapt_bk && L - i + 1 >= ADAPT_MIN_ROT && exact && st.an == 0 && st.n <= AS_MAX &&
+            std::max(st.n, A.max_terms) <= st.acap_logical) {
             // no early merge from here on: the rest on buckets
             const int rr = run_adapt<NW>(h, i - 1, L, last_flags, chan_flags, prof, A);
             if (rr != BK_NOFIT) return rr;
             adapt_bk = false;
         }
-        if (2 * st.an + st.n > st.acap_logical) {
+        if (exact && 2 * st.an + st.n > st.acap_logical) {
             long long ni, no;
-            TRY(general_boundary<NW>(h, 0, &ni, &no));
+            TRY(general_boundary<NW>(h, 0, &ni, &no, &st));
             if (A.on) TRY(adapt_step(h, A));
             since = 0;
             TRY(read_state(h, &st));
@@ -2328,27 +2343,29 @@ static int run_general(pp_spv *h, const std::vector<GenRec> &G, long long window
                 st.acap_logical = std::max(2 * st.acap_logical, st.n);
                 TRY(write_state(h, &st));
             }
+            ub = st.an;
         }
-        TRY(ensure_append(h, std::max(st.acap_logical, 2 * st.an + st.n), st.an));
+        TRY(ensure_append(h, std::max(st.acap_logical, 2 * ub + st.n), ub));
         TRY(alloc_merge_ws(h, h->cap, h->acap_phys));
         Bufs B = make_bufs(h);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         if (ctr && ctr->t_rotate) { cudaEventCreate(&e0); cudaEventCreate(&e1); cudaEventRecord(e0, h->stream); }
         const long long an_before = st.an;
-        const int ntiles = (int)std::max(1ll, (st.n + st.an + G_TILE - 1) / G_TILE);
+        const int ntiles = (int)std::max(1ll, (st.n + ub + G_TILE - 1) / G_TILE);
         k_rotate_general<NW><<<std::min(ntiles, h->nsm * h->occG), G_THREADS, 0, h->stream>>>(B, G[i - 1]);
-        k_rotate_commit<<<1, 1, 0, h->stream>>>(B);
         if (e1) cudaEventRecord(e1, h->stream);
-        TRY(sync_check(h));
-        TRY(read_state(h, &st));
-        TRY(check_err(h, st));
-        if (ctr && w <= ctr->nwin) {
-            if (ctr->terms_created) ctr->terms_created[w - 1] += st.an - an_before;
-            if (e0) { float ms = 0; cudaEventElapsedTime(&ms, e0, e1); ctr->t_rotate[w - 1] += ms * 1e-3; }
+        exact = false;
+        ub = 2 * ub + st.n;
+        if (ctr) {
+            TRY(look());
+            if (w <= ctr->nwin) {
+                if (ctr->terms_created) ctr->terms_created[w - 1] += st.an - an_before;
+                if (e0) { float ms = 0; cudaEventElapsedTime(&ms, e0, e1); ctr->t_rotate[w - 1] += ms * 1e-3; }
+            }
         }
         if (e0) { cudaEventDestroy(e0); cudaEventDestroy(e1); }
         since++;
-        prof->launches += 2;
+        prof->launches += 1;
         const bool layer_end = period > 0 && irel == period;
         if (irel % window == 0 || layer_end || i == L) {
             long long ni, no;
@@ -2356,10 +2373,12 @@ static int run_general(pp_spv *h, const std::vector<GenRec> &G, long long window
             if (ctr && ctr->t_merge) { cudaEventCreate(&m0); cudaEventCreate(&m1); cudaEventRecord(m0, h->stream); }
             const int fl = (i == L ? last_flags : 0) | (layer_end ? chan_flags : 0);
             if (!A.on) {
-                TRY(general_boundary<NW>(h, fl, &ni, &no));
+                TRY(general_boundary<NW>(h, fl, &ni, &no, &st));
+                exact = true;
+                ub = st.an;
             } else {
                 // merge unfiltered, then the strategy, then the layer's channel, then <ket|O|ket>
-                TRY(general_boundary<NW>(h, 0, &ni, &no));
+                TRY(general_boundary<NW>(h, 0, &ni, &no, &st));
                 TRY(adapt_step(h, A));
                 if (fl & GEN_CHANNEL) {
                     Bufs Bc = make_bufs(h);
@@ -2376,6 +2395,8 @@ static int run_general(pp_spv *h, const std::vector<GenRec> &G, long long window
                     s2.measure_valid = 1;
                     TRY(write_state(h, &s2));
                 }
+                exact = false;             // the strategy left another set
+                TRY(look());
             }
             prof->launches += 3;
             if (m0) {
@@ -2475,7 +2496,7 @@ static int evolve_impl(pp_spv *h, const void *gz, const void *gx, const double *
     st.peak = 0;
     st.corr_energy = O.corr_energy ? *O.corr_energy : 0.0;
     st.measure_valid = 0;
-    st.b_tile_ctr = 0; st.g_tile_ctr = 0;
+    st.b_tile_ctr = 0; st.g_tile_ctr = 0; st.g_done = 0;
     TRY(write_state(h, &st));
     pp_counters *ctr = O.counters;
     RunProf prof;

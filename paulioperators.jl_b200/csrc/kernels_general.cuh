@@ -98,21 +98,24 @@ __global__ void __launch_bounds__(G_THREADS) k_rotate_general(Bufs B, GenRec g) 
         }
         __syncthreads();
     }
-}
-
-// Commit of k_rotate_general: an += created (one thread, after the launch).
-__global__ void k_rotate_commit(Bufs B) {
-    DevState *S = B.S;
-    if (S->err & ~ERR_TIMEOUT) return;
-    const long long n = S->n, an = S->an, tot = n + an;
-    const int ntiles = (int)max(1ll, (tot + G_TILE - 1) / G_TILE);
-    const u64 st = st_load(B.gstat + (ntiles - 1));
-    const long long created = (long long)(unsigned)(st & 0xffffffffu);
-    S->an = an + created;
-    S->created += created;
-    S->live_in += n + an;
-    S->g_tile_ctr = 0;
-    S->epoch += 1;
+    // the last CTA to finish commits the rotation: an += created (a launch of its own took
+    // 3.5 us, against 6 for the rotation of 1e4 terms)
+    if (tid == 0) {
+        __threadfence();
+        if (atomicAdd(&S->g_done, 1) == (int)gridDim.x - 1) {
+            __threadfence();
+            if (!(*(volatile int *)&S->err & ~ERR_TIMEOUT)) {
+                const u64 stv = st_load(B.gstat + (ntiles - 1));
+                const long long created = (long long)(unsigned)(stv & 0xffffffffu);
+                S->an = an + created;
+                S->created += created;
+                S->live_in += n + an;
+                S->epoch += 1;
+            }
+            S->g_tile_ctr = 0;
+            S->g_done = 0;
+        }
+    }
 }
 
 // ------------------------------------------------------------ radix sort

@@ -145,7 +145,7 @@ struct pp_spv {
     unsigned *bk_delta = nullptr;           // bucket hash of each generator of the call
     long long bk_delta_cap = 0;
     BkStat *bk_stat = nullptr;              // pinned, two chunks
-    int bb_occ[3] = {0, 0, 0};              // resident CTAs per SM of k_bb_block (plain, batched, adaptive)
+    int bb_occ[3][2] = {};                  // resident CTAs per SM of k_bb_block (plain, batched, adaptive; warp or CTA per coset)
     double *bk_thr = nullptr, *bk_vals = nullptr;   // adaptive sequences: thresholds, survivors' |c|
     long long bk_thr_cap = 0, bk_vals_cap = 0;
     int bk_cap = 0;
@@ -1382,9 +1382,8 @@ static BbPlan bb_plan(const unsigned *delta, long long r0, int len, int bits, in
 
 template <int NW>
 static int bb_init(pp_spv *h) {
-    if (h->bb_occ[0]) return PP_OK;
-    constexpr size_t smem = bb_smem_bytes<NW>();
-    auto set = [&](auto kern, int *occ) -> int {
+    if (h->bb_occ[0][0]) return PP_OK;
+    auto set = [&](auto kern, size_t smem, int *occ) -> int {
         CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         CU(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
         int o = 0;
@@ -1392,19 +1391,26 @@ static int bb_init(pp_spv *h) {
         *occ = std::max(1, o);
         return PP_OK;
     };
-    if constexpr (NW == 2) TRY(set(k_bb_block<2, BB_BATCH>, &h->bb_occ[1]));
-    TRY(set(k_bb_block<NW, BB_ADAPT>, &h->bb_occ[2]));
-    return set(k_bb_block<NW, BB_PLAIN>, &h->bb_occ[0]);
+    constexpr size_t sw = bb_smem_bytes<NW, 32>(), sc = bb_smem_bytes<NW, 128>();
+    if constexpr (NW == 2) {
+        TRY(set(k_bb_block<2, BB_BATCH, 32>, sw, &h->bb_occ[BB_BATCH][0]));
+        TRY(set(k_bb_block<2, BB_BATCH, 128>, sc, &h->bb_occ[BB_BATCH][1]));
+    }
+    TRY(set(k_bb_block<NW, BB_ADAPT, 32>, sw, &h->bb_occ[BB_ADAPT][0]));
+    TRY(set(k_bb_block<NW, BB_PLAIN, 128>, sc, &h->bb_occ[BB_PLAIN][1]));
+    return set(k_bb_block<NW, BB_PLAIN, 32>, sw, &h->bb_occ[BB_PLAIN][0]);
 }
 
+// cta: the CTA per coset (else a warp).
 template <int NW>
-static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl) {
+static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl, bool cta) {
     const int mode = A.thr ? BB_ADAPT : NW == 2 && h->batch_on ? BB_BATCH : BB_PLAIN;
+    const int groups = cta ? 1 : BB_WARPS;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)std::min(((1ll << (pl.bits - pl.d)) + BB_WARPS - 1) / BB_WARPS,
-                                          (long long)h->nsm * h->bb_occ[mode]));
+    cfg.gridDim = dim3((unsigned)std::min(((1ll << (pl.bits - pl.d)) + groups - 1) / groups,
+                                          (long long)h->nsm * h->bb_occ[mode][cta ? 1 : 0]));
     cfg.blockDim = dim3(32 * BB_WARPS);
-    cfg.dynamicSmemBytes = bb_smem_bytes<NW>();
+    cfg.dynamicSmemBytes = cta ? bb_smem_bytes<NW, 128>() : bb_smem_bytes<NW, 32>();
     cfg.stream = h->stream;
     // programmatic dependent launch: a block's prologue overlaps the previous block's tail
     cudaLaunchAttribute at[1];
@@ -1412,28 +1418,29 @@ static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaError_t e;
-    if (mode == BB_ADAPT) e = cudaLaunchKernelEx(&cfg, k_bb_block<NW, BB_ADAPT>, A, pl);
-    else if (mode == BB_PLAIN) e = cudaLaunchKernelEx(&cfg, k_bb_block<NW, BB_PLAIN>, A, pl);
-    else if constexpr (NW == 2) e = cudaLaunchKernelEx(&cfg, k_bb_block<2, BB_BATCH>, A, pl);
-    else e = cudaErrorInvalidValue;
+    cudaError_t e = cudaErrorInvalidValue;
+    if (mode == BB_ADAPT) e = cudaLaunchKernelEx(&cfg, k_bb_block<NW, BB_ADAPT, 32>, A, pl);
+    else if (mode == BB_PLAIN) e = cudaLaunchKernelEx(&cfg, cta ? k_bb_block<NW, BB_PLAIN, 128> : k_bb_block<NW, BB_PLAIN, 32>, A, pl);
+    else if constexpr (NW == 2) e = cudaLaunchKernelEx(&cfg, cta ? k_bb_block<2, BB_BATCH, 128> : k_bb_block<2, BB_BATCH, 32>, A, pl);
     return e == cudaSuccess ? PP_OK : fail(PP_DEVICE_ERROR, std::string("launch failure: ") + cudaGetErrorString(e));
 }
 
-// Dimension of the cosets for n live terms in 2^bits buckets.  While the cosets are
-// fewer than the resident warps, a block's time is that of one warp's chain of steps,
-// which hardly depends on the coset's size up to about 128 terms (one scan, one batch
-// of pairs): larger cosets mean more rotations a launch.  With more cosets than that,
-// cosets as large as leave the resident set room for growth fill the warps' batches.
-static int bb_dims(long long n, int bits, int slots, int limit, long long warps) {
+// Dimension of the cosets for n live terms in 2^bits buckets, and whether a CTA or a
+// warp takes a coset.  Below BB_CTA_MAX terms the SMs are not full of warps' work and a
+// block's time is its chain of steps: a CTA per coset has the shorter chain, and cosets of
+// up to BB_CTA_TERMS terms (more rotations a launch) cost it little.  Above, a warp per
+// coset: no barriers, and cosets as large as leave the resident set room for growth fill
+// the warps' batches.  (127-qubit graph, 8e4 terms: 16.3 ms with the line at 3e5, 18.8 at
+// 6e4; cosets of 256 or 800 terms 18.9 and 18.5; a 36-qubit batch of 1e6: 38 and 41.)
+static constexpr long long BB_CTA_MAX = 300000;
+static constexpr long long BB_CTA_TERMS = 512;
+template <int NW>
+static int bb_dims(long long n, int bits, int limit, bool *cta) {
+    *cta = n <= BB_CTA_MAX;
+    // (a set that may double within the block: 3/4 of the slots at most)
+    const long long most = *cta ? BB_CTA_TERMS : 3 * bb_slots<NW, 32>() / 4;
     int d = 1;
-    while (d < limit && d < bits) {
-        const long long mean_num = n << (d + 1);                  // terms of a coset of d + 1 dimensions, times 2^bits
-        const bool small = mean_num <= (128ll << bits);
-        const bool fits = 4 * mean_num <= 3 * ((long long)slots << bits);
-        if (!(small || (fits && (1ll << (bits - d - 1)) >= warps))) break;
-        ++d;
-    }
+    while (d < limit && d < bits && (n << (d + 1)) <= (most << bits)) ++d;
     return d;
 }
 
@@ -1578,7 +1585,8 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
             return fail(PP_ERROR_EXCEPTION, "internal error: inconsistent bucket layout before a launch");
         const int slot = (int)(seq & 1);
         const BkArgs A = bk_args(h, bits, h->bk_rec);
-        const int dims = bb_dims(n, bits, bb_slots<NW>(), limit, (long long)h->nsm * BB_WARPS * h->bb_occ[0]);
+        bool cta = false;
+        const int dims = bb_dims<NW>(n, bits, limit, &cta);
         Chunk c{(long long)blocks.size(), 0, n, dims};
         if (timed && !per_rot) CU(cudaEventRecord(cev[slot][0], s));
         while (launched < end) {
@@ -1593,7 +1601,7 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
             pl.kprev = blocks.empty() ? 0 : blocks.back().K;
             pl.cur = cur;
             if (per_rot) CU(cudaEventRecord(cev[slot][0], s));
-            TRY(bb_launch<NW>(h, A, pl));
+            TRY(bb_launch<NW>(h, A, pl, cta));
             if (per_rot) {
                 CU(cudaEventRecord(cev[slot][1], s));
                 TRY(sync_check(h));
@@ -2204,7 +2212,9 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
         A.thr = h->bk_thr;
         A.vals = h->bk_vals;
         A.vals_cap = h->bk_vals_cap;
-        const int dims = bb_dims(most, bits, bb_slots<NW>(), limit, (long long)h->nsm * BB_WARPS * h->bb_occ[2]);
+        // a block of one rotation: cosets of about 64 terms, a warp each
+        int dims = 1;
+        while (dims < limit && dims < bits && (most << (dims + 1)) <= (64ll << bits)) ++dims;
         st.bk_fail = 0x7fffffffffffffffll;
         st.bk_pad = 0;
         TRY(write_state(h, &st));
@@ -2212,7 +2222,7 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
             BbPlan pl = bb_plan(delta.data(), r, 1, bits, dims);
             pl.cur = (cur + (int)(r - done)) & 1;
             pl.prechan = r > start && (h->gens_h[r - 1].flags & chan_flags) && h->Ph->chan_kind >= 0 ? 1 : 0;
-            TRY(bb_launch<NW>(h, A, pl));
+            TRY(bb_launch<NW>(h, A, pl, false));
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(1);
             cfg.blockDim = dim3(AS_THREADS);

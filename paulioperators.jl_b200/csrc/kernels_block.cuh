@@ -16,17 +16,19 @@
 // values may not have passed it: at the first rotation of a call and after a
 // channel (a block ends at a channel, which scales every survivor at its end).
 //
-// What bounds it: latency and instruction issue.  At 8e5 terms a block of six
-// rotations takes 64 us, of which DRAM traffic would take 10: a warp issues one
-// instruction every 11 cycles (fixed latencies, shared memory), and twelve warps are
-// what the resident sets leave room for.  A warp per coset, not a CTA: with a CTA of
-// eight warps per coset each warp found too few anticommuting terms to fill a batch,
-// and waited at a barrier per rotation (130 against 102 ms for the lattice circuit
-// below).  The index over all resident terms is built once per block and pays from
-// about three rotations on.
+// What bounds it: latency and instruction issue, and above a million terms the scattered
+// reads and writes of short bucket runs.  A warp issues one instruction every 11 cycles
+// (fixed latencies, shared memory), and twelve warps are what the resident sets leave
+// room for.  Large sets: a warp per coset, no block barrier between rotations.  Small
+// sets (an SM has a few cosets at most): a CTA per coset, whose chain of a rotation is
+// shorter -- a thread per slot, or a batch per warp -- and whose larger resident set
+// takes more rotations per launch.  The index over all resident terms is built once per
+// block and pays from about three rotations on.
 // Measured (one B200, whole calls, one rotation per launch before): 8 x 8 lattice,
-// 3,520 rotations, up to 3.9e6 terms 154.9 -> 101.7 ms; 127-qubit graph, 6,504
-// rotations, up to 8e4 terms 43.4 -> 23.0 ms; 48 batched instances 60.1 -> 40.9 ms.
+// 3,520 rotations, up to 3.9e6 terms 154.9 -> 95 ms; 127-qubit graph, 6,504 rotations, up
+// to 8e4 terms 43.4 -> 16.3 ms; 48 batched instances 60.1 -> 38 ms.  (A warp per coset
+// everywhere: 109, 19.6 and 42.6; a CTA everywhere: 111, 16.2 and 38.4 with cosets of 512
+// terms, 96, 18.9 and 38.4 with cosets of 900.)
 #pragma once
 #include "kernels_bucket.cuh"
 
@@ -37,22 +39,24 @@ constexpr int BB_CAP_LOG = 5;
 constexpr int BB_KMAX = 8;                     // rotations of a block at most
 constexpr int BB_DMAX = 8;                     // dimension of a coset at most
 constexpr int BB_MEMBERS = 1 << BB_DMAX;       // buckets of a coset at most
-constexpr int BB_WARPS = 4;                    // warps of a CTA, each with a coset of its own
+constexpr int BB_WARPS = 4;                    // warps of a CTA
 constexpr unsigned BB_DEAD = 0x8000u;          // tag bit: the slot holds no live term
 
-// Slots of a warp's resident set and of its key index (twelve warps fit on an SM).
-template <int NW>
-__host__ __device__ constexpr int bb_slots() { return NW == 1 ? 448 : 288; }
-constexpr int BB_TAB = 1024;
+// Slots of the resident set and of its key index that T threads share: a warp (T = 32;
+// twelve fit on an SM) or the CTA (T = 128; three).
+template <int NW, int T>
+__host__ __device__ constexpr int bb_slots() { return T == 32 ? (NW == 1 ? 448 : 288) : (NW == 1 ? 1920 : 1152); }
+template <int T>
+__host__ __device__ constexpr int bb_tab() { return T == 32 ? 1024 : 4096; }
 
 constexpr int RS_QCAP = 160;                   // entries of a warp's queue of slots (31 + 4 * 32 at most)
 
 // Shared memory of one resident set: coefficients, key words, index, tags.
 template <int NW, int SLOTS, int TAB>
 __host__ __device__ constexpr size_t rs_set_bytes() { return (size_t)SLOTS * (8 + 16 * NW + 2) + (size_t)TAB * 4; }
-template <int NW>
+template <int NW, int T>
 __host__ __device__ constexpr size_t bb_smem_bytes() {
-    return BB_WARPS * (rs_set_bytes<NW, bb_slots<NW>(), BB_TAB>() + RS_QCAP * 2);
+    return 32 * BB_WARPS / T * rs_set_bytes<NW, bb_slots<NW, T>(), bb_tab<T>()>() + BB_WARPS * RS_QCAP * 2;
 }
 
 // One rotation as the steps use it: the generator's key words in 32-bit pieces
@@ -450,36 +454,47 @@ constexpr int BB_PLAIN = 0, BB_BATCH = 1, BB_ADAPT = 2;
 // an output bucket beyond BB_CAP -- is flagged and run again by the host, after a
 // split or with fewer rotations).  Persistent grid; every warp takes cosets of its
 // own, so no block barrier stands between a rotation and the next.
-template <int NW, int MODE>
+template <int NW, int MODE, int T>
 __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_constant__ BkArgs A,
                                                                const __grid_constant__ BbPlan pl) {
     constexpr bool BATCH = MODE == BB_BATCH;
     constexpr bool ADAPT = MODE == BB_ADAPT;
-    constexpr int SLOTS = bb_slots<NW>();
-    constexpr int TAB = BB_TAB;
+    constexpr int SLOTS = bb_slots<NW, T>();
+    constexpr int TAB = bb_tab<T>();
+    constexpr int GROUPS = 32 * BB_WARPS / T;              // cosets a CTA works on at a time
+    constexpr int ME = BB_MEMBERS / T;                     // members per thread at most
+    static_assert(T == 32 || T == 32 * BB_WARPS, "a warp or the CTA per coset");
     static_assert(2 * 2 * BB_CAP <= SLOTS, "a block of one rotation always fits");
     static_assert(!BATCH || NW == 2, "batched instances use two-word keys");
     DevState *S = A.S;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ RsGen<NW> s_g[BB_KMAX];
     __shared__ int s_x[BB_MEMBERS];                        // a member's place in its coset
-    __shared__ int s_cw[BB_WARPS][BB_MEMBERS];
-    __shared__ unsigned short s_ow[BB_WARPS][BB_MEMBERS];
-    __shared__ int s_fw[BB_WARPS][2];                      // fresh slots of the step, resident set full
+    __shared__ int s_cw[GROUPS][BB_MEMBERS];
+    __shared__ unsigned short s_ow[GROUPS][BB_MEMBERS];
+    __shared__ int s_fw[GROUPS][BB_KMAX + 1];              // fresh slots of each step, resident set full
+    __shared__ int s_aw[GROUPS][BB_KMAX + 1][2];           // change of the live count, sin branches of each step
+    __shared__ int s_scan[BB_WARPS + 1];
     __shared__ int s_tot[BB_KMAX][2], s_np, s_mx, s_over, s_err, s_pref, s_bad;
     __shared__ double s_thr;
     extern __shared__ __align__(16) unsigned char bbm[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gt = tid & (T - 1), grp = tid / T;           // thread of the group, group of the CTA
+    auto sync = [&]() {
+        if constexpr (T == 32) __syncwarp();
+        else __syncthreads();
+    };
     ResidentSet<NW, SLOTS, TAB> set;
-    unsigned char *mine = bbm + warp * rs_set_bytes<NW, SLOTS, TAB>();
+    unsigned char *mine = bbm + grp * rs_set_bytes<NW, SLOTS, TAB>();
     set.c = reinterpret_cast<double *>(mine);
     set.w = reinterpret_cast<unsigned *>(set.c + SLOTS);
     set.tab = set.w + 4 * NW * SLOTS;
     set.tag = reinterpret_cast<unsigned short *>(set.tab + TAB);
-    unsigned short *queue = reinterpret_cast<unsigned short *>(bbm + BB_WARPS * rs_set_bytes<NW, SLOTS, TAB>()) + warp * RS_QCAP;
-    int *scnt = s_cw[warp];
-    unsigned short *soff = s_ow[warp];
-    int *fresh = &s_fw[warp][0], *full = &s_fw[warp][1];
+    unsigned short *queue = reinterpret_cast<unsigned short *>(bbm + GROUPS * rs_set_bytes<NW, SLOTS, TAB>()) + warp * RS_QCAP;
+    int *scnt = s_cw[grp];
+    unsigned short *soff = s_ow[grp];
+    int *fresh = s_fw[grp], *full = &s_fw[grp][BB_KMAX];
+    int (*acc)[2] = s_aw[grp];
     const int K = pl.K, d = pl.d, mem = 1 << d;
     const long long r0 = pl.r0;
     for (int j = warp; j < K; j += BB_WARPS) rs_gen<NW>(&s_g[j], A.gens[r0 + j], pl.dl[j]);
@@ -492,7 +507,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
             if ((m >> e) & 1) b ^= pl.basis[e];
         s_x[m] = (int)b;
     }
-    for (int i = lane; i < TAB / 4; i += 32) reinterpret_cast<uint4 *>(set.tab)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (int i = gt; i < TAB / 4; i += T) reinterpret_cast<uint4 *>(set.tab)[i] = make_uint4(0u, 0u, 0u, 0u);
     const DevParams &P = *A.P;
     RsParams q;
     q.strict = fquick(P.strict);
@@ -556,22 +571,39 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
         return;
     }
     const long long ncos = nb >> d;
-    int tot_out = 0, tot_cre = 0;                          // lane j < K: rotation r0 + j
-    int tot_np = 0, mx = 0;
+    int tot_out = 0, tot_cre = 0;                          // thread j < K of the group: rotation r0 + j
+    int tot_np = 0, mx = 0;                                // (tot_np: the group's thread 0)
     bool over = false;
-    for (long long cs = blockIdx.x * BB_WARPS + warp; cs < ncos; cs += (long long)gridDim.x * BB_WARPS) {
+    // one barrier has to follow a step's counts before they are read: with a warp per
+    // coset they stay in registers, with a CTA they meet in acc[j]
+    auto counted = [&](int out, int j) {                   // call with the whole group; returns after the barrier
+        out = __reduce_add_sync(0xffffffffu, out);
+        if constexpr (T == 32) {
+            sync();
+            return out;
+        } else {
+            if (lane == 0 && out) {
+                const int dn = (int)(short)(out & 0xffff);
+                atomicAdd(&acc[j][0], dn);
+                atomicAdd(&acc[j][1], (out - dn) >> 16);
+            }
+            sync();
+            return 0;
+        }
+    };
+    for (long long cs = (long long)blockIdx.x * GROUPS + grp; cs < ncos; cs += (long long)gridDim.x * GROUPS) {
         // ---- the coset's buckets and their places in the resident set
         int total = 0;
         unsigned rep = (unsigned)cs;                       // member m is bucket rep ^ s_x[m]
+        for (int e = 0; e < d; ++e) {
+            const int p = pl.piv[e];
+            rep = ((rep >> p) << (p + 1)) | (rep & ((1u << p) - 1u));
+        }
         {
-            for (int e = 0; e < d; ++e) {
-                const int p = pl.piv[e];
-                rep = ((rep >> p) << (p + 1)) | (rep & ((1u << p) - 1u));
-            }
-            int nm[BB_MEMBERS / 32];
+            int nm[ME];
 #pragma unroll
-            for (int e = 0; e < BB_MEMBERS / 32; ++e) {
-                const int m = 32 * e + lane;
+            for (int e = 0; e < ME; ++e) {
+                const int m = T * e + gt;
                 nm[e] = 0;
                 if (m < mem) {
                     const unsigned b = rep ^ (unsigned)s_x[m];
@@ -579,35 +611,45 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                     else { flag_bounds(S, 3, b); s_bad = 1; }
                 }
             }
+            if (gt <= BB_KMAX) {
+                fresh[gt] = 0;                             // and *full
+                acc[gt][0] = acc[gt][1] = 0;
+            }
 #pragma unroll
-            for (int e = 0; e < BB_MEMBERS / 32; ++e) {
-                if (32 * e < mem) {
+            for (int e = 0; e < ME; ++e) {
+                if (T * e < mem) {                         // uniform
                     if (nm[e] < 0 || nm[e] > BB_CAP) { flag_bounds(S, 4, nm[e]); s_bad = 1; nm[e] = 0; }
-                    const int inc = warp_incl_scan(nm[e], OpSum());
-                    const int m = 32 * e + lane;
-                    const int o = total + inc - nm[e];
+                    int o, sum;
+                    if constexpr (T == 32) {
+                        const int inc = warp_incl_scan(nm[e], OpSum());
+                        o = total + inc - nm[e];
+                        sum = __shfl_sync(0xffffffffu, inc, 31);
+                    } else {
+                        o = total + block_excl_scan<T>(nm[e], 0, OpSum(), s_scan, &sum);
+                    }
+                    const int m = T * e + gt;
                     if (m < mem) {
                         soff[m] = (unsigned short)o;
                         scnt[m] = 0;
                         if (o + nm[e] <= SLOTS)            // each slot's bucket
                             for (int t = 0; t < nm[e]; ++t) set.tag[o + t] = (unsigned short)m;
                     }
-                    total += __shfl_sync(0xffffffffu, inc, 31);
+                    total += sum;
                 }
             }
-            if (lane == 0) { *fresh = 0; *full = 0; }
-            __syncwarp();
+            sync();
         }
         if (total > SLOTS) { over = true; continue; }      // uniform
-        // ---- load and index, four terms a lane in flight
+        // ---- load and index, LU terms a thread in flight
+        constexpr int LU = 2;
         int dropped = 0;
-        for (int b0 = 0; b0 < total; b0 += 128) {
-            Key<NW> kk[4];
-            double cc[4];
-            int lb[4];
+        for (int b0 = 0; b0 < total; b0 += LU * T) {
+            Key<NW> kk[LU];
+            double cc[LU];
+            int lb[LU];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = b0 + u * 32 + lane;
+            for (int u = 0; u < LU; ++u) {
+                const int i = b0 + u * T + gt;
                 if (i < total) {
                     lb[u] = set.tag[i];
                     const long long o = ((long long)(rep ^ (unsigned)s_x[lb[u]]) << BB_CAP_LOG) + (i - soff[lb[u]]);
@@ -616,8 +658,8 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int i = b0 + u * 32 + lane;
+            for (int u = 0; u < LU; ++u) {
+                const int i = b0 + u * T + gt;
                 if (i < total) {
                     const Key32<NW> k = key_narrow<NW>(kk[u]);
                     bool dead = false;
@@ -636,28 +678,33 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
         }
         int alive = total;
         if (drop_first) {
-            alive -= __reduce_add_sync(0xffffffffu, dropped);
-            tot_np += alive;
+            dropped = __reduce_add_sync(0xffffffffu, dropped);
+            if constexpr (T == 32) {
+                alive -= dropped;
+            } else {
+                if (lane == 0 && dropped) atomicAdd(&acc[BB_KMAX][0], dropped);
+                sync();
+                alive -= acc[BB_KMAX][0];
+            }
+            if (gt == 0) tot_np += alive;
         }
-        __syncwarp();
+        sync();
         // ---- the K rotations
         int n = total;
         for (int j = 0; j < K; ++j) {
-            int out = rs_step<NW, SLOTS, TAB, 32, BATCH>(set, s_g[j], q, n, queue, fresh, full, r0 + j);
-            out = __reduce_add_sync(0xffffffffu, out);
-            __syncwarp();
-            n = min(n + *fresh, SLOTS);
-            __syncwarp();
-            if (lane == 0) *fresh = 0;
-            __syncwarp();
-            int dn = (int)(short)(out & 0xffff);
-            if (lane == j) tot_cre += (out - dn) >> 16;
-            if (j == 0 && pl.full) {
-                dn += __reduce_add_sync(0xffffffffu, rs_filter<NW, SLOTS, TAB, 32, BATCH>(set, q, n, r0));
-                __syncwarp();
+            int out = counted(rs_step<NW, SLOTS, TAB, T, BATCH>(set, s_g[j], q, n, queue, &fresh[j], full, r0 + j), j);
+            n = min(n + fresh[j], SLOTS);
+            if (j == 0 && pl.full) out += counted(rs_filter<NW, SLOTS, TAB, T, BATCH>(set, q, n, r0), 0);
+            int dn, cre;
+            if constexpr (T == 32) {
+                dn = (int)(short)(out & 0xffff);
+                cre = (out - dn) >> 16;
+            } else {
+                dn = acc[j][0];
+                cre = acc[j][1];
             }
             alive += dn;
-            if (lane == j) tot_out += alive;
+            if (gt == j) { tot_cre += cre; tot_out += alive; }
         }
         // ---- the survivors to their buckets of the output set, the index cleared
         if (*full) {
@@ -665,10 +712,11 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
         } else {
             long long vat = 0;                             // adaptive: where this coset's values go
             if constexpr (ADAPT) {
+                static_assert(T == 32, "adaptive sequences use a warp per coset");
                 if (lane == 0) vat = (long long)atomicAdd(&A.rec[r0 + 1].nval, (unsigned long long)alive);
                 vat = __shfl_sync(0xffffffffu, vat, 0);
             }
-            for (int base = 0; base < n; base += 32) {
+            for (int base = T == 32 ? 0 : warp * 32; base < n; base += T) {
                 const int i = base + lane;
                 const unsigned t = i < n ? set.tag[i] : BB_DEAD | 0x7fffu;
                 const bool live = !(t & BB_DEAD);
@@ -693,21 +741,21 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                 }
             }
         }
-        for (int i = lane; i < TAB / 4; i += 32) reinterpret_cast<uint4 *>(set.tab)[i] = make_uint4(0u, 0u, 0u, 0u);
-        __syncwarp();
-        for (int m = lane; m < mem; m += 32) {
+        for (int i = gt; i < TAB / 4; i += T) reinterpret_cast<uint4 *>(set.tab)[i] = make_uint4(0u, 0u, 0u, 0u);
+        sync();
+        for (int m = gt; m < mem; m += T) {
             const int c = scnt[m];
             const unsigned b = rep ^ (unsigned)s_x[m];
             if (b < nb) OCNT[b] = min(c, BB_CAP);
             mx = max(mx, c);
         }
-        __syncwarp();
+        sync();
     }
     // ---- the block's totals
     mx = __reduce_max_sync(0xffffffffu, mx);
-    if (lane < K) {
-        atomicAdd(&s_tot[lane][0], tot_out);
-        atomicAdd(&s_tot[lane][1], tot_cre);
+    if (gt < K) {
+        atomicAdd(&s_tot[gt][0], tot_out);
+        atomicAdd(&s_tot[gt][1], tot_cre);
     }
     if (lane == 0) {
         atomicMax(&s_mx, mx);

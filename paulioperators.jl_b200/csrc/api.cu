@@ -145,7 +145,7 @@ struct pp_spv {
     unsigned *bk_delta = nullptr;           // bucket hash of each generator of the call
     long long bk_delta_cap = 0;
     BkStat *bk_stat = nullptr;              // pinned, two chunks
-    int bb_occ[3][2] = {};                  // resident CTAs per SM of k_bb_block (plain, batched, adaptive; warp or CTA per coset)
+    int bb_occ[4][2] = {};                  // resident CTAs per SM of k_bb_block (each mode; warp or CTA per coset)
     double *bk_thr = nullptr, *bk_vals = nullptr;   // adaptive sequences: thresholds, survivors' |c|
     long long bk_thr_cap = 0, bk_vals_cap = 0;
     int bk_cap = 0;
@@ -1072,7 +1072,11 @@ struct RunProf {
 // (kernels_block.cuh); the sequence ends with a packing into a dense array and a
 // sort, so the live set is dense and sorted between calls as before.
 static int expect_dev(pp_spv *h, const u64 *k, double *out);
-static constexpr int BK_MIN_ROT = 32;     // shorter sequences keep the sorted-merge kernels
+// Shorter sequences keep the sorted-merge kernels, which need no conversion: into buckets
+// and back costs about 0.2 ms up to 3e5 terms and 0.7 ms for 1.5e6, and saves 0.05 and 0.08
+// ms a rotation.  (With per-rotation times asked for, only long sequences: a block has no
+// separate rotate and merge times.)
+static int bk_min_rot(long long n, bool per_rot) { return per_rot ? 32 : n <= 300000 ? 6 : 12; }
 // Internal status (never returned by the C ABI): a bucket layout for the live set
 // would not fit in device memory; the sequence continues on the sorted-merge
 // kernels from the rotation the device cursor is at.
@@ -1380,6 +1384,8 @@ static BbPlan bb_plan(const unsigned *delta, long long r0, int len, int bits, in
     return pl;
 }
 
+static int norm2_dev(pp_spv *h, int cur, long long n, double *out);
+
 template <int NW>
 static int bb_init(pp_spv *h) {
     if (h->bb_occ[0][0]) return PP_OK;
@@ -1398,13 +1404,15 @@ static int bb_init(pp_spv *h) {
     }
     TRY(set(k_bb_block<NW, BB_ADAPT, 32>, sw, &h->bb_occ[BB_ADAPT][0]));
     TRY(set(k_bb_block<NW, BB_PLAIN, 128>, sc, &h->bb_occ[BB_PLAIN][1]));
+    TRY(set(k_bb_block<NW, BB_ENERGY, 32>, sw, &h->bb_occ[BB_ENERGY][0]));
+    TRY(set(k_bb_block<NW, BB_ENERGY, 128>, sc, &h->bb_occ[BB_ENERGY][1]));
     return set(k_bb_block<NW, BB_PLAIN, 32>, sw, &h->bb_occ[BB_PLAIN][0]);
 }
 
 // cta: the CTA per coset (else a warp).
 template <int NW>
 static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl, bool cta) {
-    const int mode = A.thr ? BB_ADAPT : NW == 2 && h->batch_on ? BB_BATCH : BB_PLAIN;
+    const int mode = A.thr ? BB_ADAPT : NW == 2 && h->batch_on ? BB_BATCH : A.energy ? BB_ENERGY : BB_PLAIN;
     const int groups = cta ? 1 : BB_WARPS;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)std::min(((1ll << (pl.bits - pl.d)) + groups - 1) / groups,
@@ -1420,6 +1428,7 @@ static int bb_launch(pp_spv *h, const BkArgs &A, const BbPlan &pl, bool cta) {
     cfg.numAttrs = 1;
     cudaError_t e = cudaErrorInvalidValue;
     if (mode == BB_ADAPT) e = cudaLaunchKernelEx(&cfg, k_bb_block<NW, BB_ADAPT, 32>, A, pl);
+    else if (mode == BB_ENERGY) e = cudaLaunchKernelEx(&cfg, cta ? k_bb_block<NW, BB_ENERGY, 128> : k_bb_block<NW, BB_ENERGY, 32>, A, pl);
     else if (mode == BB_PLAIN) e = cudaLaunchKernelEx(&cfg, cta ? k_bb_block<NW, BB_PLAIN, 128> : k_bb_block<NW, BB_PLAIN, 32>, A, pl);
     else if constexpr (NW == 2) e = cudaLaunchKernelEx(&cfg, cta ? k_bb_block<2, BB_BATCH, 128> : k_bb_block<2, BB_BATCH, 32>, A, pl);
     return e == cudaSuccess ? PP_OK : fail(PP_DEVICE_ERROR, std::string("launch failure: ") + cudaGetErrorString(e));
@@ -1464,6 +1473,17 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
     if (L > h->bk_delta_cap) {
         TRY(dalloc(h, &h->bk_delta, L));
         h->bk_delta_cap = L;
+    }
+    // EnergyCorrection: the dropped values are added up as multiples of a unit under the
+    // 2-norm of the entering set, which no rotation, filter or channel enlarges
+    double escale = 0.0;
+    if (h->Ph->corr_kind == 1) {
+        double nrm = 0.0;
+        TRY(norm2_dev(h, st.cur, n0, &nrm));
+        if (!std::isfinite(nrm) || nrm > 0x1p900) return BK_NOFIT;         // (the sorted-merge kernels add doubles)
+        int e = 0;
+        std::frexp(nrm, &e);
+        escale = std::ldexp(1.0, -std::max(e + 1, -900));
     }
     BkRec r0;
     memset(&r0, 0, sizeof r0);
@@ -1540,6 +1560,14 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         for (const Block &b : blocks)      // a block reads its first rotation's terms and writes its last one's
             prof->bk_bytes += (double)(16 * NW + 8) * ((double)rec[(size_t)(b.r0 - start)].n_out +
                                                        (double)rec[(size_t)(b.r0 + b.K - start)].n_out);
+        if (escale != 0.0) {
+            __int128 e[3] = {0, 0, 0};
+            for (const Block &b : blocks)
+                for (int t = 0; t < 3; ++t) e[t] += (long long)rec[(size_t)(b.r0 + 1 - start)].energy[t];
+            // smallest unit first: one rounding each
+            const double sum = (double)e[2] * 0x1p-110 + (double)e[1] * 0x1p-70 + (double)e[0] * 0x1p-30;
+            st.corr_energy -= sum / escale;
+        }
         if (h->rec_on && upto > start)
             CU(cudaMemcpy(h->rec + 4 * start, rr.data(), rr.size() * sizeof(long long), cudaMemcpyHostToDevice));
         st.acap_logical = acap;
@@ -1584,7 +1612,9 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         if (bits < 1 || bits > h->bk_bits_cap || h->bk_cap != BB_CAP || L + 1 > h->bk_rec_cap || (cur & ~1))
             return fail(PP_ERROR_EXCEPTION, "internal error: inconsistent bucket layout before a launch");
         const int slot = (int)(seq & 1);
-        const BkArgs A = bk_args(h, bits, h->bk_rec);
+        BkArgs A = bk_args(h, bits, h->bk_rec);
+        A.energy = escale != 0.0 ? 1 : 0;
+        A.escale = escale;
         bool cta = false;
         const int dims = bb_dims<NW>(n, bits, limit, &cta);
         Chunk c{(long long)blocks.size(), 0, n, dims};
@@ -1715,10 +1745,10 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
     std::vector<cudaEvent_t> ev;   // 5 per rotation when timed
     bool table = false;            // the device segment table describes the (dense) live set
     const bool small_ok = !per_rot && !h->batch_on && !h->Ph->local_active && h->Ph->corr_kind == 0;
-    bool use_bk = bk_enabled() && h->Ph->corr_kind == 0;
+    bool use_bk = bk_enabled();
     long long ncur = small_cap<NW>() + 1;   // live terms at the chunk's start (read when small_ok)
     bool dense = false;                      // the last state read showed a dense live set
-    if (small_ok) {
+    if (small_ok || n_known >= 0) {
         if (n_known >= 0) {
             ncur = n_known;
         } else {
@@ -1743,7 +1773,7 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
             done = st.rot;
             continue;
         }
-        if (use_bk && L - done >= BK_MIN_ROT) {
+        if (use_bk && L - done >= bk_min_rot(ncur, per_rot)) {
             const int rb = run_bucket<NW>(h, done, L, ctr, prof, per_rot);
             if (rb != BK_NOFIT) return rb;
             bk_release(h);                  // their memory goes to the sorted-merge kernels
@@ -3707,6 +3737,27 @@ extern "C" int pp_scale(pp_spv *h, double a) {
     TRY(read_state(h, &st));
     if (st.n > 0) k_scale<<<h->nsm * 8, 256, 0, h->stream>>>(h->c[st.cur], st.n, a);
     return sync_check(h);
+}
+
+// The 2-norm of n coefficients of set cur (to a few roundings).
+static int norm2_dev(pp_spv *h, int cur, long long n, double *out) {
+    *out = 0.0;
+    if (n == 0) return PP_OK;
+    Scratch sc(h);
+    const int nb = std::min(4096, h->nsm * 8);
+    double *part, *res, *val;
+    TRY(sc.get(&part, nb));
+    TRY(sc.get(&res, 1));
+    TRY(sc.get(&val, n));
+    cudaStream_t s = h->stream;
+    k_norm_terms<<<h->nsm * 8, 256, 0, s>>>(h->c[cur], n, 2.0, val);
+    k_sum_partials<<<nb, 256, 0, s>>>(val, n, part);
+    k_expect_final<<<1, EF_THREADS, 0, s>>>(part, nb, res);
+    double r = 0.0;
+    CU(cudaMemcpyAsync(&r, res, sizeof r, cudaMemcpyDeviceToHost, s));
+    TRY(sync_check(h));
+    *out = std::sqrt(r);
+    return PP_OK;
 }
 
 extern "C" int pp_norm(pp_spv *h, double p, double *out) {

@@ -260,15 +260,44 @@ __device__ __forceinline__ bool rs_drop(const RsParams &q, const Key32<NW> &k, d
     return (absc <= q.strict.thresh) | rs_heavy<NW>(q, k);
 }
 
+// <ket|.|ket> of dropped terms (EnergyCorrection), added up exactly: a value, scaled to
+// at most 1 in magnitude, is cut into whole multiples of 2^-30, 2^-70 and 2^-110, whose
+// sums do not depend on the order.
+template <int NW>
+struct RsEnergy {
+    long long a[3];
+    unsigned ket[2 * NW];
+    double scale;
+    __device__ __forceinline__ void add(const Key32<NW> &k, double v) {
+        unsigned x = 0, s = 0;
+#pragma unroll
+        for (int t = 0; t < 2 * NW; ++t) {
+            x |= k.w[2 * NW + t];
+            s ^= k.w[t] & ket[t];
+        }
+        if (x) return;
+        double r = v * scale;
+        if (__popc(s) & 1) r = -r;
+        const double g[3] = {0x1p30, 0x1p70, 0x1p110}, u[3] = {0x1p-30, 0x1p-70, 0x1p-110};
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            const long long q = __double2ll_rn(r * g[t]);
+            a[t] += q;
+            r = __dsub_rn(r, (double)q * u[t]);            // exact: |q| < 2^53
+        }
+    }
+};
+
 // One rotation on one anticommuting slot i of the resident set.  Of two partners'
 // slots (live or not) the lower runs it for both, so every slot has one writer in a
 // step and no barrier is needed between the reads and the writes of a pair's
 // coefficients.  A sin branch without a slot is appended at n0 + atomicAdd(*fresh).
 // Returns the change of the live count in the low half and the sin branches appended
 // (WindowCounters) in the high half.
-template <int NW, int SLOTS, int TAB, bool BATCH>
+// en: nullptr, or where dropped values are added up.
+template <int NW, int SLOTS, int TAB, bool BATCH, bool ENERGY>
 __device__ __forceinline__ int rs_pair(const ResidentSet<NW, SLOTS, TAB> &s, const RsGen<NW> &g, const RsParams &q, int i,
-                                       int n0, int *fresh, int *full, long long r) {
+                                       int n0, int *fresh, int *full, long long r, RsEnergy<NW> *en) {
     const unsigned ti = s.tag[i];
     const double ci = s.c[i];
     const Key32<NW> k = s.key(i);
@@ -321,6 +350,10 @@ __device__ __forceinline__ int rs_pair(const ResidentSet<NW, SLOTS, TAB> &s, con
         ki &= !((fabs(vi) <= q.strict.thresh) | hk);
         kj &= !((fabs(vj) <= q.strict.thresh) | hq);
     }
+    if constexpr (ENERGY) {
+        if ((ai | okj) && !ki) en->add(k, vi);
+        if ((aj | oki) && !kj) en->add(p, vj);
+    }
     if (ki) s.c[i] = vi;
     if (ki != ai) s.tag[i] = (unsigned short)(ti ^ BB_DEAD);
     if (j >= 0) {
@@ -346,9 +379,10 @@ __device__ __forceinline__ int rs_pair(const ResidentSet<NW, SLOTS, TAB> &s, con
 // anticommuting ones, and runs rs_pair on 32 of them at a time, so that the long path
 // runs with full warps although only about a tenth of the terms take it.  Returns
 // this thread's rs_pair sums.
-template <int NW, int SLOTS, int TAB, int T, bool BATCH>
+template <int NW, int SLOTS, int TAB, int T, bool BATCH, bool ENERGY = false>
 __device__ __forceinline__ int rs_step(const ResidentSet<NW, SLOTS, TAB> &s, const RsGen<NW> &g, const RsParams &q, int n,
-                                       unsigned short *queue, int *fresh, int *full, long long r) {
+                                       unsigned short *queue, int *fresh, int *full, long long r,
+                                       RsEnergy<NW> *en = nullptr) {
     const int lane = threadIdx.x & 31, warp = T == 32 ? 0 : threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1u;
     int cnt = 0, out = 0;
@@ -359,7 +393,7 @@ __device__ __forceinline__ int rs_step(const ResidentSet<NW, SLOTS, TAB> &s, con
             unsigned a = 0;
             if (i < n)
                 for (int t = 0; t < np; ++t) a ^= s.w[g.plane[t] * SLOTS + i] & g.mask[t];
-            return __popc(a) & 1 ? rs_pair<NW, SLOTS, TAB, BATCH>(s, g, q, i, n, fresh, full, r) : 0;
+            return __popc(a) & 1 ? rs_pair<NW, SLOTS, TAB, BATCH, ENERGY>(s, g, q, i, n, fresh, full, r, en) : 0;
         }
     }
     const int p0 = g.plane[0] * SLOTS;
@@ -395,7 +429,7 @@ __device__ __forceinline__ int rs_step(const ResidentSet<NW, SLOTS, TAB> &s, con
         while (cnt >= 32 || (!more && cnt > 0)) {
             const int take = min(cnt, 32);
             cnt -= take;
-            if (lane < take) out += rs_pair<NW, SLOTS, TAB, BATCH>(s, g, q, queue[cnt + lane], n, fresh, full, r);
+            if (lane < take) out += rs_pair<NW, SLOTS, TAB, BATCH, ENERGY>(s, g, q, queue[cnt + lane], n, fresh, full, r, en);
             __syncwarp();
         }
         if (!more) break;
@@ -405,8 +439,9 @@ __device__ __forceinline__ int rs_step(const ResidentSet<NW, SLOTS, TAB> &s, con
 
 // The strict filter over every live slot (terms whose values have not passed it yet);
 // returns the change of the live count.
-template <int NW, int SLOTS, int TAB, int T, bool BATCH>
-__device__ __forceinline__ int rs_filter(const ResidentSet<NW, SLOTS, TAB> &s, const RsParams &q, int n, long long r) {
+template <int NW, int SLOTS, int TAB, int T, bool BATCH, bool ENERGY = false>
+__device__ __forceinline__ int rs_filter(const ResidentSet<NW, SLOTS, TAB> &s, const RsParams &q, int n, long long r,
+                                         RsEnergy<NW> *en = nullptr) {
     int out = 0;
     for (int i = threadIdx.x & (T - 1); i < n; i += T) {
         const unsigned t = s.tag[i];
@@ -418,6 +453,7 @@ __device__ __forceinline__ int rs_filter(const ResidentSet<NW, SLOTS, TAB> &s, c
         if (rs_drop<NW>(q, k, fabs(s.c[i]))) {
             s.tag[i] = (unsigned short)(t | BB_DEAD);
             out -= 1;
+            if constexpr (ENERGY) en->add(k, s.c[i]);
         }
     }
     return out;
@@ -446,8 +482,8 @@ __global__ void k_bb_deltas(const GenRec *gens, long long n, const u64 *rows, un
 // rotation, unfiltered: the terms that AdaptiveTruncation drops after the previous
 // rotation -- |c| at most thr[r0] -- are dropped as they are loaded, a channel between
 // the two (pl.prechan) is applied there, and the survivors' |c| are listed for the next
-// threshold).
-constexpr int BB_PLAIN = 0, BB_BATCH = 1, BB_ADAPT = 2;
+// threshold); plain with EnergyCorrection.
+constexpr int BB_PLAIN = 0, BB_BATCH = 1, BB_ADAPT = 2, BB_ENERGY = 3;
 
 // One block of rotations; input bucket set pl.cur, output set pl.cur ^ 1 (the input
 // stays intact, so a block that does not fit -- a coset beyond the resident set, or
@@ -459,6 +495,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                                                                const __grid_constant__ BbPlan pl) {
     constexpr bool BATCH = MODE == BB_BATCH;
     constexpr bool ADAPT = MODE == BB_ADAPT;
+    constexpr bool ENERGY = MODE == BB_ENERGY;
     constexpr int SLOTS = bb_slots<NW, T>();
     constexpr int TAB = bb_tab<T>();
     constexpr int GROUPS = 32 * BB_WARPS / T;              // cosets a CTA works on at a time
@@ -574,6 +611,12 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     int tot_out = 0, tot_cre = 0;                          // thread j < K of the group: rotation r0 + j
     int tot_np = 0, mx = 0;                                // (tot_np: the group's thread 0)
     bool over = false;
+    RsEnergy<NW> en = {};
+    if constexpr (ENERGY) {
+        en.scale = A.escale;
+#pragma unroll
+        for (int t = 0; t < 2 * NW; ++t) en.ket[t] = (unsigned)(P.ket[t >> 1] >> (32 * (t & 1)));
+    }
     // one barrier has to follow a step's counts before they are read: with a warp per
     // coset they stay in registers, with a CTA they meet in acc[j]
     auto counted = [&](int out, int j) {                   // call with the whole group; returns after the barrier
@@ -669,6 +712,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                     } else if (drop_first) {
                         dead = rs_drop<NW>(q, k, fabs(cc[u]));
                         if constexpr (BATCH) dead = dead && rs_instance<NW>(k, q, r0) >= 0;
+                        if constexpr (ENERGY) { if (dead) en.add(k, cc[u]); }
                     }
                     dropped += dead ? 1 : 0;
                     set.put(i, k, cc[u], (unsigned)lb[u] | (dead ? BB_DEAD : 0u));
@@ -692,9 +736,9 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
         // ---- the K rotations
         int n = total;
         for (int j = 0; j < K; ++j) {
-            int out = counted(rs_step<NW, SLOTS, TAB, T, BATCH>(set, s_g[j], q, n, queue, &fresh[j], full, r0 + j), j);
+            int out = counted(rs_step<NW, SLOTS, TAB, T, BATCH, ENERGY>(set, s_g[j], q, n, queue, &fresh[j], full, r0 + j, &en), j);
             n = min(n + fresh[j], SLOTS);
-            if (j == 0 && pl.full) out += counted(rs_filter<NW, SLOTS, TAB, T, BATCH>(set, q, n, r0), 0);
+            if (j == 0 && pl.full) out += counted(rs_filter<NW, SLOTS, TAB, T, BATCH, ENERGY>(set, q, n, r0, &en), 0);
             int dn, cre;
             if constexpr (T == 32) {
                 dn = (int)(short)(out & 0xffff);
@@ -750,6 +794,13 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
             mx = max(mx, c);
         }
         sync();
+    }
+    if constexpr (ENERGY) {
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            for (int o = 16; o > 0; o >>= 1) en.a[t] += __shfl_xor_sync(0xffffffffu, en.a[t], o);
+            if (lane == 0 && en.a[t]) atomicAdd(&A.rec[r0 + 1].energy[t], (unsigned long long)en.a[t]);
+        }
     }
     // ---- the block's totals
     mx = __reduce_max_sync(0xffffffffu, mx);

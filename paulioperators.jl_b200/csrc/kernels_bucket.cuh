@@ -58,6 +58,7 @@ struct BkRec {
     unsigned long long np;          // survivors of the early-merge pre-filter (when pref)
     unsigned long long created;     // sin branches appended (after the local filter)
     unsigned long long nval;        // adaptive sequences: values listed for the next threshold
+    unsigned long long energy[3];   // EnergyCorrection: <ket|.|ket> of what the block dropped (RsEnergy)
     int pref;                       // the rotation began with an early merge (CTA 0)
     int maxcnt;                     // largest output bucket
 };
@@ -92,6 +93,8 @@ struct BkArgs {
     const double *thr;
     double *vals;
     long long vals_cap;
+    int energy;                     // 1: EnergyCorrection, values scaled by escale (a power of two)
+    double escale;
 };
 
 // Bucket of a key: the low `bits` bits of the GF(2)-linear hash.

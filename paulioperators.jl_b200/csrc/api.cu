@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -177,7 +178,7 @@ struct pp_spv {
 // orders reuse between streams itself.  Memory it holds unused is bounded by POOL_KEEP
 // (checked whenever a handle frees a large part) and all returned when the last
 // handle is destroyed.
-static constexpr size_t POOL_KEEP = 4ull << 30;
+static constexpr size_t POOL_KEEP = 8ull << 30;
 struct DevPool {
     std::mutex mu;
     cudaMemPool_t pool = nullptr;
@@ -185,6 +186,8 @@ struct DevPool {
     std::vector<cudaStream_t> streams;     // idle streams of destroyed handles (at most MAX_STREAMS)
     bool setup[2] = {false, false};        // launch attributes and occupancies of each word count
     int occ[2][4] = {};
+    size_t room = 0;                       // the last answer of dev_room, and when it was given
+    std::chrono::steady_clock::time_point room_at;
     static constexpr size_t MAX_STREAMS = 16;
 };
 static DevPool &dev_pool(int dev) {
@@ -234,11 +237,25 @@ static void pool_trim(int dev, size_t keep) {
     cudaGetLastError();
 }
 
-// Free device memory, what the pool holds unused included.
-static bool dev_room(int dev, size_t *room) {
+// Free device memory, what the pool holds unused included.  cudaMemGetInfo takes 0.1 ms
+// and more, so an answer of the last quarter second stands in for requests of less than
+// an eighth of it.
+static bool dev_room(int dev, double want, size_t *room) {
+    DevPool &d = dev_pool(dev);
+    const auto now = std::chrono::steady_clock::now();
+    {
+        std::lock_guard<std::mutex> lk(d.mu);
+        if (d.room > 0 && 8.0 * want < (double)d.room && now - d.room_at < std::chrono::milliseconds(250)) {
+            *room = d.room;
+            return true;
+        }
+    }
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) { cudaGetLastError(); return false; }
     *room = freeb + pool_unused(dev);
+    std::lock_guard<std::mutex> lk(d.mu);
+    d.room = *room;
+    d.room_at = now;
     return true;
 }
 
@@ -411,7 +428,7 @@ static int grow_live(pp_spv *h, long long need, bool preserve = true, long long 
         // (no question where the pool holds enough: the growth takes no more of the device)
         size_t freeb = 0;
         const double per = 2.0 * (2 * h->NW * 8 + 8) + 12.0 + 4.0 * TAU_MAX * 2.0 / SEG;
-        if (1.25 * (double)newcap * per > (double)pool_unused(h->dev) && dev_room(h->dev, &freeb)) {
+        if (1.25 * (double)newcap * per > (double)pool_unused(h->dev) && dev_room(h->dev, (double)newcap * per, &freeb)) {
             const double room = (double)freeb - 4.0 * (1ull << 30);
             while ((double)newcap * per > room && newcap > need) newcap = std::max(need, newcap - newcap / 4);
             if ((double)newcap * per > room)
@@ -768,7 +785,7 @@ static bool ss_reserve(pp_spv *h, long long n) {
     const long long need = (long long)p.nbk * p.cap;
     if (need > h->ss_cap) {
         size_t freeb = 0;
-        if (dev_room(h->dev, &freeb) && (double)need * (16 * NW + 12) + 4.0 * (1ull << 30) > (double)freeb) return false;
+        if (dev_room(h->dev, (double)need * (16 * NW + 12), &freeb) && (double)need * (16 * NW + 12) + 4.0 * (1ull << 30) > (double)freeb) return false;
         h->ss_cap = 0;
         if (dalloc(h, &h->ss_z, need * NW) || dalloc(h, &h->ss_x, need * NW) || dalloc(h, &h->ss_c, need) ||
             dalloc(h, &h->ss_p, need))
@@ -1076,7 +1093,7 @@ static int expect_dev(pp_spv *h, const u64 *k, double *out);
 // and back costs about 0.2 ms up to 3e5 terms and 0.7 ms for 1.5e6, and saves 0.05 and 0.08
 // ms a rotation.  (With per-rotation times asked for, only long sequences: a block has no
 // separate rotate and merge times.)
-static int bk_min_rot(long long n, bool per_rot) { return per_rot ? 32 : n <= 300000 ? 6 : 12; }
+static int bk_min_rot(long long n, bool per_rot) { return per_rot ? 32 : n <= 300000 ? 6 : 8; }
 // Internal status (never returned by the C ABI): a bucket layout for the live set
 // would not fit in device memory; the sequence continues on the sorted-merge
 // kernels from the rotation the device cursor is at.
@@ -1242,14 +1259,16 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
     // split of headroom (2^(bits+1) buckets) when that fits, else 2^bits
     auto fits = [&](long long sl) {
         size_t freeb = 0;
-        if (dev_room(h->dev, &freeb)) {
-            const double B = 16.0 * NW + 8.0;
+        const double B = 16.0 * NW + 8.0;
+        if (dev_room(h->dev, 3.5 * (double)sl * B, &freeb)) {
             if (3.5 * (double)sl * B + 4.0 * (1ull << 30) > (double)freeb) return false;
         }
         const long long lim = g_bk_slot_limit.load();
         return !(lim > 0 && sl > lim);
     };
-    int nbits = std::min(BK_ROWS, std::max(bits + 1, h->bk_cap == cap ? h->bk_bits_cap : 0));
+    // (no headroom for layouts above 2^21 slots: a split there moves to new sets anyway)
+    int nbits = std::min(BK_ROWS, std::max(bits + (((long long)cap << bits) <= (1ll << 21) ? 1 : 0),
+                                           h->bk_cap == cap ? h->bk_bits_cap : 0));
     if (!fits((long long)cap << nbits)) nbits = bits;
     if (!fits((long long)cap << nbits)) return BK_NOFIT;
     const long long slots = (long long)cap << nbits;
@@ -1748,6 +1767,7 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
     bool use_bk = bk_enabled();
     long long ncur = small_cap<NW>() + 1;   // live terms at the chunk's start (read when small_ok)
     bool dense = false;                      // the last state read showed a dense live set
+    bool roomy = false;                      // the live sets have room for a merge's output slots
     if (small_ok || n_known >= 0) {
         if (n_known >= 0) {
             ncur = n_known;
@@ -1787,6 +1807,14 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
             done = st.rot;
             ncur = small_ok ? st.n : small_cap<NW>() + 1;
             continue;
+        }
+        if (!roomy) {
+            // output slots for the first merges (buckets and the small kernel need none)
+            DevState st;
+            TRY(read_state(h, &st));
+            if (3 * st.n + 2 * SEG > h->cap) table = false;
+            TRY(ensure_live(h, 3 * st.n + 2 * SEG));
+            roomy = true;
         }
         dense = false;                       // the merge kernels leave a segment table
         Bufs B = make_bufs(h);
@@ -2542,7 +2570,6 @@ static int evolve_impl(pp_spv *h, const void *gz, const void *gx, const double *
     RunProf prof;
     prof.on = O.profile != 0;
     if (O.window == 1 && all_struct && !A.on) {
-        TRY(ensure_live(h, 3 * st.n + 2 * SEG));
         const bool want_rec = ctr && ctr->nwin > 0;
         if (want_rec && L > h->rec_cap) {
             TRY(dalloc(h, &h->rec, 4 * L));
@@ -2864,7 +2891,6 @@ static int batch_impl(pp_spv *h, const void *gz, const void *gx, long long L, co
     st.b_tile_ctr = 0;
     st.g_tile_ctr = 0;
     TRY(write_state(h, &st));
-    TRY(ensure_live(h, 3 * st.n + 2 * SEG));
     // harvest points: the distinct instance ends, in order
     std::vector<long long> pts(ends);
     std::sort(pts.begin(), pts.end());

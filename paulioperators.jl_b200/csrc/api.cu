@@ -1224,6 +1224,10 @@ static BkArgs bk_args(pp_spv *h, int bits, BkRec *rec) {
     return A;
 }
 
+// Whether bucket sets of cap slots a bucket hold records (one buffer per set, x and c
+// pointing into the first record) or three arrays: k_bb_block's of one-word keys do.
+static bool bk_records(int nw, int cap) { return nw == 1 && cap == BB_CAP; }
+
 // Scatters (SZ, SX, SC) -- dense n terms, or the bucket set `from` of 2^sbits
 // buckets -- into bucket set `to` with 2^bits buckets.  Returns the largest
 // bucket count in *maxcnt, or -1 if a bucket overflowed.
@@ -1236,9 +1240,12 @@ static int bk_scatter(pp_spv *h, const u64 *SZ, const u64 *SX, const double *SC,
     CU(cudaMemsetAsync(h->bk_aux, 0, 2 * sizeof(int), s));
     const long long slots = from >= 0 ? ((long long)cap << sbits) : n;
     const int grid = (int)std::max(1ll, std::min((slots + 255) / 256, (long long)h->nsm * 16));
-    k_bk_scatter<NW><<<grid, 256, 0, s>>>(SZ, SX, SC, n, from >= 0 ? h->bkcnt[from] : nullptr, sbits, h->bkz[to],
-                                          h->bkx[to], h->bkc[to], h->bkcnt[to], bits, __builtin_ctz(cap), h->bk_rows,
-                                          h->bk_aux, h->bk_aux + 1);
+    const bool rec = bk_records(NW, cap);
+    const int dk = rec ? BK_REC : NW, dc = rec ? BK_REC : 1;
+    k_bk_scatter<NW><<<grid, 256, 0, s>>>(SZ, SX, SC, from >= 0 ? dk : NW, from >= 0 ? dc : 1, n,
+                                          from >= 0 ? h->bkcnt[from] : nullptr, sbits, h->bkz[to], h->bkx[to], h->bkc[to],
+                                          dk, dc, h->bkcnt[to], bits, __builtin_ctz(cap), h->bk_rows, h->bk_aux,
+                                          h->bk_aux + 1);
     int aux[2] = {0, 0};
     CU(cudaMemcpyAsync(aux, h->bk_aux, sizeof aux, cudaMemcpyDeviceToHost, s));
     TRY(sync_check(h));
@@ -1259,7 +1266,7 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
     // split of headroom (2^(bits+1) buckets) when that fits, else 2^bits
     auto fits = [&](long long sl) {
         size_t freeb = 0;
-        const double B = 16.0 * NW + 8.0;
+        const double B = bk_records(NW, cap) ? 8.0 * BK_REC : 16.0 * NW + 8.0;
         if (dev_room(h->dev, 3.5 * (double)sl * B, &freeb)) {
             if (3.5 * (double)sl * B + 4.0 * (1ull << 30) > (double)freeb) return false;
         }
@@ -1275,14 +1282,24 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
     u64 *nz[2] = {nullptr, nullptr}, *nx[2] = {nullptr, nullptr};
     double *nc[2] = {nullptr, nullptr};
     int *nn[2] = {nullptr, nullptr};
+    const bool rec = bk_records(NW, cap);
+    constexpr int W = BK_REC;
     auto drop = [&]() {
-        for (int q = 0; q < 2; ++q) { dfree(h, nz[q]); dfree(h, nx[q]); dfree(h, nc[q]); dfree(h, nn[q]); }
+        for (int q = 0; q < 2; ++q) {
+            dfree(h, nz[q]);
+            if (!rec) { dfree(h, nx[q]); dfree(h, nc[q]); }
+            dfree(h, nn[q]);
+        }
     };
     int r = 0;
     for (int q = 0; q < 2 && !r; ++q) {
-        r = dalloc(h, &nz[q], slots * NW);
-        if (!r) r = dalloc(h, &nx[q], slots * NW);
-        if (!r) r = dalloc(h, &nc[q], slots);
+        r = dalloc(h, &nz[q], slots * (rec ? W : NW));
+        if (rec) {
+            if (!r) { nx[q] = nz[q] + NW; nc[q] = reinterpret_cast<double *>(nz[q] + 2 * NW); }
+        } else {
+            if (!r) r = dalloc(h, &nx[q], slots * NW);
+            if (!r) r = dalloc(h, &nc[q], slots);
+        }
         if (!r) r = dalloc(h, &nn[q], 1ll << nbits);
     }
     if (r) { drop(); return r; }
@@ -1290,16 +1307,18 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
         // the live bucket set keeps its layout: copy it into new set 0
         const long long os = (long long)h->bk_cap << cur_bits;
         cudaStream_t s = h->stream;
-        cudaError_t e = cudaMemcpyAsync(nz[0], h->bkz[*cur], os * NW * 8, cudaMemcpyDeviceToDevice, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(nx[0], h->bkx[*cur], os * NW * 8, cudaMemcpyDeviceToDevice, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(nc[0], h->bkc[*cur], os * 8, cudaMemcpyDeviceToDevice, s);
+        cudaError_t e = cudaMemcpyAsync(nz[0], h->bkz[*cur], os * (rec ? W : NW) * 8, cudaMemcpyDeviceToDevice, s);
+        if (!rec && e == cudaSuccess) e = cudaMemcpyAsync(nx[0], h->bkx[*cur], os * NW * 8, cudaMemcpyDeviceToDevice, s);
+        if (!rec && e == cudaSuccess) e = cudaMemcpyAsync(nc[0], h->bkc[*cur], os * 8, cudaMemcpyDeviceToDevice, s);
         if (e == cudaSuccess) e = cudaMemcpyAsync(nn[0], h->bkcnt[*cur], sizeof(int) << cur_bits, cudaMemcpyDeviceToDevice, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) { drop(); return fail(PP_DEVICE_ERROR, cudaGetErrorString(e)); }
         *cur = 0;
     }
     for (int q = 0; q < 2; ++q) {
-        dfree(h, h->bkz[q]); dfree(h, h->bkx[q]); dfree(h, h->bkc[q]); dfree(h, h->bkcnt[q]);
+        dfree(h, h->bkz[q]);
+        if (!bk_records(h->NW, h->bk_cap)) { dfree(h, h->bkx[q]); dfree(h, h->bkc[q]); }
+        dfree(h, h->bkcnt[q]);
         h->bkz[q] = nz[q]; h->bkx[q] = nx[q]; h->bkc[q] = nc[q]; h->bkcnt[q] = nn[q];
     }
     h->bk_bits_cap = nbits;
@@ -1310,7 +1329,9 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
 // Frees the bucket sets (the live set is dense again).
 static void bk_release(pp_spv *h) {
     for (int q = 0; q < 2; ++q) {
-        dfree(h, h->bkz[q]); dfree(h, h->bkx[q]); dfree(h, h->bkc[q]); dfree(h, h->bkcnt[q]);
+        dfree(h, h->bkz[q]);
+        if (!bk_records(h->NW, h->bk_cap)) { dfree(h, h->bkx[q]); dfree(h, h->bkc[q]); }
+        dfree(h, h->bkcnt[q]);
         h->bkz[q] = h->bkx[q] = nullptr;
         h->bkc[q] = nullptr;
         h->bkcnt[q] = nullptr;
@@ -1352,7 +1373,8 @@ static int bk_to_dense(pp_spv *h, int cur, int bits, long long n) {
     TRY(ensure_live(h, n + 1, false));
     unsigned long long *total = reinterpret_cast<unsigned long long *>(h->bk_aux);
     CU(cudaMemsetAsync(total, 0, sizeof *total, s));
-    k_bk_pack<NW><<<(nb + 255) / 256, 256, 0, s>>>(h->bkz[cur], h->bkx[cur], h->bkc[cur], h->bkcnt[cur], nb,
+    const int w = bk_records(NW, h->bk_cap) ? BK_REC : 0;
+    k_bk_pack<NW><<<(nb + 255) / 256, 256, 0, s>>>(h->bkz[cur], h->bkx[cur], h->bkc[cur], w ? w : NW, w ? w : 1, h->bkcnt[cur], nb,
                                                   __builtin_ctz(h->bk_cap), total, h->z[0], h->x[0], h->c[0], h->cap, h->S);
     unsigned long long got = 0;
     CU(cudaMemcpyAsync(&got, total, sizeof got, cudaMemcpyDeviceToHost, s));

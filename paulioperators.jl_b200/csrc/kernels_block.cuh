@@ -17,7 +17,7 @@
 // channel (a block ends at a channel, which scales every survivor at its end).
 //
 // What bounds it: latency and instruction issue, and above a million terms the scattered
-// reads and writes of short bucket runs.  A warp issues one instruction every 11 cycles
+// reads and writes of short bucket runs (one sector a term).  A warp issues one instruction every 11 cycles
 // (fixed latencies, shared memory), and twelve warps are what the resident sets leave
 // room for.  Large sets: a warp per coset, no block barrier between rotations.  Small
 // sets (an SM has a few cosets at most): a CTA per coset, whose chain of a rotation is
@@ -25,10 +25,10 @@
 // takes more rotations per launch.  The index over all resident terms is built once per
 // block and pays from about three rotations on.
 // Measured (one B200, whole calls, one rotation per launch before): 8 x 8 lattice,
-// 3,520 rotations, up to 3.9e6 terms 154.9 -> 95 ms; 127-qubit graph, 6,504 rotations, up
+// 3,520 rotations, up to 3.9e6 terms 154.9 -> 86 ms; 127-qubit graph, 6,504 rotations, up
 // to 8e4 terms 43.4 -> 16.3 ms; 48 batched instances 60.1 -> 38 ms.  (A warp per coset
 // everywhere: 109, 19.6 and 42.6; a CTA everywhere: 111, 16.2 and 38.4 with cosets of 512
-// terms, 96, 18.9 and 38.4 with cosets of 900.)
+// terms, 96, 18.9 and 38.4 with cosets of 900; the lattice at 95 then.)
 #pragma once
 #include "kernels_bucket.cuh"
 
@@ -103,21 +103,34 @@ __device__ __forceinline__ void rs_gen(RsGen<NW> *o, const GenRec &g, int delta)
     if (lane == 0) o->np = __popc(on);
 }
 
-// load_key through L2 only: a bucket set is rewritten by every second launch, and a
-// dependent launch may start before its predecessor's predecessor has ended, so its
-// lines must not be served from an SM's L1.
+// The term in slot o of a bucket set (one-word keys: records at Z; two-word keys: three
+// arrays), through L2 only: a bucket set is rewritten by every second launch, and a
+// dependent launch may start before its predecessor's predecessor has ended, so its lines
+// must not be served from an SM's L1.
 template <int NW>
-__device__ __forceinline__ Key<NW> load_key_cg(const u64 *Z, const u64 *X, long long i) {
-    Key<NW> k;
+__device__ __forceinline__ void load_term(const u64 *Z, const u64 *X, const double *C, long long o, Key<NW> *k, double *c) {
     if constexpr (NW == 1) {
-        k.z[0] = __ldcg(Z + i);
-        k.x[0] = __ldcg(X + i);
+        const ulonglong2 *p = reinterpret_cast<const ulonglong2 *>(Z + o * BK_REC);
+        const ulonglong2 a = __ldcg(p), b = __ldcg(p + 1);
+        k->z[0] = a.x; k->x[0] = a.y;
+        *c = __longlong_as_double((long long)b.x);
     } else {
-        const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2 *>(Z) + i);
-        const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2 *>(X) + i);
-        k.z[0] = a.x; k.z[1] = a.y; k.x[0] = b.x; k.x[1] = b.y;
+        const ulonglong2 a = __ldcg(reinterpret_cast<const ulonglong2 *>(Z) + o);
+        const ulonglong2 b = __ldcg(reinterpret_cast<const ulonglong2 *>(X) + o);
+        k->z[0] = a.x; k->z[1] = a.y; k->x[0] = b.x; k->x[1] = b.y;
+        *c = __ldcg(C + o);
     }
-    return k;
+}
+template <int NW>
+__device__ __forceinline__ void store_term(u64 *Z, u64 *X, double *C, long long o, const Key<NW> &k, double c) {
+    if constexpr (NW == 1) {
+        ulonglong2 *p = reinterpret_cast<ulonglong2 *>(Z + o * BK_REC);
+        p[0] = make_ulonglong2(k.z[0], k.x[0]);
+        p[1] = make_ulonglong2((u64)__double_as_longlong(c), 0ull);      // the padding, too: a whole sector is written
+    } else {
+        store_key<NW>(Z, X, o, k);
+        C[o] = c;
+    }
 }
 
 // A key in 32-bit words: z low to high, then x.
@@ -696,8 +709,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                 if (i < total) {
                     lb[u] = set.tag[i];
                     const long long o = ((long long)(rep ^ (unsigned)s_x[lb[u]]) << BB_CAP_LOG) + (i - soff[lb[u]]);
-                    kk[u] = load_key_cg<NW>(Z, X, o);
-                    cc[u] = __ldcg(C + o);
+                    load_term<NW>(Z, X, C, o, &kk[u], &cc[u]);
                 }
             }
 #pragma unroll
@@ -780,8 +792,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
                     if constexpr (BATCH) ch = ch && rs_instance<NW>(set.key(i), q, r0 + K - 1) >= 0;
                     if (ch) v = __dmul_rn(v, channel_factor<NW>(P, kw));
                     const long long o = ((long long)(rep ^ (unsigned)s_x[lb]) << BB_CAP_LOG) + po;
-                    store_key<NW>(OZ, OX, o, kw);
-                    OC[o] = v;
+                    store_term<NW>(OZ, OX, OC, o, kw, v);
                 }
             }
         }

@@ -860,14 +860,19 @@ __global__ void __launch_bounds__(256) k_sel64_pick(Select64 *sel, int shift) {
 // AdaptiveTruncation's threshold (spv_evolve.jl:103-114) in one launch, for the n <=
 // AS_MAX terms of the live set: with n > max_terms the (max_terms + 1)-th largest |c|,
 // else min_thresh, written to *thresh.  One CTA: the two leading digits of 11 bits by
-// histograms over all n values, the values that share them (usually a few) to shared
-// memory, and the rest of the digits over those.  Exact: the threshold is one of the
-// values.  Bound by the latency of its two or three passes over n values; 16 launches
-// of a histogram and a pick per 8-bit digit, this replaced, took 100 us at 2e4 terms.
+// histograms over all n values, the values that share them to shared memory, and there
+// each of up to AS_COUNT values counts the ones above it, or the rest of the digits are
+// walked.  Exact: the threshold is one of the values.  Bound by the latency of its two or
+// three passes over n values; 16 launches of a histogram and a pick per 8-bit digit, this
+// replaced, took 100 us at 2e4 terms.
 constexpr int AS_THREADS = 1024;
 constexpr long long AS_MAX = 1 << 18;
 constexpr int AS_BINS = 2048;
 constexpr int AS_KEEP = 3072;
+// Candidates at most that are ranked by counting: that is one pass of m shared loads per
+// thread, about 1 us, where the digits left cost three or four histograms with their scans
+// (351 rotations under a budget of 2e4 terms: 5.61 ms, by counting 5.12).
+constexpr unsigned AS_COUNT = 384;
 
 // With nval, the values are C0[0, *nval) instead of the live set's.
 __global__ void __launch_bounds__(AS_THREADS) k_abs_select(const double *C0, const double *C1, const DevState *S,
@@ -938,6 +943,22 @@ __global__ void __launch_bounds__(AS_THREADS) k_abs_select(const double *C0, con
             __syncthreads();
             m = min(s_n, (unsigned)AS_KEEP);
             listed = true;
+            if (m <= AS_COUNT) {
+                // few candidates: each thread counts the ones above and at its own
+                const long long rem2 = s_rem;
+                __syncthreads();
+                if (tid < (int)m) {
+                    const unsigned long long k = keep[tid];
+                    int above = 0, same = 0;
+                    for (unsigned j = 0; j < m; ++j) {
+                        above += keep[j] > k;
+                        same += keep[j] == k;
+                    }
+                    if (above < rem2 && rem2 <= above + same) s_pre = k;     // (ties write the same)
+                }
+                __syncthreads();
+                break;
+            }
         }
     }
     if (tid == 0) *thresh = __longlong_as_double((long long)s_pre);

@@ -38,6 +38,27 @@ def test_adaptive_threshold(n, values, keep):
     assert np.array_equal(got.view(np.uint64), c[on].view(np.uint64))
 
 
+@pytest.mark.parametrize("cand", [1, 2, 383, 384, 385, 3000])
+@pytest.mark.parametrize("tied", [False, True])
+@pytest.mark.parametrize("at", [0.0, 0.5, 1.0])
+def test_adaptive_threshold_few_candidates(cand, tied, at):
+    # the values in [1, 2) share the leading digit, the others are far away on both
+    # sides: at most 384 candidates are ranked by counting, more by their digits
+    n = 4000
+    rng = np.random.default_rng([cand, int(tied), int(10 * at)])
+    pool = 1.0 + rng.integers(0, 3, cand) / 4 if tied else 1.0 + (rng.permutation(cand) + 0.5) / cand
+    c = np.concatenate([pool, np.full(400, 100.0), np.full(n - 400 - cand, 1e-5)]) * rng.choice([-1.0, 1.0], n)
+    c = c[rng.permutation(n)]
+    m = 400 + int(at * (cand - 1))            # the threshold is one of the candidates
+    v = _vector(40, n, c)
+    pp.truncate_(v, pp.AdaptiveTruncation(m, 1e-3))
+    a = np.abs(c)
+    on = a > np.sort(a)[n - 1 - m]
+    z, _, got = v.to_arrays()
+    assert np.array_equal(z[:, 0], np.flatnonzero(on).astype(np.uint64))
+    assert np.array_equal(got.view(np.uint64), c[on].view(np.uint64))
+
+
 @pytest.mark.parametrize("group", [1, 64, 65, 66, 127, 1000, 40001])
 def test_variance_of_long_entries(group):
     """Var = sum over x of |sigma_x|^2 - sigma_psi^2, `group` terms in each of three

@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(G_THREADS) k_rotate_general(Bufs B, GenRec g) 
         }
         __syncthreads();
         if (warp == 0) {
-            constexpr int NE = G_ITEMS * (G_THREADS / 32);  // 64 entries, 2 per lane
+            constexpr int NE = G_ITEMS * (G_THREADS / 32);  // 32 entries, one per lane
             int v[NE / 32];
             int s = 0;
 #pragma unroll

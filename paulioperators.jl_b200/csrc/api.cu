@@ -1519,6 +1519,11 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
     // 2-norm of the entering set, which no rotation, filter or channel enlarges
     double escale = 0.0;
     if (h->Ph->corr_kind == 1) {
+        // (cos and sin are the caller's: a pair that is no rotation could enlarge the set)
+        for (long long r = start; r < L; ++r) {
+            const GenRec &g = h->gens_h[r];
+            if (!(g.cosv * g.cosv + g.sinv * g.sinv <= 1.0 + 1e-12)) return BK_NOFIT;
+        }
         double nrm = 0.0;
         TRY(norm2_dev(h, st.cur, n0, &nrm));
         if (!std::isfinite(nrm) || nrm > 0x1p900) return BK_NOFIT;         // (the sorted-merge kernels add doubles)
@@ -1602,11 +1607,11 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
             prof->bk_bytes += (double)(16 * NW + 8) * ((double)rec[(size_t)(b.r0 - start)].n_out +
                                                        (double)rec[(size_t)(b.r0 + b.K - start)].n_out);
         if (escale != 0.0) {
-            __int128 e[3] = {0, 0, 0};
+            __int128 e[4] = {0, 0, 0, 0};
             for (const Block &b : blocks)
-                for (int t = 0; t < 3; ++t) e[t] += (long long)rec[(size_t)(b.r0 + 1 - start)].energy[t];
+                for (int t = 0; t < 4; ++t) e[t] += (long long)rec[(size_t)(b.r0 + 1 - start)].energy[t];
             // smallest unit first: one rounding each
-            const double sum = (double)e[2] * 0x1p-110 + (double)e[1] * 0x1p-70 + (double)e[0] * 0x1p-30;
+            const double sum = (double)e[3] * 0x1p-126 + (double)e[2] * 0x1p-94 + (double)e[1] * 0x1p-62 + (double)e[0] * 0x1p-30;
             st.corr_energy -= sum / escale;
         }
         if (h->rec_on && upto > start)

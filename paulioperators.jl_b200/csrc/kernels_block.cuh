@@ -274,11 +274,12 @@ __device__ __forceinline__ bool rs_drop(const RsParams &q, const Key32<NW> &k, d
 }
 
 // <ket|.|ket> of dropped terms (EnergyCorrection), added up exactly: a value, scaled to
-// at most 1 in magnitude, is cut into whole multiples of 2^-30, 2^-70 and 2^-110, whose
-// sums do not depend on the order.
+// at most 1 in magnitude, is cut into whole multiples of 2^-30, 2^-62, 2^-94 and 2^-126,
+// whose sums do not depend on the order.  A multiple is at most 2^31: the sums of all the
+// terms that a set may hold (2^31) stay within 64 bits.
 template <int NW>
 struct RsEnergy {
-    long long a[3];
+    long long a[4];
     unsigned ket[2 * NW];
     double scale;
     __device__ __forceinline__ void add(const Key32<NW> &k, double v) {
@@ -291,9 +292,9 @@ struct RsEnergy {
         if (x) return;
         double r = v * scale;
         if (__popc(s) & 1) r = -r;
-        const double g[3] = {0x1p30, 0x1p70, 0x1p110}, u[3] = {0x1p-30, 0x1p-70, 0x1p-110};
+        const double g[4] = {0x1p30, 0x1p62, 0x1p94, 0x1p126}, u[4] = {0x1p-30, 0x1p-62, 0x1p-94, 0x1p-126};
 #pragma unroll
-        for (int t = 0; t < 3; ++t) {
+        for (int t = 0; t < 4; ++t) {
             const long long q = __double2ll_rn(r * g[t]);
             a[t] += q;
             r = __dsub_rn(r, (double)q * u[t]);            // exact: |q| < 2^53
@@ -808,7 +809,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     }
     if constexpr (ENERGY) {
 #pragma unroll
-        for (int t = 0; t < 3; ++t) {
+        for (int t = 0; t < 4; ++t) {
             for (int o = 16; o > 0; o >>= 1) en.a[t] += __shfl_xor_sync(0xffffffffu, en.a[t], o);
             if (lane == 0 && en.a[t]) atomicAdd(&A.rec[r0 + 1].energy[t], (unsigned long long)en.a[t]);
         }

@@ -64,7 +64,7 @@ struct BkRec {
     unsigned long long np;          // survivors of the early-merge pre-filter (when pref)
     unsigned long long created;     // sin branches appended (after the local filter)
     unsigned long long nval;        // adaptive sequences: values listed for the next threshold
-    unsigned long long energy[3];   // EnergyCorrection: <ket|.|ket> of what the block dropped (RsEnergy)
+    unsigned long long energy[4];   // EnergyCorrection: <ket|.|ket> of what the block dropped (RsEnergy)
     int pref;                       // the rotation began with an early merge (CTA 0)
     int maxcnt;                     // largest output bucket
 };

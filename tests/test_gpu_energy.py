@@ -54,3 +54,21 @@ def test_energy_on_buckets(N, n, L, early, scale, local):
     # the oracle takes differences of <ket|O|ket>, each rounded to the size of the set's diagonal
     tol = 4 * L * np.finfo(float).eps * float(np.abs(c[np.all(x == 0, axis=1)]).sum())
     assert abs(corr.accumulated_energy - e) <= tol
+
+
+def test_energy_of_many_equal_terms():
+    # 2^25 equal diagonal terms, all dropped by one rotation: the parts of the exact sum
+    # grow with the number of terms; their rest below the first unit is nearly half of it
+    n, N = 1 << 25, 30
+    c = (87654 + 0.4999) * 2.0 ** -30
+    z = np.arange(n, dtype=np.uint64).reshape(-1, 1)
+    g = pp.SparsePauliVector(N, n, 16)
+    g.upload(z, np.zeros_like(z), np.full(n, c), sorted=True)
+    # <ket|Z-string|ket> = (-1)^popcount(z & ket): with ket 0 every term counts as +c
+    corr = pp.EnergyCorrection(0)
+    pp.evolve_(g, [pp.PauliBasis(N, 1 << i, 0) for i in range(8)], [0.3] * 8, truncation=pp.CoeffTruncation(1.0),
+               correction=corr)
+    assert len(g) == 0
+    assert abs(abs(corr.accumulated_energy) - n * c) <= 4 * np.finfo(float).eps * n * c
+    g.close()
+

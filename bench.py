@@ -60,11 +60,12 @@ BYTES_PER_TERM = {1: 24, 2: 40}     # B = 2*(W/8) + 8
 # dram__bytes_write.sum = 115.1 MB per launch against B(n + a + m) = 150.9 MB:
 # the gathered sin branches re-read live terms that are still in L2)
 MERGE_TRAFFIC_PER_ALG_BYTE = 115.09 / 150.88
-# DRAM traffic of k_bk_rotate<1,512,4> per algorithmic byte, from one ncu capture of
-# three launches of this workload at n = 1.90e6 live terms: (dram__bytes_read.sum +
-# dram__bytes_write.sum) = 60.6 MB per launch against B(n_in + n_out) = 91.0 MB (part
-# of a launch's writes is still in L2 when it ends and is written back later)
-BUCKET_TRAFFIC_PER_ALG_BYTE = 60.58 / 91.02
+# DRAM traffic of k_bb_block<1> per algorithmic byte, from one ncu capture of
+# the four launches of 24 rotations of this circuit at n = 2.06e6 live terms:
+# (dram__bytes_read.sum + dram__bytes_write.sum) = 170.1 MB per launch of six rotations
+# against B(n_in + n_out) = 99.1 MB (a term is a 32-byte record, short bucket runs share
+# their DRAM bursts with empty slots; part of the writes is still in L2 at the end)
+BUCKET_TRAFFIC_PER_ALG_BYTE = 680.26 / 396.58
 
 
 def parse():
@@ -413,12 +414,11 @@ def run_ours_batch(args):
     sp = rp.stats
     B = BYTES_PER_TERM[2]
     if sp["bucket_rot"] > 0:
-        # rotations on buckets: B*(n_in + n_out) per k_bk_rotate launch over the timed
-        # graph replays (t_merge also holds any span that ran on the sorted-merge kernels)
+        # blocks of rotations on buckets: B*(n_in + n_out) per k_bb_block launch over the
+        # timed chunks (t_merge also holds any span that ran on the sorted-merge kernels)
         dom_bytes = sp["bucket_bytes"]
-        tune = pp.tune.get_tuning(v)
-        dom_kernel = (f"k_bk_rotate<2,{tune[0]},{tune[1]},batched> (rotation + partner merge + filter over "
-                      f"bucket pairs, 40-byte instance-tagged terms)")
+        dom_kernel = ("k_bb_block<2,batched> (up to 8 rotations + partner merge + filter per launch, cosets of "
+                      "buckets in shared memory, 40-byte instance-tagged terms)")
     else:
         dom_bytes = B * (sp["merge_in"] + sp["merge_out"])
         dom_kernel = "k_merge<2,0> (merge + reduce-by-key + filter, 40-byte batched terms)"
@@ -738,12 +738,13 @@ def _measure(args, wname, ws, rank, local, dev, orc):
     pipe_bytes = B * (sp["terms_in"] + sp["merge_out"])          # B*(n + m) per rotation, summed
     tuning = pp.tune.get_tuning(g)
     if sp["bucket_rot"] > 0:
-        # bucketed rotations: one k_bk_rotate launch per rotation reads its n live
-        # terms and writes its m survivors, B*(n + m) per launch
-        dom_bytes, dom_launches = sp["bucket_bytes"], sp["bucket_rot"]
-        dom_kernel = (f"k_bk_rotate<{nw},{tuning[0]},{tuning[1]}> (rotation + partner merge + filter + "
-                      f"channel over bucket pairs)")
-        traffic_ratio = BUCKET_TRAFFIC_PER_ALG_BYTE
+        # rotations on buckets: a k_bb_block launch reads the n live terms of its first
+        # rotation and writes the m survivors of its last, B*(n + m) per launch of up to
+        # eight rotations (launches: all of the step's, the blocks but for a few dozen)
+        dom_bytes, dom_launches = sp["bucket_bytes"], sp["launches"]
+        dom_kernel = (f"k_bb_block<{nw}> (up to 8 rotations + partner merge + filter + channel per launch, "
+                      f"cosets of buckets in shared memory)")
+        traffic_ratio = BUCKET_TRAFFIC_PER_ALG_BYTE if nw == 1 else None
     elif sp["t_merge"] > 0:
         dom_bytes, dom_launches = B * (sp["merge_in"] + sp["merge_out"]), len(gens)   # B*(n + a + m)
         dom_kernel = "k_merge<1,0> (merge + reduce-by-key + filter + channel + compaction)"

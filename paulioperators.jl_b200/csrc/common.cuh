@@ -113,8 +113,8 @@ constexpr int B_CAP = B_THREADS * B_IPTMAX;   // 2560: a tile plus an equal-key 
 constexpr int SEG = B_CAP;                    // slot of one window-1 merge tile's output; dense segment size
 static_assert(A_TILE >= SEG, "a classify tile holds one live segment");
 constexpr int G_THREADS = 256;
-// Four terms a thread: a window's pending set is 1e4 to 1e5 terms, where tiles of 2,048
-// left most SMs without one (a window-8 sequence of 351 rotations, up to 1.6e4 live terms:
+// Four terms a thread: a window's live and pending terms are 1e4 to 1e5, where tiles of 2,048
+// left most SMs without one (a window-8 sequence of 372 rotations, up to 6.9e3 live terms:
 // 7.76 ms with eight, 7.31 with four).
 constexpr int G_ITEMS = 4;
 constexpr int G_TILE = G_THREADS * G_ITEMS;   // general rotate tile

@@ -1,9 +1,11 @@
 """Autotuner of the bucketed window-1 rotations (no counterpart in the reference).
 
-The launch configuration of k_bk_rotate -- bucket capacity (the CTA's tile of
-terms), items per thread, the bucketing load divisor and the rotations launched
-between host checks -- changes how fast a sequence runs, never what it computes
-(every variant is checked bit for bit against the oracle in the GPU tests).
+The bucketing load divisor and the rotations launched between host checks change
+how fast a sequence runs, never what it computes.  Bucket capacity (the CTA's tile
+of terms) and items per thread choose the variant of k_bk_rotate, which only
+key-sharded runs launch (every variant is checked bit for bit against the oracle
+in the GPU tests); k_bb_block, which runs an unsharded vector's rotations, has a
+fixed capacity.
 `tune()` times each candidate on the device (CUDA events on the vector's
 stream) on a representative sequence per word count and writes the fastest to a JSON cache keyed by the device's SM count
 and compute capability; `apply_cached(v)` gives a new vector the cached setting.

@@ -1262,13 +1262,15 @@ static int bk_reserve(pp_spv *h, int bits, int *cur, int cur_bits, int cap) {
     if (cur_bits >= 0 && h->bk_cap != cap)
         return fail(PP_ERROR_EXCEPTION, "internal error: bucket capacity changed inside a call");
     // the two bucket sets, and room to convert a full layout (at most slots / 2
-    // terms before the next split) back to a dense sorted set, plus 4 GiB; one
-    // split of headroom (2^(bits+1) buckets) when that fits, else 2^bits
+    // terms before the next split; of k_bb_block's small buckets slots / 3, more do
+    // not go in) back to a dense sorted set, plus 4 GiB; one split of headroom
+    // (2^(bits+1) buckets) when that fits, else 2^bits
+    const double room = cap == BB_CAP ? 3.0 : 3.5;
     auto fits = [&](long long sl) {
         size_t freeb = 0;
         const double B = bk_records(NW, cap) ? 8.0 * BK_REC : 16.0 * NW + 8.0;
-        if (dev_room(h->dev, 3.5 * (double)sl * B, &freeb)) {
-            if (3.5 * (double)sl * B + 4.0 * (1ull << 30) > (double)freeb) return false;
+        if (dev_room(h->dev, room * (double)sl * B, &freeb)) {
+            if (room * (double)sl * B + 4.0 * (1ull << 30) > (double)freeb) return false;
         }
         const long long lim = g_bk_slot_limit.load();
         return !(lim > 0 && sl > lim);
@@ -1345,16 +1347,26 @@ static void bk_release(pp_spv *h) {
 // Moves the live bucket set *cur (2^*bits buckets) to a layout with more
 // buckets, doubling until the largest bucket holds at most half its capacity
 // (then no bucket of the next rotation's output can overflow).
+// For k_bb_block's buckets half full is what a new layout aims at, not what it needs: an
+// overflow is detected and its block runs again.  With 2^24 buckets and more the fullest
+// is beyond half at a mean of 5; where the next layout does not fit in memory, this one is
+// kept until a bucket overflows.  (256 instances of the 8 x 8 lattice, 3e8 terms at the
+// peak: 176 rotations of 2.4e8 terms 1.2 s in 2^25 buckets, 4.3 s on the sorted merges.)
+static constexpr int BB_FULL = 7 * BB_CAP / 8;
 template <int NW>
 static int bk_regrid(pp_spv *h, int *cur, int *bits) {
     int nbits = *bits;
+    bool held = false;
     for (;;) {
         if (nbits + 1 > BK_ROWS) return fail(PP_OUT_OF_MEMORY, "bucketed live set exceeds 2^26 buckets");
         ++nbits;
-        TRY(bk_reserve<NW>(h, nbits, cur, *bits, h->bk_cap));
+        const int rr = bk_reserve<NW>(h, nbits, cur, *bits, h->bk_cap);
+        if (rr == BK_NOFIT && held) { --nbits; break; }    // the last layout holds the set, fuller than wanted
+        TRY(rr);
         int mx = 0;
         TRY(bk_scatter<NW>(h, h->bkz[*cur], h->bkx[*cur], h->bkc[*cur], 0, *cur, *bits, *cur ^ 1, nbits, &mx));
         if (mx >= 0 && mx <= h->bk_cap / 2) break;
+        held = h->bk_cap == BB_CAP && mx >= 0;
     }
     *cur ^= 1;
     *bits = nbits;
@@ -1547,7 +1559,7 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
     int bits = bk_bits_for(n0, BB_CAP, h->tune.load_div), cur = 0;
     PP_TRACE("buckets: rotations [%lld, %lld), %lld live terms, 2^%d buckets of %d", start, L, n0, bits, BB_CAP);
     // (when that layout does not fit, fewer and fuller buckets down to a mean load
-    // of cap / 3, as long as no bucket is more than half full)
+    // of cap / 3, as long as they hold the set)
     const int bmin = bk_bits_for(n0, BB_CAP, 3);
     bool lowered = false;
     for (;;) {
@@ -1560,8 +1572,8 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         if (rr) return rr;                  // BK_NOFIT: nothing changed, the dense set is the input
         int mx = 0;
         TRY(bk_scatter<NW>(h, h->z[st.cur], h->x[st.cur], h->c[st.cur], n0, -1, 0, 0, bits, &mx));
-        if (mx >= 0 && mx <= BB_CAP / 2) break;
-        if (lowered) return BK_NOFIT;       // the fuller layout fails the half-full rule, a larger one does not fit
+        if (mx >= 0 && (lowered || mx <= BB_CAP / 2)) break;
+        if (lowered) return BK_NOFIT;       // the fuller layout does not hold the set, a larger one does not fit
         if (++bits > BK_ROWS) return fail(PP_OUT_OF_MEMORY, "bucketed live set exceeds 2^26 buckets");
     }
     // a rotation whose input values may not have passed the strict filter starts a block
@@ -1701,6 +1713,7 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         return PP_OK;
     };
     int split = 0;                         // the layout is to be split before the next launch
+    bool tight = false;                    // a larger layout does not fit: this one is used until a bucket overflows
     while (done < L) {
         // a second chunk goes out before the first is looked at, unless the set grows so fast
         // that it would outgrow the layout by then
@@ -1748,13 +1761,18 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         }
         growth = std::max(1.0, (double)last.n_out / std::max(1.0, (double)c.n));
         n = (long long)last.n_out;
-        if (done < L && ((over & 1) || last.maxcnt > 7 * BB_CAP / 8 || n > ((long long)(BB_CAP / 4) << bits)))
+        if (done < L && ((over & 1) || (tight ? n > ((long long)BB_CAP << bits) / 3
+                                           : last.maxcnt > BB_FULL || n > ((long long)(BB_CAP / 4) << bits))))
             split = 1;
         if (done == L || !split || !inflight.empty()) continue;
         split = 0;
         const int rr = bk_regrid<NW>(h, &cur, &bits);
         PP_TRACE("buckets: split at rotation %lld (%lld terms, largest bucket %d) -> 2^%d buckets%s", done, n, last.maxcnt,
-                 bits, rr == BK_NOFIT ? ": does not fit, hand-over to the sorted-merge kernels" : "");
+                 bits, rr == BK_NOFIT ? ": does not fit" : "");
+        if (rr == BK_NOFIT && !tight && !(over & 1)) {
+            tight = true;                  // (nothing has overflowed yet)
+            continue;
+        }
         if (rr == BK_NOFIT) {
             // no room for a larger layout: the rotations so far go back to the
             // dense sorted set, the bucket sets are freed, and the sorted-merge

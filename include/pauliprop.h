@@ -358,10 +358,13 @@ int pp_shard_end(pp_spv *h, double *expect_partial, double *stats_out);
  * pp_debug_bucket_limit: bucket layouts of more than `slots` term slots count as
  * not fitting in device memory (slots <= 0: only the real free memory limits
  * them); a sequence whose live set outgrows the layout that fits continues on the
- * sorted-merge kernels with the same result. */
+ * sorted-merge kernels with the same result.
+ * pp_debug_sort_overflow: while on, every sort by samples of more than one bucket finds
+ * a bucket beyond its slots and sorts by digits, with the same result. */
 int pp_debug_fail_alloc(int64_t after);
 int pp_debug_lookback_timeout(int64_t limit);
 int pp_debug_bucket_limit(int64_t slots);
+int pp_debug_sort_overflow(int32_t on);
 
 #ifdef __cplusplus
 }

@@ -303,6 +303,9 @@ static std::atomic<long long> g_fail_alloc_after{0};
 // Test hook (pp_debug_bucket_limit): bucket layouts above this many term slots
 // count as not fitting in device memory (0: no limit).
 static std::atomic<long long> g_bk_slot_limit{0};
+// Test hook (pp_debug_sort_overflow): every sample sort of several buckets finds one of
+// them beyond its slots.
+static std::atomic<int> g_ss_overflow{0};
 
 template <typename T>
 static int dalloc(pp_spv *h, T **p, long long count) {
@@ -819,6 +822,7 @@ static int ss_sort(pp_spv *h, u64 *z, u64 *x, double *c, long long n, bool *ok) 
     const int rb = (p.S + SSR - 1) / SSR;
     k_ss_rank<NW><<<dim3(rb, rb), SSR, 0, s>>>(key, pos, p.S, rank);
     k_ss_split<NW><<<rb, SSR, 0, s>>>(key, pos, rank, p.S, p.os, p.nbk, skey, spos);
+    if (g_ss_overflow.load()) CU(cudaMemsetAsync(over, 1, sizeof *over, s));
     const long long per = SS_THREADS * SS_ITEMS;
     k_ss_scatter<NW><<<(int)((n + per - 1) / per), SS_THREADS, ss_scatter_smem<NW>(p.nbk), s>>>(
         z, x, c, n, skey, spos, p.nbk, cnt, h->ss_z, h->ss_x, h->ss_c, h->ss_p, p.cap, over);
@@ -1374,14 +1378,15 @@ static int bk_regrid(pp_spv *h, int *cur, int *bits) {
 }
 
 // Packs the n terms of the bucket set `cur` (2^bits buckets) into live set 0 and sorts
-// it: the live set is dense and sorted again.  Every allocation the packing needs
-// comes first, so a failure leaves the dense live set as it was.
+// it: the live set is dense and sorted again.  Every allocation of the packing and of
+// either sort comes first, so a failure leaves the dense live set as it was.
 template <int NW>
 static int bk_to_dense(pp_spv *h, int cur, int bits, long long n) {
     const int nb = 1 << bits;
     cudaStream_t s = h->stream;
     PP_TRACE("buckets -> dense: %lld terms (2^%d buckets)", n, bits);
-    if (!ss_reserve<NW>(h, n)) TRY(radix_reserve(h, n));
+    ss_reserve<NW>(h, n);
+    TRY(radix_reserve(h, n));               // (a bucket of the sample sort may overflow)
     TRY(ensure_live(h, n + 1, false));
     unsigned long long *total = reinterpret_cast<unsigned long long *>(h->bk_aux);
     CU(cudaMemsetAsync(total, 0, sizeof *total, s));
@@ -2795,6 +2800,11 @@ extern "C" int pp_device_info(pp_spv *h, int32_t *sm_count, int32_t *cc_major, i
 // ------------------------------------------------------------------ test hooks
 extern "C" int pp_debug_fail_alloc(int64_t after) {
     g_fail_alloc_after.store(after > 0 ? after : 0);
+    return PP_OK;
+}
+
+extern "C" int pp_debug_sort_overflow(int32_t on) {
+    g_ss_overflow = on ? 1 : 0;
     return PP_OK;
 }
 

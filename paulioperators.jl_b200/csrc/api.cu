@@ -171,17 +171,30 @@ struct pp_spv {
 };
 
 // ------------------------------------------------------------------ device memory
-// Device memory comes from a stream-ordered pool per device (cudaMallocFromPoolAsync),
-// shared by every handle of the process: an evolve of a copy, or a product into a new
+// Shared by every handle of a device: an evolve of a copy, or a product into a new
 // vector, allocates and frees some fifty buffers, and cudaMalloc / cudaFree cost more
-// than the kernels between them (1.5e6 terms, nine rotations: 12 of 14 ms).  The pool
-// orders reuse between streams itself.  Memory it holds unused is bounded by POOL_KEEP
-// (checked whenever a handle frees a large part) and all returned when the last
-// handle is destroyed.
-static constexpr size_t POOL_KEEP = 8ull << 30;
+// than the kernels between them (1.5e6 terms, nine rotations: 12 of 14 ms).  Blocks below
+// MEM_BIG come from a stream-ordered pool (cudaMallocFromPoolAsync), which orders reuse
+// between streams itself; larger ones from cudaMalloc, and a freed one is listed, once its
+// stream has ended, for the next request that it fits with at most a fifth to spare.
+// The pool takes and returns memory in pieces of 32 MiB, 0.2 ms each: a block of 1 GiB
+// that it does not hold costs 6.5 ms, and as much when it is trimmed away, where cudaMalloc
+// and cudaFree take 0.66 and 0.93 (64 MiB: 0.41 and 0.39, 0.35 and 0.30).  Where a call's
+// buffers are beyond what is kept that is what it costs: an evolve of a copy of 6.9e6 terms
+// by 32 rotations took 321 ms with one pool for all sizes, 79 so, 49 in kernels; one of
+// 2.2e6 terms 148 and 34.
+// What is held unused is bounded by MEM_KEEP (checked when a handle frees a large block or
+// is destroyed; the longest unused blocks go first; 3 GiB instead of 8: an evolve of a copy
+// of 2.2e6 terms by eight rotations 6.0 ms instead of 3.3) and all returned when the last
+// handle is destroyed, or when an allocation fails.
+static constexpr size_t MEM_BIG = 64ull << 20;
+static constexpr size_t MEM_KEEP = 8ull << 30;
 struct DevPool {
     std::mutex mu;
     cudaMemPool_t pool = nullptr;
+    std::unordered_map<void *, size_t> big;            // blocks of cudaMalloc in use
+    std::vector<std::pair<void *, size_t>> idle;       // and freed ones, the longest unused first
+    size_t idle_bytes = 0;
     long long handles = 0;                 // handles alive on the device
     std::vector<cudaStream_t> streams;     // idle streams of destroyed handles (at most MAX_STREAMS)
     bool setup[2] = {false, false};        // launch attributes and occupancies of each word count
@@ -206,7 +219,7 @@ static int pool_get(int dev, cudaMemPool_t *out) {
         pr.location.type = cudaMemLocationTypeDevice;
         pr.location.id = dev;
         CU(cudaMemPoolCreate(&d.pool, &pr));
-        unsigned long long keep = ~0ull;   // trimmed by pool_trim, not at every synchronisation
+        unsigned long long keep = ~0ull;   // trimmed by mem_trim, not at every synchronisation
         CU(cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep));
     }
     *out = d.pool;
@@ -225,19 +238,38 @@ static size_t pool_unused(int dev) {
     return res > used ? (size_t)(res - used) : 0;
 }
 
-// Returns what the pool holds unused above keep bytes.
-static void pool_trim(int dev, size_t keep) {
-    cudaMemPool_t pool = dev_pool(dev).pool;
-    if (!pool) return;
-    const size_t un = pool_unused(dev);
-    if (un <= keep) return;
-    unsigned long long used = 0;
-    if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
-        cudaMemPoolTrimTo(pool, (size_t)used + keep);
+// Bytes held and not in use: the pool's and the listed blocks'.
+static size_t mem_unused(int dev) {
+    DevPool &d = dev_pool(dev);
+    const size_t pu = pool_unused(dev);
+    std::lock_guard<std::mutex> lk(d.mu);
+    return pu + d.idle_bytes;
+}
+
+// Returns what is held unused above keep bytes.
+static void mem_trim(int dev, size_t keep) {
+    DevPool &d = dev_pool(dev);
+    const size_t pu = pool_unused(dev);
+    std::vector<void *> out;
+    {
+        std::lock_guard<std::mutex> lk(d.mu);
+        size_t k = 0;
+        for (; k < d.idle.size() && pu + d.idle_bytes > keep; ++k) {
+            out.push_back(d.idle[k].first);
+            d.idle_bytes -= d.idle[k].second;
+        }
+        d.idle.erase(d.idle.begin(), d.idle.begin() + (long)k);
+    }
+    for (void *p : out) cudaFree(p);
+    if (pu > keep) {
+        unsigned long long used = 0;
+        if (cudaMemPoolGetAttribute(d.pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+            cudaMemPoolTrimTo(d.pool, (size_t)used + keep);
+    }
     cudaGetLastError();
 }
 
-// Free device memory, what the pool holds unused included.  cudaMemGetInfo takes 0.1 ms
+// Free device memory, what is held unused included.  cudaMemGetInfo takes 0.1 ms
 // and more, so an answer of the last quarter second stands in for requests of less than
 // an eighth of it.
 static bool dev_room(int dev, double want, size_t *room) {
@@ -252,7 +284,7 @@ static bool dev_room(int dev, double want, size_t *room) {
     }
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) { cudaGetLastError(); return false; }
-    *room = freeb + pool_unused(dev);
+    *room = freeb + mem_unused(dev);
     std::lock_guard<std::mutex> lk(d.mu);
     d.room = *room;
     d.room_at = now;
@@ -260,38 +292,78 @@ static bool dev_room(int dev, double want, size_t *room) {
 }
 
 // ------------------------------------------------------------------ helpers
-static void dfree(pp_spv *h, void *p) {
-    if (!p) return;
-    auto it = h->sizes.find(p);
-    size_t b = 0;
-    if (it != h->sizes.end()) {
-        b = it->second;
-        h->bytes -= (long long)b;
-        h->sizes.erase(it);
-    }
-    cudaFreeAsync(p, h->stream);
-    if (b >= (1ull << 28)) {               // (only memory whose free has run can be returned)
-        cudaStreamSynchronize(h->stream);
-        pool_trim(h->dev, POOL_KEEP);
-    }
-}
-
-// Memory of the pool for work on stream s; nullptr when the device has no more (after
-// one try with everything unused returned to it).
-static void *pool_alloc(int dev, size_t b, cudaStream_t s, cudaError_t *e) {
+// Device memory for work on stream s; nullptr when the device has no more (after one try
+// with everything unused returned to it).
+static void *mem_get(int dev, size_t b, cudaStream_t s, cudaError_t *e) {
+    DevPool &d = dev_pool(dev);
     cudaMemPool_t pool = nullptr;
     void *q = nullptr;
     *e = cudaErrorMemoryAllocation;
     if (pool_get(dev, &pool)) return nullptr;
-    *e = cudaMallocFromPoolAsync(&q, b, pool, s);
+    const bool big = b >= MEM_BIG;
+    if (big) {
+        std::lock_guard<std::mutex> lk(d.mu);
+        size_t at = d.idle.size();
+        for (size_t k = 0; k < d.idle.size(); ++k) {
+            const size_t w = d.idle[k].second;
+            if (w >= b && w - b <= b / 4 && (at == d.idle.size() || w < d.idle[at].second)) at = k;
+        }
+        if (at < d.idle.size()) {
+            q = d.idle[at].first;
+            d.big[q] = d.idle[at].second;
+            d.idle_bytes -= d.idle[at].second;
+            d.idle.erase(d.idle.begin() + (long)at);
+            *e = cudaSuccess;
+            return q;
+        }
+    }
+    auto ask = [&]() { return big ? cudaMalloc(&q, b) : cudaMallocFromPoolAsync(&q, b, pool, s); };
+    *e = ask();
     if (*e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         cudaStreamSynchronize(s);
-        pool_trim(dev, 0);
-        *e = cudaMallocFromPoolAsync(&q, b, pool, s);
+        mem_trim(dev, 0);
+        *e = ask();
     }
     if (*e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    if (big) {
+        std::lock_guard<std::mutex> lk(d.mu);
+        d.big[q] = b;
+    }
     return q;
+}
+
+// Frees a block whose last work is on stream s (ended: that stream has been waited for).
+static void mem_put(int dev, void *p, cudaStream_t s, bool ended = false) {
+    DevPool &d = dev_pool(dev);
+    bool big;
+    {
+        std::lock_guard<std::mutex> lk(d.mu);
+        big = d.big.count(p) != 0;
+    }
+    if (!big) {
+        cudaFreeAsync(p, s);
+        return;
+    }
+    if (!ended) cudaStreamSynchronize(s);
+    {
+        std::lock_guard<std::mutex> lk(d.mu);
+        auto it = d.big.find(p);
+        d.idle.emplace_back(p, it->second);
+        d.idle_bytes += it->second;
+        d.big.erase(it);
+    }
+    mem_trim(dev, MEM_KEEP);
+}
+
+static void dfree(pp_spv *h, void *p) {
+    if (!p) return;
+    auto it = h->sizes.find(p);
+    if (it != h->sizes.end()) {
+        h->bytes -= (long long)it->second;
+        h->sizes.erase(it);
+    }
+    mem_put(h->dev, p, h->stream);
 }
 
 // (Re)allocates *p for count elements.  The new buffer is allocated before the
@@ -314,7 +386,7 @@ static int dalloc(pp_spv *h, T **p, long long count) {
         return fail(PP_OUT_OF_MEMORY, "cudaMalloc: injected allocation failure (pp_debug_fail_alloc)");
     const size_t b = (size_t)count * sizeof(T);
     cudaError_t e;
-    void *q = pool_alloc(h->dev, b, h->stream, &e);
+    void *q = mem_get(h->dev, b, h->stream, &e);
     if (!q) return fail(PP_OUT_OF_MEMORY, std::string("device allocation: ") + cudaGetErrorString(e));
     dfree(h, *p);
     *p = (T *)q;
@@ -428,10 +500,10 @@ static int grow_live(pp_spv *h, long long need, bool preserve = true, long long 
     // refuse a growth that would leave less than 4 GiB of device memory free; when
     // the doubled capacity does not fit, step down towards the capacity needed
     {
-        // (no question where the pool holds enough: the growth takes no more of the device)
+        // (no question where enough is held: the growth takes no more of the device)
         size_t freeb = 0;
         const double per = 2.0 * (2 * h->NW * 8 + 8) + 12.0 + 4.0 * TAU_MAX * 2.0 / SEG;
-        if (1.25 * (double)newcap * per > (double)pool_unused(h->dev) && dev_room(h->dev, (double)newcap * per, &freeb)) {
+        if (1.25 * (double)newcap * per > (double)mem_unused(h->dev) && dev_room(h->dev, (double)newcap * per, &freeb)) {
             const double room = (double)freeb - 4.0 * (1ull << 30);
             while ((double)newcap * per > room && newcap > need) newcap = std::max(need, newcap - newcap / 4);
             if ((double)newcap * per > room)
@@ -943,13 +1015,13 @@ extern "C" int pp_destroy(pp_spv *h) {
     std::vector<void *> live;              // every device buffer of the handle
     live.reserve(h->sizes.size());
     for (auto &kv : h->sizes) live.push_back(kv.first);
-    for (void *p : live) cudaFreeAsync(p, h->stream);
+    for (void *p : live) mem_put(h->dev, p, h->stream, true);
     if (h->bytes >= (1ll << 28)) cudaStreamSynchronize(h->stream);   // (freed memory can be returned then)
     if (h->Ph) cudaFreeHost(h->Ph);
     if (h->gens_h) cudaFreeHost(h->gens_h);
     if (h->bk_stat) cudaFreeHost(h->bk_stat);
     {
-        // the stream goes to the next handle; unused memory beyond the pool's bound, or all
+        // the stream goes to the next handle; unused memory beyond the bound, or all
         // of it with the last handle, goes back to the device
         DevPool &dp = dev_pool(h->dev);
         bool last;
@@ -963,7 +1035,7 @@ extern "C" int pp_destroy(pp_spv *h) {
         }
         if (h->stream) cudaStreamDestroy(h->stream);
         if (last) cudaDeviceSynchronize();
-        pool_trim(h->dev, last ? 0 : POOL_KEEP);
+        mem_trim(h->dev, last ? 0 : MEM_KEEP);
     }
     delete h;
     return PP_OK;
@@ -2077,11 +2149,11 @@ struct Scratch {
     std::vector<void *> p;
     explicit Scratch(pp_spv *h_) : h(h_) {}
     Scratch(const Scratch &) = delete;
-    ~Scratch() { for (void *q : p) cudaFreeAsync(q, h->stream); }
+    ~Scratch() { for (void *q : p) mem_put(h->dev, q, h->stream); }
     template <typename T>
     int get(T **out, long long count) {
         cudaError_t e;
-        void *q = pool_alloc(h->dev, (size_t)std::max(1ll, count) * sizeof(T), h->stream, &e);
+        void *q = mem_get(h->dev, (size_t)std::max(1ll, count) * sizeof(T), h->stream, &e);
         if (!q) return fail(PP_OUT_OF_MEMORY, "device allocation (scratch buffer)");
         p.push_back(q);
         *out = (T *)q;

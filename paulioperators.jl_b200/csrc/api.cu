@@ -1423,11 +1423,16 @@ static void bk_release(pp_spv *h) {
 // Moves the live bucket set *cur (2^*bits buckets) to a layout with more
 // buckets, doubling until the largest bucket holds at most half its capacity
 // (then no bucket of the next rotation's output can overflow).
-// For k_bb_block's buckets half full is what a new layout aims at, not what it needs: an
-// overflow is detected and its block runs again.  With 2^24 buckets and more the fullest
-// is beyond half at a mean of 5; where the next layout does not fit in memory, this one is
-// kept until a bucket overflows.  (256 instances of the 8 x 8 lattice, 3e8 terms at the
-// peak: 176 rotations of 2.4e8 terms 1.2 s in 2^25 buckets, 4.3 s on the sorted merges.)
+// For k_bb_block's buckets at most BB_ROOM, and that is what a new layout aims at, not
+// what it needs: an overflow is detected and its block runs again.  (A split doubles a mean
+// of 8 down to 4, where the fullest of 2^20 buckets and more is beyond half: asking for half
+// there took a layout of twice the size, and copied the set once more.  An evolve of a copy
+// of 2.2e6 terms by 32 rotations, 1.4e7 at the end: 34 ms with half, 14 so; the 8 x 8
+// lattice 85.3 and 84.5; a vector of 9.3e7 terms held 69 GiB, 37 so.)
+// Where the next layout does not fit in memory, the last one is kept until a bucket
+// overflows.  (256 instances of the 8 x 8 lattice, 3e8 terms at the peak: 176 rotations of
+// 2.4e8 terms 1.2 s in 2^25 buckets, 4.3 s on the sorted merges.)
+static constexpr int BB_ROOM = 3 * BB_CAP / 4;
 static constexpr int BB_FULL = 7 * BB_CAP / 8;
 template <int NW>
 static int bk_regrid(pp_spv *h, int *cur, int *bits) {
@@ -1441,7 +1446,7 @@ static int bk_regrid(pp_spv *h, int *cur, int *bits) {
         TRY(rr);
         int mx = 0;
         TRY(bk_scatter<NW>(h, h->bkz[*cur], h->bkx[*cur], h->bkc[*cur], 0, *cur, *bits, *cur ^ 1, nbits, &mx));
-        if (mx >= 0 && mx <= h->bk_cap / 2) break;
+        if (mx >= 0 && mx <= (h->bk_cap == BB_CAP ? BB_ROOM : h->bk_cap / 2)) break;
         held = h->bk_cap == BB_CAP && mx >= 0;
     }
     *cur ^= 1;

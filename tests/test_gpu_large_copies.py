@@ -1,5 +1,6 @@
 """An evolve of a copy of a large operator allocates and frees gigabytes on every call:
-that takes no multiple of the time of its kernels."""
+that takes no multiple of the time of its kernels, and the buckets of a grown set no
+layout of twice the size it needs."""
 import time
 
 import numpy as np
@@ -29,12 +30,16 @@ def _operator(N, n):
     return z.reshape(-1, 1), x.reshape(-1, 1), 10.0 ** rng.uniform(-4, -1, len(z))
 
 
+def _gens(N):
+    return [g for q in range(1, 13) for g in (circuits.zz(N, q, q + 1), circuits.xq(N, q))]
+
+
 def test_time_of_a_large_copy():
     # measured: in place 19 ms; a copy 192 ms when the bucket sets (8 GiB) came from a pool
     # that maps memory in small pieces, 27 since
     N = 64
     z, x, c = _operator(N, 2_300_000)
-    gens = [g for q in range(1, 13) for g in (circuits.zz(N, q, q + 1), circuits.xq(N, q))]
+    gens = _gens(N)
     trunc = pp.CompositeTruncation(pp.CoeffTruncation(1e-5), pp.WeightTruncation(12))
 
     def best(call):
@@ -69,4 +74,19 @@ def test_time_of_a_large_copy():
     assert n1 == n0 > 10_000_000
     assert t1 < 5 * min(times)
     v.close()
+    g.close()
+
+
+def test_buckets_of_a_grown_set():
+    # 3.0e7 terms of 24 bytes at the end: 17.8 GiB when a split asked for buckets at most
+    # half full, 9.7 since
+    N = 64
+    z, x, c = _operator(N, 2_300_000)
+    g = pp.SparsePauliVector(N, len(c), 16)
+    g.upload(z, x, c, sorted=True)
+    st = {}
+    pp.evolve_(g, _gens(N), [0.3] * 24, stats=st,
+               truncation=pp.CompositeTruncation(pp.CoeffTruncation(1e-5), pp.WeightTruncation(12)))
+    assert len(g) > 30_000_000 and st["bucket_rot"] == 24
+    assert g.device_bytes() < 12 << 30
     g.close()

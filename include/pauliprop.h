@@ -360,11 +360,14 @@ int pp_shard_end(pp_spv *h, double *expect_partial, double *stats_out);
  * them); a sequence whose live set outgrows the layout that fits continues on the
  * sorted-merge kernels with the same result.
  * pp_debug_sort_overflow: while on, every sort by samples of more than one bucket finds
- * a bucket beyond its slots and sorts by digits, with the same result. */
+ * a bucket beyond its slots and sorts by digits, with the same result.
+ * pp_debug_sort_plan (host only): buckets, samples per bucket and slots per bucket of a
+ * sort of n records (buckets 0: by digits). */
 int pp_debug_fail_alloc(int64_t after);
 int pp_debug_lookback_timeout(int64_t limit);
 int pp_debug_bucket_limit(int64_t slots);
 int pp_debug_sort_overflow(int32_t on);
+int pp_debug_sort_plan(int64_t n, int32_t *buckets, int32_t *samples, int32_t *slots);
 
 #ifdef __cplusplus
 }

@@ -2,9 +2,9 @@
 //
 // Records are ranked by (key, position), which no two share, so the sort is stable
 // and equal keys cannot make a bucket large:
-//   k_ss_sample  S = 8 (4 for the largest sets) evenly strided records per bucket;
+//   k_ss_sample  S = 8 evenly strided records per bucket;
 //   k_ss_rank    the rank of each sample, by counting over blocks of 256 x 256;
-//   k_ss_split   every 8th (4th) sample in rank order is a splitter;
+//   k_ss_split   every 8th sample in rank order is a splitter;
 //   k_ss_scatter each record to its bucket (binary search over the splitters in
 //                shared memory; a CTA takes a range of every bucket it meets from one
 //                atomic; the order inside a bucket does not matter);
@@ -25,10 +25,10 @@
 
 namespace pp {
 
-constexpr int SS_CAP = 4096;                   // slots of a bucket at most (2048 for small means: three CTAs per SM)
+constexpr int SS_CAP = 4096;                   // slots of a bucket at most (half of it for small means: three CTAs per SM)
 constexpr int SS_MAXB = 2048;                  // buckets at most
-constexpr int SS_SAMPLES = 8192;               // samples at most
-constexpr long long SS_MAX = 2200000;          // records at most (2048 buckets of 1075 on average)
+constexpr int SS_SAMPLES = 16384;              // samples at most
+constexpr long long SS_MAX = 2200000;          // records at most (2048 buckets of 1,075 on average)
 constexpr int SS_THREADS = 512;                // scatter
 constexpr int SS_ITEMS = 4;
 constexpr int SSS_THREADS = 512;               // bucket sort

@@ -135,6 +135,7 @@ SIGNATURES = {
     "pp_debug_lookback_timeout": (c_int32, [c_int64]),
     "pp_debug_bucket_limit": (c_int32, [c_int64]),
     "pp_debug_sort_overflow": (c_int32, [c_int32]),
+    "pp_debug_sort_plan": (c_int32, [c_int64, POINTER(c_int32), POINTER(c_int32), POINTER(c_int32)]),
     "pp_shard_owner": (c_int32, [c_int32, c_void_p, c_void_p, c_int64, c_int32, c_void_p]),
     "pp_shard_begin": (c_int32, [c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                  POINTER(PPEvolveOpts), c_int32, c_void_p]),

@@ -1174,11 +1174,32 @@ struct RunProf {
 // (kernels_block.cuh); the sequence ends with a packing into a dense array and a
 // sort, so the live set is dense and sorted between calls as before.
 static int expect_dev(pp_spv *h, const u64 *k, double *out);
-// Shorter sequences keep the sorted-merge kernels, which need no conversion: into buckets
-// and back costs about 0.2 ms up to 3e5 terms and 0.7 ms for 1.5e6, and saves 0.05 and 0.08
-// ms a rotation.  (With per-rotation times asked for, only long sequences: a block has no
-// separate rotate and merge times.)
-static int bk_min_rot(long long n, bool per_rot) { return per_rot ? 32 : n <= 300000 ? 6 : 8; }
+// Shorter sequences keep the sorted-merge kernels, which need no conversion into buckets and
+// back; they need room for a merge's output slots instead (roomy: the live sets have it, as
+// those of a vector that is evolved again and again; those of a copy have not).  Measured
+// (one B200; ms on merges and on buckets; n terms enter and grow by a tenth a rotation):
+//   n       rotations  one word    two words
+//   3.5e5    6 roomy   .52  .51    .61  .72
+//   3.5e5    6         .97  .93    1.06 1.03
+//   7.6e5    8 roomy   .82  .87    1.19 1.19
+//   7.6e5    8        1.39 1.14    1.72 1.44
+//   7.6e5   10 roomy  1.01  .94    1.51 1.25
+//   1.1e6    8        1.58 1.64    2.12 1.82
+//   1.1e6   12 roomy  1.54 1.99    2.45 2.03
+//   1.5e6   16 roomy  2.56 2.74    4.19 4.96
+//   1.5e6   24 roomy  4.44 4.42    6.84 6.11
+//   6.9e6   24        19.2 35.4    30.6 27.1
+//   6.9e6   32        48.9 47.3    45.5 66.2
+// What ends above SS_MAX records leaves buckets by the digit sort (from about 1e6 entering
+// terms on), and layouts of gigabytes have to be allocated.
+// (With per-rotation times asked for, only long sequences: a block has no separate rotate
+// and merge times.)
+static int bk_min_rot(long long n, bool roomy, bool per_rot) {
+    if (per_rot || n > 3000000) return 32;
+    if (n <= 300000) return 6;
+    if (n <= (roomy ? 1000000 : 1300000)) return roomy ? 10 : 8;
+    return 24;
+}
 // Internal status (never returned by the C ABI): a bucket layout for the live set
 // would not fit in device memory; the sequence continues on the sorted-merge
 // kernels from the rotation the device cursor is at.
@@ -1887,13 +1908,13 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
 }
 
 // Structured window-1 sequence over rotations [start, L) (the device cursor
-// S->rot is at start): chunks of CHUNK_ROT rotations between state read-backs; on
-// ERR_OVERFLOW grow and resume at the rotation that stopped.  While the live set
+// S->rot is at start, ncur terms are live): chunks of CHUNK_ROT rotations between
+// state read-backs; on ERR_OVERFLOW grow and resume at the rotation that stopped.  While the live set
 // fits k_small_run's shared memory (and the call has no local truncation,
 // correction or batched instances, and no per-rotation timing), one launch of it
 // runs the rotations instead.
 template <int NW>
-static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr, RunProf *prof, long long n_known = -1) {
+static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr, RunProf *prof, long long ncur) {
     long long done = start;
     const bool per_rot = ctr && (ctr->t_rotate || ctr->t_merge);   // per-rotation times asked for
     const bool timed = prof->on || per_rot;
@@ -1901,18 +1922,8 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
     bool table = false;            // the device segment table describes the (dense) live set
     const bool small_ok = !per_rot && !h->batch_on && !h->Ph->local_active && h->Ph->corr_kind == 0;
     bool use_bk = bk_enabled();
-    long long ncur = small_cap<NW>() + 1;   // live terms at the chunk's start (read when small_ok)
     bool dense = false;                      // the last state read showed a dense live set
     bool roomy = false;                      // the live sets have room for a merge's output slots
-    if (small_ok || n_known >= 0) {
-        if (n_known >= 0) {
-            ncur = n_known;
-        } else {
-            DevState st;
-            TRY(read_state(h, &st));
-            ncur = st.n;
-        }
-    }
     while (done < L) {
         if (small_ok && ncur <= small_cap<NW>()) {
             Bufs B = make_bufs(h);
@@ -1929,7 +1940,7 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
             done = st.rot;
             continue;
         }
-        if (use_bk && L - done >= bk_min_rot(ncur, per_rot)) {
+        if (use_bk && L - done >= bk_min_rot(ncur, 3 * ncur + 2 * SEG <= h->cap, per_rot)) {
             const int rb = run_bucket<NW>(h, done, L, ctr, prof, per_rot);
             if (rb != BK_NOFIT) return rb;
             bk_release(h);                  // their memory goes to the sorted-merge kernels
@@ -1941,7 +1952,7 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
             DevState st;
             TRY(read_state(h, &st));
             done = st.rot;
-            ncur = small_ok ? st.n : small_cap<NW>() + 1;
+            ncur = st.n;
             continue;
         }
         if (!roomy) {
@@ -3064,7 +3075,7 @@ static int batch_impl(pp_spv *h, const void *gz, const void *gx, long long L, co
             TRY(read_state(h, &st));
             st.rot_end = r;
             TRY(write_state(h, &st));
-            TRY(run_struct<2>(h, done, r, nullptr, &prof));
+            TRY(run_struct<2>(h, done, r, nullptr, &prof, st.n));
             done = r;
         }
         fin.clear();

@@ -199,7 +199,7 @@ struct DevPool {
     std::vector<cudaStream_t> streams;     // idle streams of destroyed handles (at most MAX_STREAMS)
     bool setup[2] = {false, false};        // launch attributes and occupancies of each word count
     int occ[2][4] = {};
-    size_t room = 0;                       // the last answer of dev_room, and when it was given
+    size_t room = 0;                       // the last answer of dev_room less the requests since, and when it was given
     std::chrono::steady_clock::time_point room_at;
     static constexpr size_t MAX_STREAMS = 16;
 };
@@ -269,16 +269,18 @@ static void mem_trim(int dev, size_t keep) {
     cudaGetLastError();
 }
 
-// Free device memory, what is held unused included.  cudaMemGetInfo takes 0.1 ms
-// and more, so an answer of the last quarter second stands in for requests of less than
-// an eighth of it.
+// Free device memory, what is held unused included, for a request of want bytes.
+// cudaMemGetInfo takes 0.1 ms and more, so an answer of the last quarter second, less what
+// was requested since, stands in where it leaves another 8 GiB.
 static bool dev_room(int dev, double want, size_t *room) {
     DevPool &d = dev_pool(dev);
     const auto now = std::chrono::steady_clock::now();
+    auto granted = [&]() { d.room -= (size_t)std::min(want, (double)d.room); };
     {
         std::lock_guard<std::mutex> lk(d.mu);
-        if (d.room > 0 && 8.0 * want < (double)d.room && now - d.room_at < std::chrono::milliseconds(250)) {
+        if (want + (double)(8ull << 30) < (double)d.room && now - d.room_at < std::chrono::milliseconds(250)) {
             *room = d.room;
+            granted();
             return true;
         }
     }
@@ -288,6 +290,7 @@ static bool dev_room(int dev, double want, size_t *room) {
     std::lock_guard<std::mutex> lk(d.mu);
     d.room = *room;
     d.room_at = now;
+    granted();
     return true;
 }
 

@@ -292,6 +292,9 @@ int pp_check(pp_spv *h, int32_t *ok);
 int pp_stream(pp_spv *h, void **stream);
 /* Bytes of device memory held by the handle. */
 int pp_device_bytes(pp_spv *h, int64_t *bytes);
+/* Returns to the current device what closed and shrunk vectors left: up to 8 GiB is kept
+ * for the next calls while any vector is alive (all of it goes back with the last one). */
+int pp_release_memory(void);
 /* lambda^k for k = 0..kmax with the compensated integer power used by the channel
  * tables (the algorithm of Julia's Float64^Integer). Host-only helper. */
 int pp_power_table(double lambda, int32_t kmax, double *out);

@@ -359,6 +359,19 @@ static void mem_put(int dev, void *p, cudaStream_t s, bool ended = false) {
     mem_trim(dev, MEM_KEEP);
 }
 
+// cudaMalloc for buffers outside the handles; what is held unused goes back to the device
+// where it has no more.
+static cudaError_t raw_malloc(void **q, size_t b) {
+    cudaError_t e = cudaMalloc(q, b);
+    int dev = 0;
+    if (e == cudaErrorMemoryAllocation && cudaGetDevice(&dev) == cudaSuccess) {
+        cudaGetLastError();
+        mem_trim(dev, 0);
+        e = cudaMalloc(q, b);
+    }
+    return e;
+}
+
 static void dfree(pp_spv *h, void *p) {
     if (!p) return;
     auto it = h->sizes.find(p);
@@ -2947,6 +2960,19 @@ extern "C" int pp_debug_lookback_timeout(int64_t limit) {
     return fail(PP_ERROR_EXCEPTION, "the look-back wait did not report its timeout");
 }
 
+extern "C" int pp_release_memory(void) {
+    int dev = 0;
+    CU(cudaGetDevice(&dev));
+    {
+        // (only memory whose free has run can be returned: destroyed handles free on their streams)
+        DevPool &d = dev_pool(dev);
+        std::lock_guard<std::mutex> lk(d.mu);
+        for (cudaStream_t s : d.streams) CU(cudaStreamSynchronize(s));
+    }
+    mem_trim(dev, 0);
+    return PP_OK;
+}
+
 extern "C" int pp_device_bytes(pp_spv *h, int64_t *bytes) {
     if (!h || !bytes) return fail(PP_ARGUMENT_ERROR, "null argument");
     *bytes = h->bytes;
@@ -3516,7 +3542,7 @@ struct pp_mlp {
 template <typename T>
 static int malloc_n(T **p, long long n) {
     T *q = nullptr;
-    MCU(cudaMalloc((void **)&q, (size_t)std::max(1ll, n) * sizeof(T)));
+    MCU(raw_malloc((void **)&q, (size_t)std::max(1ll, n) * sizeof(T)));
     if (*p) cudaFree(*p);
     *p = q;
     return PP_OK;
@@ -3711,8 +3737,8 @@ extern "C" int pp_features(pp_spv *h, const pp_feature_ctx *ctx, float *out, int
     if (!out) return fail(PP_ARGUMENT_ERROR, "null output");
     FeatCtx *dctx = nullptr;
     float *dout = nullptr;
-    CU(cudaMalloc((void **)&dctx, sizeof(FeatCtx)));
-    cudaError_t e = cudaMalloc((void **)&dout, (size_t)n * MLP_F * 4);
+    CU(raw_malloc((void **)&dctx, sizeof(FeatCtx)));
+    cudaError_t e = raw_malloc((void **)&dout, (size_t)n * MLP_F * 4);
     if (e != cudaSuccess) { cudaFree(dctx); return fail(PP_OUT_OF_MEMORY, "features buffer"); }
     cudaMemcpyAsync(dctx, ctx, sizeof(FeatCtx), cudaMemcpyHostToDevice, h->stream);
     k_features<<<h->nsm * 8, 256, 0, h->stream>>>(h->z[st.cur], h->x[st.cur], h->c[st.cur], n, dctx, dout);
@@ -3838,7 +3864,7 @@ extern "C" int pp_sample_terms(pp_spv *h, int32_t nbins, double lg_lo, double lg
     cudaStream_t s = h->stream;
     const int cur = st.cur;
     unsigned long long *dbuf = nullptr;
-    CU(cudaMalloc((void **)&dbuf, (size_t)(2 * 64 + 1 + 3 * cap) * 8));
+    CU(raw_malloc((void **)&dbuf, (size_t)(2 * 64 + 1 + 3 * cap) * 8));
     unsigned long long *hist = dbuf, *thr = dbuf + 64, *cnt = dbuf + 128;
     u64 *sz = dbuf + 129, *sx = sz + cap;
     double *sc = reinterpret_cast<double *>(sx + cap);

@@ -30,7 +30,7 @@ _DEVICE_NAMES = {
             "check_spv", "clip_", "coeff_clip_", "dephasing_channel", "dephasing_channel_",
             "depolarizing_channel", "depolarizing_channel_", "depolarizing_p_for_weight_decay", "evolve",
             "evolve_", "expectation_value", "majorana_weight_clip_", "pauli_channel", "pauli_channel_",
-            "phase_flip_channel_", "power_table", "truncate_", "weight_clip_", "weight_damped_clip_",
+            "phase_flip_channel_", "power_table", "release_memory", "truncate_", "weight_clip_", "weight_damped_clip_",
             "stochastic_clip_", "variance", "x_weight_clip_", "x_weight_damped_clip_"),
     "batch": ("BatchResult", "evolve_batch", "split_instances", "tagged_terms"),
     "learned": ("MLP", "features", "lattice_feature_ctx", "learned_truncate_"),

@@ -106,6 +106,7 @@ SIGNATURES = {
     "pp_stochastic_sample": (c_int32, [c_void_p, c_int64, c_uint64]),
     "pp_check": (c_int32, [c_void_p, POINTER(c_int32)]),
     "pp_stream": (c_int32, [c_void_p, POINTER(c_void_p)]),
+    "pp_release_memory": (c_int32, []),
     "pp_device_bytes": (c_int32, [c_void_p, POINTER(c_int64)]),
     "pp_power_table": (c_int32, [c_double, c_int32, c_void_p]),
     "pp_mlp_create": (c_int32, [POINTER(c_void_p)]),

@@ -606,3 +606,10 @@ def power_table(lam, kmax):
     out = np.zeros(kmax + 1, dtype=np.float64)
     check(lib.pp_power_table(float(lam), int(kmax), _ptr(out)))
     return out
+
+
+def release_memory():
+    """Returns to the device what closed and shrunk vectors left.  Up to 8 GiB of it is kept
+    for the next calls while any vector is alive; a program that needs it elsewhere (another
+    allocator of the process) calls this."""
+    check(lib.pp_release_memory())

@@ -153,6 +153,8 @@ struct pp_spv {
     u64 *bk_rows = nullptr;
     BkRec *bk_rec = nullptr;
     long long bk_rec_cap = 0;
+    unsigned long long *bk_rest = nullptr;  // EnergyCorrection: parts of the energy outside the units (BK_REST words a record)
+    long long bk_rest_cap = 0;
     u64 *ss_z = nullptr, *ss_x = nullptr, *ss_ws = nullptr;   // sample sort: bucketed records, samples
     double *ss_c = nullptr;
     unsigned *ss_p = nullptr;
@@ -1567,6 +1569,42 @@ static BbPlan bb_plan(const unsigned *delta, long long r0, int len, int bits, in
 
 static int norm2_dev(pp_spv *h, int cur, long long n, double *out);
 
+struct BbBlock {
+    long long r0;
+    int K;
+};
+
+// What rs_energy_rest added up over the blocks (rec: the records from start on), each of
+// the words' sums exact.
+static int energy_rest(pp_spv *h, long long start, const std::vector<BbBlock> &blocks, const std::vector<BkRec> &rec, double *out) {
+    __int128 a[BK_REST - 1] = {};
+    double special = 0.0;
+    bool any = false;
+    u64 w[BK_REST];
+    for (const BbBlock &b : blocks) {
+        if (!rec[(size_t)(b.r0 + 1 - start)].rest) continue;
+        any = true;
+        CU(cudaMemcpyAsync(w, h->bk_rest + (b.r0 + 1) * BK_REST, sizeof w, cudaMemcpyDeviceToHost, h->stream));
+        TRY(sync_check(h));
+        for (int k = 0; k + 1 < BK_REST; ++k) a[k] += (long long)w[k];
+        double d;
+        memcpy(&d, &w[BK_REST - 1], sizeof d);
+        special += d;
+    }
+    *out = 0.0;
+    if (!any) return PP_OK;
+    // words of 32 bits with a sign, then the smallest first
+    __int128 carry = 0;
+    for (int k = 0; k + 1 < BK_REST; ++k) {
+        const __int128 v = a[k] + carry;
+        const long long low = (long long)(int)(unsigned)(v & 0xffffffff);
+        carry = k + 2 < BK_REST ? (v - low) >> 32 : 0;
+        *out += k + 2 < BK_REST ? std::ldexp((double)low, 32 * k - 1074) : std::ldexp((double)v, 32 * k - 1074);
+    }
+    *out += special;
+    return PP_OK;
+}
+
 template <int NW>
 static int bb_init(pp_spv *h) {
     if (h->bb_occ[0][0]) return PP_OK;
@@ -1656,10 +1694,12 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         h->bk_delta_cap = L;
     }
     // EnergyCorrection: the dropped values are added up as multiples of a unit under the
-    // 2-norm of the entering set, which no rotation, filter or channel enlarges
+    // 2-norm of the entering set, which rotations, filters and channels do not enlarge.
+    // (A local truncation may, which drops one of two partners' sin branches, and a caller's
+    // cos and sin that are no rotation; values that the unit does not fit are added up too,
+    // one by one in memory.)
     double escale = 0.0;
     if (h->Ph->corr_kind == 1) {
-        // (cos and sin are the caller's: a pair that is no rotation could enlarge the set)
         for (long long r = start; r < L; ++r) {
             const GenRec &g = h->gens_h[r];
             if (!(g.cosv * g.cosv + g.sinv * g.sinv <= 1.0 + 1e-12)) return BK_NOFIT;
@@ -1669,7 +1709,12 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         if (!std::isfinite(nrm) || nrm > 0x1p900) return BK_NOFIT;         // (the sorted-merge kernels add doubles)
         int e = 0;
         std::frexp(nrm, &e);
-        escale = std::ldexp(1.0, -std::max(e + 1, -900));
+        escale = std::ldexp(1.0, -(e + 1));
+        if (L + 1 > h->bk_rest_cap) {
+            TRY(dalloc(h, &h->bk_rest, (L + 1) * BK_REST));
+            h->bk_rest_cap = L + 1;
+        }
+        CU(cudaMemsetAsync(h->bk_rest + (start + 1) * BK_REST, 0, (L - start) * BK_REST * sizeof(u64), s));
     }
     BkRec r0;
     memset(&r0, 0, sizeof r0);
@@ -1707,8 +1752,7 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
     // a rotation whose input values may not have passed the strict filter starts a block
     // that applies it to every term
     auto full_at = [&](long long r) { return r == start || (h->gens_h[r - 1].flags & GEN_CHANNEL) != 0; };
-    struct Block { long long r0; int K; };
-    std::vector<Block> blocks;             // completed blocks, in order
+    std::vector<BbBlock> blocks;           // completed blocks, in order
     // totals and counters of rotations [start, upto) into the device state, and the
     // live set (bucket set cur) back to the dense sorted layout
     auto finish = [&](long long upto) -> int {
@@ -1743,16 +1787,18 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
                 q[3] = pref ? 1 : 0;
             }
         }
-        for (const Block &b : blocks)      // a block reads its first rotation's terms and writes its last one's
+        for (const BbBlock &b : blocks)      // a block reads its first rotation's terms and writes its last one's
             prof->bk_bytes += (double)(16 * NW + 8) * ((double)rec[(size_t)(b.r0 - start)].n_out +
                                                        (double)rec[(size_t)(b.r0 + b.K - start)].n_out);
         if (escale != 0.0) {
             __int128 e[4] = {0, 0, 0, 0};
-            for (const Block &b : blocks)
+            for (const BbBlock &b : blocks)
                 for (int t = 0; t < 4; ++t) e[t] += (long long)rec[(size_t)(b.r0 + 1 - start)].energy[t];
             // smallest unit first: one rounding each
             const double sum = (double)e[3] * 0x1p-126 + (double)e[2] * 0x1p-94 + (double)e[1] * 0x1p-62 + (double)e[0] * 0x1p-30;
-            st.corr_energy -= sum / escale;
+            double rest = 0.0;
+            TRY(energy_rest(h, start, blocks, rec, &rest));
+            st.corr_energy -= rest + sum / escale;
         }
         if (h->rec_on && upto > start)
             CU(cudaMemcpy(h->rec + 4 * start, rr.data(), rr.size() * sizeof(long long), cudaMemcpyHostToDevice));
@@ -1801,6 +1847,7 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         BkArgs A = bk_args(h, bits, h->bk_rec);
         A.energy = escale != 0.0 ? 1 : 0;
         A.escale = escale;
+        A.rest = h->bk_rest;
         bool cta = false;
         const int dims = bb_dims<NW>(n, bits, limit, &cta);
         Chunk c{(long long)blocks.size(), 0, n, dims};
@@ -1879,6 +1926,7 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
             st.bk_pad = 0;
             TRY(write_state(h, &st));
             CU(cudaMemsetAsync(h->bk_rec + done + 1, 0, (launched - done) * sizeof(BkRec), s));
+            if (escale != 0.0) CU(cudaMemsetAsync(h->bk_rest + (done + 1) * BK_REST, 0, (launched - done) * BK_REST * sizeof(u64), s));
             CU(cudaMemcpyAsync(&last, h->bk_rec + done, sizeof last, cudaMemcpyDeviceToHost, s));
             TRY(sync_check(h));
             inflight.clear();

@@ -273,15 +273,39 @@ __device__ __forceinline__ bool rs_drop(const RsParams &q, const Key32<NW> &k, d
     return (absc <= q.strict.thresh) | rs_heavy<NW>(q, k);
 }
 
-// <ket|.|ket> of dropped terms (EnergyCorrection), added up exactly: a value, scaled to
-// at most 1 in magnitude, is cut into whole multiples of 2^-30, 2^-62, 2^-94 and 2^-126,
-// whose sums do not depend on the order.  A multiple is at most 2^31: the sums of all the
-// terms that a set may hold (2^31) stay within 64 bits.
+// <ket|.|ket> of dropped terms (EnergyCorrection), added up exactly, so that the sum does
+// not depend on the order.  A value, scaled by the unit of the call (about the 2-norm of the
+// entering set), is cut into whole multiples of 2^-30, 2^-62, 2^-94 and 2^-126: from 2^-70 to
+// 2 in magnitude that is all of it, and the sums of all the terms that a set may hold (2^31)
+// stay within 64 bits.  Other values, which are rare, go to words in global memory that
+// cover every double: word k counts multiples of 2^(32 k - 1074).
+static __device__ __noinline__ void rs_energy_rest(unsigned long long *word, int *flag, double v) {
+    *flag = 1;
+    const u64 b = (u64)__double_as_longlong(v);
+    int e = (int)(b >> 52) & 0x7ff;
+    u64 m = b & ((1ull << 52) - 1);
+    if (e == 0x7ff) {                                          // an infinity or NaN
+        atomicAdd(reinterpret_cast<double *>(word + BK_REST - 1), v);
+        return;
+    }
+    if (e) {
+        m |= 1ull << 52;
+        --e;
+    }
+    const int k = e >> 5, o = e & 31;                          // v = m 2^(e - 1074), 53 + 31 bits from word k on
+    const u64 part[3] = {(m << o) & 0xffffffffu, (m >> (32 - o)) & 0xffffffffu, o ? m >> (64 - o) : 0};
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+        if (part[t]) atomicAdd(word + k + t, (unsigned long long)((b >> 63) ? 0 - part[t] : part[t]));
+}
+
 template <int NW>
 struct RsEnergy {
     long long a[4];
     unsigned ket[2 * NW];
     double scale;
+    unsigned long long *rest;
+    int *rest_flag;
     __device__ __forceinline__ void add(const Key32<NW> &k, double v) {
         unsigned x = 0, s = 0;
 #pragma unroll
@@ -290,8 +314,12 @@ struct RsEnergy {
             s ^= k.w[t] & ket[t];
         }
         if (x) return;
+        if (__popc(s) & 1) v = -v;
         double r = v * scale;
-        if (__popc(s) & 1) r = -r;
+        if (!(fabs(r) >= 0x1p-70 && fabs(r) <= 2.0)) {
+            if (v != 0.0) rs_energy_rest(rest, rest_flag, v);
+            return;
+        }
         const double g[4] = {0x1p30, 0x1p62, 0x1p94, 0x1p126}, u[4] = {0x1p-30, 0x1p-62, 0x1p-94, 0x1p-126};
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
@@ -628,6 +656,8 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
     RsEnergy<NW> en = {};
     if constexpr (ENERGY) {
         en.scale = A.escale;
+        en.rest = A.rest + (r0 + 1) * BK_REST;
+        en.rest_flag = &A.rec[r0 + 1].rest;
 #pragma unroll
         for (int t = 0; t < 2 * NW; ++t) en.ket[t] = (unsigned)(P.ket[t >> 1] >> (32 * (t & 1)));
     }

@@ -67,7 +67,9 @@ struct BkRec {
     unsigned long long energy[4];   // EnergyCorrection: <ket|.|ket> of what the block dropped (RsEnergy)
     int pref;                       // the rotation began with an early merge (CTA 0)
     int maxcnt;                     // largest output bucket
+    int rest, pad;                  // EnergyCorrection: 1 if the block's energy has a part in BkArgs::rest
 };
+constexpr int BK_REST = 67;         // words of that part (rs_energy_rest)
 
 struct BkArgs {
     u64 *z[2], *x[2];               // bucket sets: slot j of bucket b at b * CAP + j (NW words per key)
@@ -101,6 +103,7 @@ struct BkArgs {
     long long vals_cap;
     int energy;                     // 1: EnergyCorrection, values scaled by escale (a power of two)
     double escale;
+    unsigned long long *rest;       // EnergyCorrection: BK_REST words per record
 };
 
 // Bucket of a key: the low `bits` bits of the GF(2)-linear hash.

@@ -2407,7 +2407,8 @@ static int adapt_step(pp_spv *h, AdaptSpec &A) {
 // listed |c|; nothing comes back to the host but the state of a chunk of rotations.
 // For sequences without early merges (the caller has seen to that: n and max_terms are
 // at most the append capacity), corrections and WindowCounters.  period: a channel after
-// every period-th rotation, behind its truncation.  BK_NOFIT: nothing was changed.
+// every period-th rotation, behind its truncation.  BK_NOFIT: a layout does not fit; the
+// rotations up to *reached have run (it is not touched where none has).
 // Measured (one B200, budget 20,000 on a 30-qubit chain, 351 rotations): 70.5 ms with a
 // sorted merge, a select and a clip per rotation, each with host round trips (200 us a
 // rotation).
@@ -2415,7 +2416,8 @@ static constexpr int ADAPT_MIN_ROT = 8;
 static constexpr int ADAPT_CHUNK = 64;
 
 template <int NW>
-static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, int chan_flags, RunProf *prof, AdaptSpec &Q) {
+static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, int chan_flags, RunProf *prof, AdaptSpec &Q,
+                     long long *reached) {
     TRY(bk_rows_init(h));
     TRY(bb_init<NW>(h));
     cudaStream_t s = h->stream;
@@ -2473,6 +2475,42 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
                        cudaMemcpyDeviceToHost, s));
     TRY(sync_check(h));
     PP_TRACE("adaptive on buckets: rotations [%lld, %lld), %lld live terms, 2^%d buckets", start, L, n0, bits);
+    // rotations [start, upto) into the state: totals, as the merges and clips of the general
+    // path count them; the live set dense and sorted; the cut after the last rotation and its
+    // channel
+    auto finish = [&](long long upto) -> int {
+        std::vector<BkRec> rec((size_t)(upto - start + 1));
+        CU(cudaMemcpyAsync(rec.data(), h->bk_rec + start, rec.size() * sizeof(BkRec), cudaMemcpyDeviceToHost, s));
+        TRY(sync_check(h));
+        for (long long r = start; r < upto; ++r) {
+            const BkRec &o = rec[(size_t)(r - start + 1)];
+            st.live_in += (long long)o.np;
+            st.created += (long long)o.created;
+            st.merge_in += (long long)o.np + (long long)o.created + (long long)o.n_out;
+            st.merge_out += (long long)o.n_out + (r + 1 < upto ? (long long)rec[(size_t)(r - start + 2)].np : 0);
+            st.peak = std::max(st.peak, (long long)o.n_out);
+        }
+        const long long n = (long long)rec.back().n_out;
+        st.merge_in -= n;                  // the last clip is a merge of its own below
+        prof->bk_rot += upto - start;
+        TRY(write_state(h, &st));
+        TRY(bk_to_dense<NW>(h, cur, bits, n));
+        compile_filter(nullptr, &h->Ph->clip);
+        TRY(upload_params(h));
+        CU(cudaMemcpyAsync(&h->P->clip.thresh, h->bk_thr + upto, sizeof(double), cudaMemcpyDeviceToDevice, s));
+        Bufs B = make_bufs(h);
+        launch_merge<NW, 2>(h, B, 0);
+        prof->launches += 3;
+        TRY(sync_check(h));
+        TRY(read_state(h, &st));
+        TRY(check_err(h, st));
+        if (h->Ph->chan_kind >= 0 && (h->gens_h[upto - 1].flags & chan_flags)) {
+            Bufs Bc = make_bufs(h);
+            k_channel<NW><<<h->nsm * 8, 256, 0, s>>>(Bc);
+            TRY(sync_check(h));
+        }
+        return PP_OK;
+    };
     int limit = BB_DMAX;
     long long done = start;
     while (done < L) {
@@ -2520,44 +2558,17 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
             if (over & 2) limit = std::max(1, dims - 1);
             if (over & 1) {
                 const int rr = bk_regrid<NW>(h, &cur, &bits);
-                if (rr == BK_NOFIT) return fail(PP_OUT_OF_MEMORY, "the bucket layout of this sequence does not fit in device memory");
+                if (rr == BK_NOFIT && done > start) {
+                    // no room for a larger layout: what has run goes back to the dense set
+                    TRY(finish(done));
+                    *reached = done;
+                }
                 if (rr) return rr;
                 TRY(vals_reserve());
             }
         }
     }
-    // totals, as the merges and clips of the general path count them
-    std::vector<BkRec> rec((size_t)(L - start + 1));
-    CU(cudaMemcpyAsync(rec.data(), h->bk_rec + start, rec.size() * sizeof(BkRec), cudaMemcpyDeviceToHost, s));
-    TRY(sync_check(h));
-    for (long long r = start; r < L; ++r) {
-        const BkRec &o = rec[(size_t)(r - start + 1)];
-        st.live_in += (long long)o.np;
-        st.created += (long long)o.created;
-        st.merge_in += (long long)o.np + (long long)o.created + (long long)o.n_out;
-        st.merge_out += (long long)o.n_out + (r + 1 < L ? (long long)rec[(size_t)(r - start + 2)].np : 0);
-        st.peak = std::max(st.peak, (long long)o.n_out);
-    }
-    const long long n = (long long)rec.back().n_out;
-    st.merge_in -= n;                      // the last clip is a merge of its own below
-    prof->bk_rot += L - start;
-    TRY(write_state(h, &st));
-    TRY(bk_to_dense<NW>(h, cur, bits, n));
-    // the cut after the last rotation, its channel, and <ket|O|ket>
-    compile_filter(nullptr, &h->Ph->clip);
-    TRY(upload_params(h));
-    CU(cudaMemcpyAsync(&h->P->clip.thresh, h->bk_thr + L, sizeof(double), cudaMemcpyDeviceToDevice, s));
-    Bufs B = make_bufs(h);
-    launch_merge<NW, 2>(h, B, 0);
-    prof->launches += 3;
-    TRY(sync_check(h));
-    TRY(read_state(h, &st));
-    TRY(check_err(h, st));
-    if (h->Ph->chan_kind >= 0 && (h->gens_h[L - 1].flags & chan_flags)) {
-        Bufs Bc = make_bufs(h);
-        k_channel<NW><<<h->nsm * 8, 256, 0, s>>>(Bc);
-        TRY(sync_check(h));
-    }
+    TRY(finish(L));
     if (last_flags & GEN_MEASURE) {
         double e = 0.0;
         TRY(expect_dev(h, h->Ph->ket, &e));
@@ -2603,9 +2614,17 @@ static int run_general(pp_spv *h, const std::vector<GenRec> &G, long long window
         if (adapt_bk && L - i + 1 >= ADAPT_MIN_ROT && exact && st.an == 0 && st.n <= AS_MAX &&
             std::max(st.n, A.max_terms) <= st.acap_logical) {
             // no early merge from here on: the rest on buckets
-            const int rr = run_adapt<NW>(h, i - 1, L, last_flags, chan_flags, prof, A);
+            long long reached = i - 1;
+            const int rr = run_adapt<NW>(h, i - 1, L, last_flags, chan_flags, prof, A, &reached);
             if (rr != BK_NOFIT) return rr;
             adapt_bk = false;
+            bk_release(h);
+            if (reached >= i) {
+                exact = false;
+                TRY(look());
+                i = reached;
+                continue;
+            }
         }
         if (exact && 2 * st.an + st.n > st.acap_logical) {
             long long ni, no;

@@ -2489,6 +2489,7 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
             st.merge_in += (long long)o.np + (long long)o.created + (long long)o.n_out;
             st.merge_out += (long long)o.n_out + (r + 1 < upto ? (long long)rec[(size_t)(r - start + 2)].np : 0);
             st.peak = std::max(st.peak, (long long)o.n_out);
+            prof->bk_bytes += (double)(16 * NW + 8) * ((double)rec[(size_t)(r - start)].n_out + (double)o.n_out);
         }
         const long long n = (long long)rec.back().n_out;
         st.merge_in -= n;                  // the last clip is a merge of its own below
@@ -2511,6 +2512,13 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
         }
         return PP_OK;
     };
+    cudaEvent_t ev[2] = {nullptr, nullptr};   // around a chunk's launches (profiled calls)
+    struct EvGuard {
+        cudaEvent_t *v;
+        ~EvGuard() { for (int k = 0; k < 2; ++k) if (v[k]) cudaEventDestroy(v[k]); }
+    } evg{ev};
+    if (prof->on)
+        for (auto &e : ev) CU(cudaEventCreate(&e));
     int limit = BB_DMAX;
     long long done = start;
     while (done < L) {
@@ -2525,6 +2533,7 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
         st.bk_fail = 0x7fffffffffffffffll;
         st.bk_pad = 0;
         TRY(write_state(h, &st));
+        if (prof->on) CU(cudaEventRecord(ev[0], s));
         for (long long r = done; r < end; ++r) {
             BbPlan pl = bb_plan(delta.data(), r, 1, bits, dims);
             pl.cur = (cur + (int)(r - done)) & 1;
@@ -2544,7 +2553,13 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
                                   h->bk_thr + r + 1));
             prof->launches += 2;
         }
+        if (prof->on) CU(cudaEventRecord(ev[1], s));
         TRY(sync_check(h));
+        if (prof->on) {
+            float ms = 0.f;
+            CU(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+            prof->t_merge += ms * 1e-3;
+        }
         TRY(read_state(h, &st));
         if (st.err & ~ERR_OVERFLOW) return check_err(h, st);
         const long long upto = st.err & ERR_OVERFLOW ? std::max(done, std::min(end, st.bk_fail)) : end;

@@ -137,8 +137,7 @@ struct pp_spv {
     cudaGraphExec_t gexec[3] = {nullptr, nullptr, nullptr};
     long long gexec_gen[3] = {-1, -1, -1};
     // bucketed window-1 rotations (kernels_bucket.cuh): two bucket sets of
-    // 2^bk_bits_cap buckets of bk_cap slots, hash rows, per-rotation records,
-    // dense offsets, and the captured rotation graphs per bucket count
+    // 2^bk_bits_cap buckets of bk_cap slots, hash rows, per-rotation records
     u64 *bkz[2] = {nullptr, nullptr}, *bkx[2] = {nullptr, nullptr};
     double *bkc[2] = {nullptr, nullptr};
     int *bkcnt[2] = {nullptr, nullptr};
@@ -1231,7 +1230,7 @@ static bool bk_enabled() {
 }
 
 // Compiled variants of k_bk_rotate (key-sharded runs): (bucket capacity, staged items per thread).
-typedef void (*BkKernel)(BkArgs, int);
+typedef void (*BkKernel)(BkArgs, long long, int, int);
 struct BkVariant {
     int cap, items;
     BkKernel k1, k2;                // one- and two-word keys
@@ -1252,25 +1251,12 @@ static const BkVariant *bk_variant(int cap, int items) {
 }
 
 template <int NW>
-static void bk_launch(pp_spv *h, const BkVariant *v, const BkArgs &A, int k) {
+static void bk_launch(pp_spv *h, const BkVariant *v, const BkArgs &A, long long r, int cur, int pref) {
     // persistent grid: every resident CTA, or one per bucket pair (the kernel sizes its groups)
     const long long pairs = 1ll << (A.bits - 1);
     const auto &oc = h->bk_occ[v - BK_VARIANTS];
-    const int occ = NW == 1 ? oc.occ1 : oc.occ2;
-    const int grid = (int)std::min(pairs, (long long)h->nsm * occ);
-    // programmatic dependent launch: the rotation's prologue overlaps the previous
-    // rotation's tail (k_bk_rotate waits for its outputs in griddepcontrol.wait)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(BK_THREADS);
-    cfg.dynamicSmemBytes = NW == 1 ? v->smem1 : v->smem2;
-    cfg.stream = h->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, NW == 1 ? v->k1 : v->k2, A, k);
+    const int grid = (int)std::min(pairs, (long long)h->nsm * (NW == 1 ? oc.occ1 : oc.occ2));
+    (NW == 1 ? v->k1 : v->k2)<<<grid, BK_THREADS, NW == 1 ? v->smem1 : v->smem2, h->stream>>>(A, r, cur, pref);
 }
 
 // Hash rows: fixed pseudo-random words (splitmix64 from a fixed seed), so the
@@ -1337,7 +1323,6 @@ static BkArgs bk_args(pp_spv *h, int bits, BkRec *rec) {
     A.S = h->S;
     A.P = h->P;
     A.gens = h->gens;
-    A.pref_forced = -1;
     if (h->batch_on) {
         A.bcos = h->bcos;
         A.bsin = h->bsin;
@@ -1834,7 +1819,7 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
         for (int k = timed ? 0 : 2; k < 3; ++k)
             CU(cudaEventCreateWithFlags(&cev[i][k], timed ? cudaEventDefault : cudaEventDisableTiming));
     st.bk_fail = 0x7fffffffffffffffll;
-    st.bk_pad = 0;
+    st.bk_over = 0;
     TRY(write_state(h, &st));
     long long done = start, launched = start, n = n0, seq = 0;
     double growth = 4.0;                   // of the live set over the last chunk
@@ -1918,12 +1903,12 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
             // (which did nothing) run again
             TRY(sync_check(h));
             TRY(read_state(h, &st));
-            over = st.bk_pad;
+            over = st.bk_over;
             while (!blocks.empty() && blocks.back().r0 >= st.bk_fail) { blocks.pop_back(); cur ^= 1; }
             done = blocks.empty() ? start : blocks.back().r0 + blocks.back().K;
             st.err &= ~ERR_OVERFLOW;
             st.bk_fail = 0x7fffffffffffffffll;
-            st.bk_pad = 0;
+            st.bk_over = 0;
             TRY(write_state(h, &st));
             CU(cudaMemsetAsync(h->bk_rec + done + 1, 0, (launched - done) * sizeof(BkRec), s));
             if (escale != 0.0) CU(cudaMemsetAsync(h->bk_rest + (done + 1) * BK_REST, 0, (launched - done) * BK_REST * sizeof(u64), s));
@@ -2531,7 +2516,7 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
         int dims = 1;
         while (dims < limit && dims < bits && (most << (dims + 1)) <= (64ll << bits)) ++dims;
         st.bk_fail = 0x7fffffffffffffffll;
-        st.bk_pad = 0;
+        st.bk_over = 0;
         TRY(write_state(h, &st));
         if (prof->on) CU(cudaEventRecord(ev[0], s));
         for (long long r = done; r < end; ++r) {
@@ -2566,7 +2551,7 @@ static int run_adapt(pp_spv *h, long long start, long long L, int last_flags, in
         cur = (cur + (int)(upto - done)) & 1;
         done = upto;
         if (st.err & ERR_OVERFLOW) {
-            const int over = st.bk_pad;
+            const int over = st.bk_over;
             st.err &= ~ERR_OVERFLOW;
             TRY(write_state(h, &st));
             CU(cudaMemsetAsync(h->bk_rec + done + 1, 0, (end - done) * sizeof(BkRec), s));
@@ -3496,9 +3481,7 @@ static int shard_rotate_impl(pp_spv *h, int64_t r, int pref, int remote, int64_t
     A.fcnt[0] = h->bkfcnt[0];
     A.fcnt[1] = h->bkfcnt[1];
     A.remote = remote;
-    A.pref_forced = pref ? 1 : 0;
-    k_bk_begin<<<1, 1, 0, s>>>(h->S, r, h->shard_cur, 1);
-    bk_launch<NW>(h, var, A, 0);
+    bk_launch<NW>(h, var, A, r, h->shard_cur, pref ? 1 : 0);
     BkRec o;
     CU(cudaMemcpyAsync(&o, h->bk_rec + r + 1, sizeof o, cudaMemcpyDeviceToHost, s));
     TRY(sync_check(h));

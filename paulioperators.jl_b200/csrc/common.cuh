@@ -88,10 +88,9 @@ struct DevState {
     int measure_valid;
     int seg_dense;                // 0: live set cur is the last window-1 merge's per-tile slots (segment table)
     int pad;
-    long long bk_rot0;            // bucketed rotations: first rotation of the launched group
-    long long bk_fail;            // bucketed rotations: first rotation whose output overflowed a bucket
-    int bk_cur0;                  // bucketed rotations: input bucket set of the group's first rotation
-    int bk_pad;
+    long long bk_fail;            // bucketed rotations: first rotation of the first block that overflowed
+    int bk_over;                  // and how (bits): 1 a bucket, 2 a coset beyond the resident set
+    int pad2;
     unsigned long long dbg;       // first failed device check: site << 40 | value (0: none)
 };
 
@@ -115,7 +114,8 @@ static_assert(A_TILE >= SEG, "a classify tile holds one live segment");
 constexpr int G_THREADS = 256;
 // Four terms a thread: a window's live and pending terms are 1e4 to 1e5, where tiles of 2,048
 // left most SMs without one (a window-8 sequence of 372 rotations, up to 6.9e3 live terms:
-// 7.76 ms with eight, 7.31 with four).
+// 7.76 ms with eight, 7.31 with four), and larger sets lose nothing by it (16 rotations at
+// window 8 of 8e5 and 2.2e6 entering terms: 1.15 and 2.75 ms with eight, 1.12 and 2.55).
 constexpr int G_ITEMS = 4;
 constexpr int G_TILE = G_THREADS * G_ITEMS;   // general rotate tile
 constexpr int SPIN_LIMIT = 1 << 22;           // bounded look-back waits

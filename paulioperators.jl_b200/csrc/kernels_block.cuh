@@ -530,8 +530,8 @@ constexpr int BB_PLAIN = 0, BB_BATCH = 1, BB_ADAPT = 2, BB_ENERGY = 3;
 // One block of rotations; input bucket set pl.cur, output set pl.cur ^ 1 (the input
 // stays intact, so a block that does not fit -- a coset beyond the resident set, or
 // an output bucket beyond BB_CAP -- is flagged and run again by the host, after a
-// split or with fewer rotations).  Persistent grid; every warp takes cosets of its
-// own, so no block barrier stands between a rotation and the next.
+// split or with fewer rotations).  Persistent grid; T threads take a coset at a time: a
+// warp, whose rotations need no block barrier between them, or the CTA.
 template <int NW, int MODE, int T>
 __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_constant__ BkArgs A,
                                                                const __grid_constant__ BbPlan pl) {
@@ -864,7 +864,7 @@ __global__ void __launch_bounds__(32 * BB_WARPS, 3) k_bb_block(const __grid_cons
         if (drop_first) atomicAdd(&A.rec[r0 + 1].np, (unsigned long long)s_np);
         atomicMax(&A.rec[r0 + K].maxcnt, s_mx);
         if (s_over) {
-            atomicOr(&S->bk_pad, s_over);                  // 1: a bucket overflowed, 2: a coset beyond the resident set
+            atomicOr(&S->bk_over, s_over);                  // 1: a bucket overflowed, 2: a coset beyond the resident set
             atomicMin(&S->bk_fail, r0);
             atomicOr(&S->err, ERR_OVERFLOW);
         }

@@ -91,11 +91,9 @@ struct BkArgs {
     int ncol;
     // key-sharded runs: per bucket, foreign terms (received from the partner rank)
     // follow the local ones; remote: the sin branches of local terms belong to the
-    // partner rank; pref_forced: the early-merge decision from the global counts
-    // (-1: from the rotation record, as on one rank)
+    // partner rank
     int *fcnt[2];
     int remote;
-    int pref_forced;
     // adaptive sequences: the threshold that cuts the set entering each rotation, and the
     // list of the survivors' |c|
     const double *thr;
@@ -272,11 +270,11 @@ __device__ __forceinline__ void bk_pair(unsigned delta, long long p, int *b0, in
 // and that leaves every CTA a group.  A group whose terms exceed the staging
 // area is processed in sub-groups of consecutive pairs, loaded in turn (a single
 // pair always fits: 2 * CAP <= BK_THREADS * ITEMS).  Three block barriers per
-// group: staged terms visible, key index built, outputs claimed.  k is the
-// rotation's index within the launched graph (rotation S->bk_rot0 + k, input set
-// (S->bk_cur0 + k) & 1).
+// group: staged terms visible, key index built, outputs claimed.  Rotation r from
+// bucket set cur to the other one; pref: it starts with an early merge (the ranks
+// decide that from the counts over all of them).
 template <int NW, int CAP, int ITEMS>
-__global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rotate(BkArgs A, int k) {
+__global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rotate(BkArgs A, long long r, int cur, int pref) {
     constexpr int T = BK_THREADS;
     constexpr int SMI = T * ITEMS;                 // staged terms per area
     constexpr int TAB = 2 * SMI;                   // key index slots
@@ -286,15 +284,8 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
     static_assert(NBK <= 32, "one warp handles a group's buckets");
     static_assert(SMI < 0x10000, "16-bit key index entries");
     DevState *S = A.S;
-    // Launched as a programmatic dependent of the previous rotation: the next
-    // rotation's CTAs may start as this one's finish.  Everything before
-    // griddepcontrol.wait reads only what no rotation writes (the cursor set
-    // before the graph launch, the generator, the hash rows).
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ int s_err;
-    const long long r = S->bk_rot0 + k;
     if (r >= S->rot_end) return;
-    const int cur = (S->bk_cur0 + k) & 1;
     __shared__ GenRec g;
     __shared__ unsigned s_delta;
     __shared__ int s_b[2][NBK], s_n[2][NBK], s_nl[2][NBK], s_off[2][NBK + 1], s_j1[2];
@@ -328,24 +319,15 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
         for (int i = tid; i < TAB / 8; i += T) t4[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     if (tid < NBK) s_out[tid] = 0;
-    // the previous rotation's outputs (and error word) are visible from here on;
     // one read of the error word for the whole CTA (another CTA may set it meanwhile)
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (tid == 0) s_err = S->err;
     __syncthreads();
     if (s_err) return;
-    // the state entering this rotation, from the previous rotation's record (the
-    // early-merge rule of spv_evolve.jl:356-362)
-    const BkRec &prev = A.rec[r];
-    const long long n_r = (long long)prev.n_out;
-    long long acap = prev.acap;
-    if (prev.pref && (long long)prev.np > acap) acap = max(2 * acap, (long long)prev.np);
-    const bool pref = A.pref_forced >= 0 ? A.pref_forced != 0 : n_r > acap;
+    const long long n_r = (long long)A.rec[r].n_out;
     if (blockIdx.x == 0 && tid == 0) {
         BkRec &me = A.rec[r + 1];
         me.n_in = n_r;
-        me.acap = acap;
-        me.pref = pref ? 1 : 0;
+        me.pref = pref;
     }
     const unsigned delta = s_delta;
     const long long nb = 1ll << A.bits;
@@ -360,8 +342,8 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
     // (selected, not indexed: a runtime index into the parameter struct would copy it to the stack)
     const int *CNT = cur ? A.cnt[1] : A.cnt[0];
     int *OCNT = cur ? A.cnt[0] : A.cnt[1];
-    const int *FCNT = A.fcnt[0] ? (cur ? A.fcnt[1] : A.fcnt[0]) : nullptr;
-    int *OFCNT = A.fcnt[0] ? (cur ? A.fcnt[0] : A.fcnt[1]) : nullptr;
+    const int *FCNT = cur ? A.fcnt[1] : A.fcnt[0];
+    int *OFCNT = cur ? A.fcnt[0] : A.fcnt[1];
     const bool remote = A.remote != 0;
     const u64 *Z = cur ? A.z[1] : A.z[0], *X = cur ? A.x[1] : A.x[0];
     const double *C = cur ? A.c[1] : A.c[0];
@@ -388,7 +370,8 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
                 else {
                     n0 = CNT[b0];
                     n1 = CNT[b1];
-                    if (FCNT) { f0 = FCNT[b0]; f1 = FCNT[b1]; }
+                    f0 = FCNT[b0];
+                    f1 = FCNT[b1];
                     if (n0 < 0 || n1 < 0 || f0 < 0 || f1 < 0 || n0 + f0 > CAP || n1 + f1 > CAP) {
                         flag_bounds(S, 4, ((long long)n0 << 20) | (n1 & 0xfffff));
                         s_bad = 1;
@@ -625,7 +608,8 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
             if (pb0 < nb && pb1 < nb) {
                 pn0 = CNT[pb0];
                 pn1 = CNT[pb1];
-                if (FCNT) { pf0 = FCNT[pb0]; pf1 = FCNT[pb1]; }
+                pf0 = FCNT[pb0];
+                pf1 = FCNT[pb1];
             }
         }
         staged(a);
@@ -650,7 +634,7 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
             if (lane < 2 * G) {
                 const int m = s_out[lane];
                 OCNT[s_b[a][lane]] = min(m, CAP);
-                if (OFCNT) OFCNT[s_b[a][lane]] = 0;
+                OFCNT[s_b[a][lane]] = 0;
                 atomicMax(&s_mx, m);
                 s_out[lane] = 0;
             }
@@ -690,20 +674,9 @@ __global__ void __launch_bounds__(BK_THREADS, bk_min_blocks(NW, ITEMS)) k_bk_rot
         atomicAdd(&me.created, (unsigned long long)ct);
         if (pref) atomicAdd(&me.np, (unsigned long long)at);
         atomicMax(&me.maxcnt, s_mx);
-        if (s_mx > CAP) {
-            atomicOr(&S->err, ERR_OVERFLOW);
-            atomicMin(&S->bk_fail, r);
-        }
+        if (s_mx > CAP) atomicOr(&S->err, ERR_OVERFLOW);
         if (s_bad) atomicOr(&S->err, ERR_BOUNDS);
     }
-}
-
-// Start of a launched group of rotations: its first rotation and input set
-// (and, at the start of a chunk, no failed rotation yet).
-__global__ void k_bk_begin(DevState *S, long long rot0, int cur0, int reset_fail) {
-    S->bk_rot0 = rot0;
-    S->bk_cur0 = cur0;
-    if (reset_fail) S->bk_fail = 0x7fffffffffffffffll;
 }
 
 // Scatter into a bucket layout of capacity 2^cap_log (counts zeroed beforehand).

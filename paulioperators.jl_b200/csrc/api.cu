@@ -1456,16 +1456,19 @@ static void bk_release(pp_spv *h) {
 // Moves the live bucket set *cur (2^*bits buckets) to a layout with more
 // buckets, doubling until the largest bucket holds at most half its capacity
 // (then no bucket of the next rotation's output can overflow).
-// For k_bb_block's buckets at most BB_ROOM, and that is what a new layout aims at, not
-// what it needs: an overflow is detected and its block runs again.  (A split doubles a mean
-// of 8 down to 4, where the fullest of 2^20 buckets and more is beyond half: asking for half
-// there took a layout of twice the size, and copied the set once more.  An evolve of a copy
-// of 2.2e6 terms by 32 rotations, 1.4e7 at the end: 34 ms with half, 14 so; the 8 x 8
-// lattice 85.3 and 84.5; a vector of 9.3e7 terms held 69 GiB, 37 so.)
+// For k_bb_block's buckets, from 2^BB_ROOM_BITS on, at most BB_ROOM, and that is what a new
+// layout aims at, not what it needs: an overflow is detected and its block runs again.  (A
+// split halves a mean of 8, and the fullest of so many buckets of 4 is beyond half: asking
+// for half there took a layout of twice the size, and copied the set once more.  An evolve of
+// a copy of 2.2e6 terms by 32 rotations, 1.4e7 at the end: 34 ms with half, 14 so; a batch of
+// 48 instances, 1e6 terms: 38.0 and 35.8; a vector of 9.3e7 terms held 69 GiB, 37 so.
+// Smaller layouts cost little, and emptier buckets split later: an evolve of a copy of 2.4e5
+// terms by 32 rotations 1.95 ms with half, 2.04 with BB_ROOM; of 1.6e4 in place 0.66, 0.72.)
 // Where the next layout does not fit in memory, the last one is kept until a bucket
 // overflows.  (256 instances of the 8 x 8 lattice, 3e8 terms at the peak: 176 rotations of
 // 2.4e8 terms 1.2 s in 2^25 buckets, 4.3 s on the sorted merges.)
 static constexpr int BB_ROOM = 3 * BB_CAP / 4;
+static constexpr int BB_ROOM_BITS = 19;
 static constexpr int BB_FULL = 7 * BB_CAP / 8;
 template <int NW>
 static int bk_regrid(pp_spv *h, int *cur, int *bits) {
@@ -1479,7 +1482,7 @@ static int bk_regrid(pp_spv *h, int *cur, int *bits) {
         TRY(rr);
         int mx = 0;
         TRY(bk_scatter<NW>(h, h->bkz[*cur], h->bkx[*cur], h->bkc[*cur], 0, *cur, *bits, *cur ^ 1, nbits, &mx));
-        if (mx >= 0 && mx <= (h->bk_cap == BB_CAP ? BB_ROOM : h->bk_cap / 2)) break;
+        if (mx >= 0 && mx <= (h->bk_cap == BB_CAP && nbits >= BB_ROOM_BITS ? BB_ROOM : h->bk_cap / 2)) break;
         held = h->bk_cap == BB_CAP && mx >= 0;
     }
     *cur ^= 1;

@@ -1976,8 +1976,9 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
     bool use_bk = bk_enabled();
     bool dense = false;                      // the last state read showed a dense live set
     bool roomy = false;                      // the live sets have room for a merge's output slots
+    bool stuck = false;                      // the last launch of k_small_run ran nothing
     while (done < L) {
-        if (small_ok && ncur <= small_cap<NW>()) {
+        if (small_ok && !stuck && ncur <= small_cap<NW>()) {
             Bufs B = make_bufs(h);
             k_small_run<NW><<<1, SM_THREADS, small_smem<NW>(), h->stream>>>(B);
             prof->launches += 1;
@@ -1988,7 +1989,7 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
             table = false;
             ncur = st.n;
             dense = st.seg_dense != 0;
-            if (st.rot == done) ncur = small_cap<NW>() + 1;   // no progress: leave it to the multi-kernel path
+            stuck = st.rot == done;             // no progress: leave it to the multi-kernel path
             done = st.rot;
             continue;
         }
@@ -2009,10 +2010,8 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
         }
         if (!roomy) {
             // output slots for the first merges (buckets and the small kernel need none)
-            DevState st;
-            TRY(read_state(h, &st));
-            if (3 * st.n + 2 * SEG > h->cap) table = false;
-            TRY(ensure_live(h, 3 * st.n + 2 * SEG));
+            if (3 * ncur + 2 * SEG > h->cap) table = false;
+            TRY(ensure_live(h, 3 * ncur + 2 * SEG));
             roomy = true;
         }
         dense = false;                       // the merge kernels leave a segment table
@@ -2059,6 +2058,7 @@ static int run_struct(pp_spv *h, long long start, long long L, pp_counters *ctr,
         DevState st;
         TRY(read_state(h, &st));
         ncur = st.n;
+        stuck = false;
         if (timed) {
             // rotations that ran are [done, st.rot); the rest were no-ops
             const long long base = (long long)ev.size() / 5 - (end - done);

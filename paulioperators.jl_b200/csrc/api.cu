@@ -1930,7 +1930,9 @@ static int run_bucket(pp_spv *h, long long start, long long L, pp_counters *ctr,
             split = 1;
         if (done == L || !split || !inflight.empty()) continue;
         split = 0;
+        const int before = bits;
         const int rr = bk_regrid<NW>(h, &cur, &bits);
+        limit = std::min(BB_DMAX, limit + bits - before);      // (half the load lets a coset have twice the buckets)
         PP_TRACE("buckets: split at rotation %lld (%lld terms, largest bucket %d) -> 2^%d buckets%s", done, n, last.maxcnt,
                  bits, rr == BK_NOFIT ? ": does not fit" : "");
         if (rr == BK_NOFIT && !tight && !(over & 1)) {

@@ -182,11 +182,11 @@ struct pp_spv {
 // that it does not hold costs 6.5 ms, and as much when it is trimmed away, where cudaMalloc
 // and cudaFree take 0.66 and 0.93 (64 MiB: 0.41 and 0.39, 0.35 and 0.30).  Where a call's
 // buffers are beyond what is kept that is what it costs: an evolve of a copy of 6.9e6 terms
-// by 32 rotations took 321 ms with one pool for all sizes, 79 so, 49 in kernels; one of
-// 2.2e6 terms 148 and 34.
+// by 32 rotations took 321 ms with one pool for all sizes, 79 so with the same layouts, 39
+// of them in kernels; one of 2.2e6 terms 148 and 34.
 // What is held unused is bounded by MEM_KEEP (checked when a handle frees a large block or
-// is destroyed; the longest unused blocks go first; 3 GiB instead of 8: an evolve of a copy
-// of 2.2e6 terms by eight rotations 6.0 ms instead of 3.3) and all returned when the last
+// is destroyed; the longest unused blocks go first; with 3 GiB instead of 8 an evolve of a
+// copy of 2.2e6 terms by 24 rotations took 9.7 ms instead of 6.5) and all returned when the last
 // handle is destroyed, or when an allocation fails.
 static constexpr size_t MEM_BIG = 64ull << 20;
 static constexpr size_t MEM_KEEP = 8ull << 30;
@@ -1034,6 +1034,14 @@ extern "C" int pp_create(int32_t N, int64_t live_cap, int64_t append_cap, pp_spv
     return PP_OK;
 }
 
+// Waits for the idle streams, on which destroyed handles freed their memory (only memory
+// whose free has run can be returned).
+static int streams_wait(DevPool &d) {
+    std::lock_guard<std::mutex> lk(d.mu);
+    for (cudaStream_t s : d.streams) CU(cudaStreamSynchronize(s));
+    return PP_OK;
+}
+
 extern "C" int pp_destroy(pp_spv *h) {
     if (!h) return PP_OK;
     if (h->stream) cudaStreamSynchronize(h->stream);
@@ -1059,8 +1067,11 @@ extern "C" int pp_destroy(pp_spv *h) {
                 h->stream = nullptr;
             }
         }
-        if (h->stream) cudaStreamDestroy(h->stream);
-        if (last) cudaDeviceSynchronize();
+        if (h->stream) {
+            cudaStreamSynchronize(h->stream);
+            cudaStreamDestroy(h->stream);
+        }
+        if (last) streams_wait(dp);
         mem_trim(h->dev, last ? 0 : MEM_KEEP);
     }
     delete h;
@@ -3035,12 +3046,7 @@ extern "C" int pp_debug_lookback_timeout(int64_t limit) {
 extern "C" int pp_release_memory(void) {
     int dev = 0;
     CU(cudaGetDevice(&dev));
-    {
-        // (only memory whose free has run can be returned: destroyed handles free on their streams)
-        DevPool &d = dev_pool(dev);
-        std::lock_guard<std::mutex> lk(d.mu);
-        for (cudaStream_t s : d.streams) CU(cudaStreamSynchronize(s));
-    }
+    TRY(streams_wait(dev_pool(dev)));
     mem_trim(dev, 0);
     return PP_OK;
 }

@@ -25,8 +25,8 @@
 // takes more rotations per launch.  The index over all resident terms is built once per
 // block and pays from about three rotations on.
 // Measured (one B200, whole calls, one rotation per launch before): 8 x 8 lattice,
-// 3,520 rotations, up to 3.9e6 terms 154.9 -> 86 ms; 127-qubit graph, 6,504 rotations, up
-// to 8e4 terms 43.4 -> 16.3 ms; 48 batched instances 60.1 -> 38 ms.  (A warp per coset
+// 3,520 rotations, up to 3.9e6 terms 154.9 -> 84 ms; 127-qubit graph, 6,504 rotations, up
+// to 8e4 terms 43.4 -> 16.3 ms; 48 batched instances 60.1 -> 35 ms.  (A warp per coset
 // everywhere: 109, 19.6 and 42.6; a CTA everywhere: 111, 16.2 and 38.4 with cosets of 512
 // terms, 96, 18.9 and 38.4 with cosets of 900; the lattice at 95 then.)
 #pragma once

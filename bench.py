@@ -62,10 +62,10 @@ BYTES_PER_TERM = {1: 24, 2: 40}     # B = 2*(W/8) + 8
 MERGE_TRAFFIC_PER_ALG_BYTE = 115.09 / 150.88
 # DRAM traffic of k_bb_block<1> per algorithmic byte, from one ncu capture of
 # the four launches of 24 rotations of this circuit at n = 2.06e6 live terms:
-# (dram__bytes_read.sum + dram__bytes_write.sum) = 170.1 MB per launch of six rotations
+# (dram__bytes_read.sum + dram__bytes_write.sum) = 172.1 MB per launch of six rotations
 # against B(n_in + n_out) = 99.1 MB (a term is a 32-byte record, short bucket runs share
 # their DRAM bursts with empty slots; part of the writes is still in L2 at the end)
-BUCKET_TRAFFIC_PER_ALG_BYTE = 680.26 / 396.58
+BUCKET_TRAFFIC_PER_ALG_BYTE = 688.21 / 396.58
 
 
 def parse():
